@@ -62,10 +62,10 @@ void launch_color(vsdmo_opt_s* o, int c, cudaStream_t s) {
         const float* Y = o->ws.Y.p;
         if (o->proposals_once) Y = o->Yall.p + (size_t)(L.v0 - o->nb_base) * mlp::OUTP;
         else o->model->m.infer_tet(m.pos.p, o->nb.p, o->nbn.p, o->nb_base, L.v0, n, o->ws.Y.p, mlp::OUTP, s);
-        launch_dmo_tet_learned(m, L, Y, mlp::OUTP, o->reduced_n, o->reduced_depth, o->reduced_scale,
+        launch_dmo_tet_learned(m, L, o->ring(), Y, mlp::OUTP, o->reduced_n, o->reduced_depth, o->reduced_scale,
                                o->counters.p, o->dirty.p, o->fb_list.p, o->fb_count.p, s);
     } else if (o->mode == MODE_TET) {
-        launch_dmo_tet(m, L, s, o->dirty.p, o->dirty.p ? o->counters.p + 3 : nullptr);
+        launch_dmo_tet(m, L, o->ring(), s, o->dirty.p, o->dirty.p ? o->counters.p + 3 : nullptr);
     } else if (o->mode == MODE_HEX) {
         if (o->kind == MK_HEX_COND) launch_dmo_hex_cond(m, L, s);
         else launch_dmo_hex(m, L, s);
@@ -82,15 +82,16 @@ void launch_color(vsdmo_opt_s* o, int c, cudaStream_t s) {
 
 }  // namespace
 
-// ring-vertex table of the inner (tet) range, built once: the topology never changes
-void vsdmo_opt_s::ensure_neighbours() {
+// ring table of the inner (tet) range, built once: the topology never changes
+void vsdmo_opt_s::ensure_rings() {
     if (nb.p) return;
     const Mesh& m = mesh->m;
     const int n = m.nV - m.nSurf;
     nb_base = m.nSurf;
     nb.alloc((size_t)std::max(n, 1) * 32, m.stream);
     nbn.alloc(std::max(n, 1), m.stream);
-    launch_tet_neighbours(m, m.nSurf, m.nV, nb.p, nbn.p, m.stream);
+    corner.alloc((size_t)std::max(n, 1) * 32, m.stream);
+    launch_tet_rings(m, m.nSurf, m.nV, nb.p, nbn.p, corner.p, m.stream);
 }
 
 namespace {
@@ -688,6 +689,7 @@ VSDMO_API vsdmo_status vsdmo_opt_create(vsdmo_mesh_t mesh, const vsdmo_params* p
         if (o->mode == MODE_SURF || o->slide || o->volsurf) init_surface_state(o.get());
         o->counters.alloc(4, s);
         o->counters.zero();
+        if (o->mode == MODE_TET) o->ensure_rings();
         if (o->mode == MODE_TET && p.active_set) {
             o->dirty.alloc(m.nV, s);
             o->dirty.fill_bytes(1);

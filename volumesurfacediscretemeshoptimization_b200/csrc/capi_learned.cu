@@ -199,7 +199,6 @@ VSDMO_API vsdmo_status vsdmo_opt_set_model(vsdmo_opt_t o, vsdmo_model_t model, i
             int maxn = 1;
             for (auto& r : o->ranges) maxn = std::max(maxn, r.second - r.first);
             o->ws.ensure(maxn, false, s);
-            o->ensure_neighbours();
             if (!o->fb_list.p || (int)o->fb_list.n < maxn) o->fb_list.alloc(maxn, s);
             if (!o->fb_count.p) o->fb_count.alloc(2, s);
             o->fb_count.zero();
@@ -219,7 +218,6 @@ VSDMO_API vsdmo_status vsdmo_opt_set_proposal_schedule(vsdmo_opt_t o, int once_a
         const Mesh& m = o->mesh->m;
         o->once_after = once_after;
         if (once_after >= 0 && !o->Yall.p) o->Yall.alloc((size_t)std::max(m.nV - m.nSurf, 1) * mlp::OUTP, m.stream);
-        if (once_after >= 0) o->ensure_neighbours();
         m.sync();
     });
 }
@@ -262,7 +260,6 @@ VSDMO_API vsdmo_status vsdmo_opt_collect_pairs(vsdmo_opt_t o, int n_iter, float*
         for (auto& r : o->ranges) maxn = std::max(maxn, r.second - r.first);
         DBuf<float> scale(maxn, s);
         DBuf<float4> old(maxn, s);
-        o->ensure_neighbours();
         for (int it = 0; it < n_iter && rows < capacity; ++it) {
             for (auto& r : o->ranges) {
                 const int n = (int)std::min<long>(r.second - r.first, capacity - rows);
@@ -270,7 +267,7 @@ VSDMO_API vsdmo_status vsdmo_opt_collect_pairs(vsdmo_opt_t o, int n_iter, float*
                 launch_tet_features(m, r.first, r.first + n, o->nb.p, o->nbn.p, o->nb_base, feats + rows * mlp::IN,
                                     nullptr, scale.p, old.p, s);
                 DmoLaunch L{r.first, r.second, o->p.grid_scale, o->p.depth};
-                launch_dmo_tet(m, L, s);
+                launch_dmo_tet(m, L, o->ring(), s);
                 launch_tet_targets(m, r.first, r.first + n, scale.p, old.p, targets + rows * mlp::OUT, s);
                 rows += n;
             }

@@ -12,13 +12,13 @@
 //     vertex and scaled by an exact power of two, the tet determinant is affine in the
 //     candidate p (det = d0 - n.p) and the sum of the six squared edge lengths is
 //     quadratic (L = C - 2 s.p + 3|p|^2); the flat-triangle area and edge sum likewise;
-//   * each lane owns 16 (tet) or 2 (2D) candidates of a separable grid, so one element
-//     costs 3 FMAs + a compare per candidate instead of a full metric evaluation;
+//   * the grid is separable: each lane owns 16 (tet) or 2 (2D) candidates; tets are judged by an
+//     exact candidate filter first (tet_search.cuh), so few candidates cost a full ring key;
 //   * the ring minimum is compared through the monotone transform det^2/L^3 (A/L in 2D),
 //     kept as a fraction and compared by cross-multiplication (no cbrt or divide per
 //     element); inverted elements key the ring by their most negative det / area, the
 //     analogue of the reference returning the negative volume / area;
-//   * the block-wide cub::ArgMax becomes a warp butterfly on (key, candidate index).
+//   * the block-wide cub::ArgMax becomes a warp reduction on (key, candidate index).
 // The library is compiled with --fmad=false: the only fused multiply-adds are the written
 // fmaf() calls, so the CPU restatement in oracle/or_dmo.c reproduces every bit.
 //
@@ -28,7 +28,7 @@
 #include "vsdmo_internal.cuh"
 #include "tc_gemm.cuh"
 #include "angle_metrics.cuh"
-#include "tet_key.cuh"
+#include "tet_search.cuh"
 #include "hex_key.cuh"
 #include "hex_cond.cuh"
 #include "quad_cond.cuh"
@@ -39,39 +39,18 @@
 namespace vsdmo {
 namespace {
 
-constexpr int NQ = 8;
 constexpr unsigned FULL = 0xffffffffu;
 
 // packed position of feature (row, col) in the network's 96-column input operand
 __device__ __forceinline__ size_t learned_pk_off(long row, int col) { return tc::pk_off(row, col, 96); }
-// launch shape of the tet kernel: 4 warps per block, measured fastest on B200 against 2 and 8
-#ifndef TET_WARPS_CFG
-#define TET_WARPS_CFG 4
-#endif
-#ifndef TET_MIN_BLOCKS
-#define TET_MIN_BLOCKS 0
-#endif
-#ifndef TET_SPLIT_Y
-#define TET_SPLIT_Y 0
-#endif
-constexpr int TET_WARPS = TET_WARPS_CFG;
+// launch shape of the tet kernels: one warp per block, so a warp's registers and shared memory go
+// to the next vertex as soon as its own is done (searches differ in length by 5 x); one / two / four
+// warps per block took 0.404 / 0.437 / 0.443 ms per iteration of the 48^3 cube
+constexpr int TET_WARPS = 1;
+constexpr int TET_MIN_BLOCKS = 28;   // 72 registers
 constexpr int TRI_WARPS = 4;
 constexpr int TET_MAX_RING = 512;
 constexpr int TRI_MAX_RING = 256;
-
-// candidate offsets (N-1-2i)/(N-1): i = 0 is +extent, i = N-1 is -extent (DMOTetImplCub.h:101-103)
-__device__ __forceinline__ float grid_offset(int i) {
-    switch (i) {
-    case 0: return 7.0f / 7.0f;
-    case 1: return 5.0f / 7.0f;
-    case 2: return 3.0f / 7.0f;
-    case 3: return 1.0f / 7.0f;
-    case 4: return -1.0f / 7.0f;
-    case 5: return -3.0f / 7.0f;
-    case 6: return -5.0f / 7.0f;
-    default: return -7.0f / 7.0f;
-    }
-}
 
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
@@ -89,77 +68,6 @@ __device__ __forceinline__ void warp_argmax(float& k, int& i) {
     }
 }
 
-// Ring minimum of the lane's candidates (fixed x, NJ y values, all NQ z values) over the k
-// tets of the ring; returns the lane's best (key, linear index), strict > in index order.
-template <int NJ>
-__device__ __forceinline__ void tet_lane_best(const float4* __restrict__ co, int k, float x, const float* y,
-                                              const float* z, const float* tz, int ci, int cj, int jbase,
-                                              float& bk, int& bi) {
-    const float tx = (3.0f * x) * x;
-    float ty[NJ];
-#pragma unroll
-    for (int jj = 0; jj < NJ; ++jj) ty[jj] = (3.0f * y[jj]) * y[jj];
-    float N[NJ][NQ], D[NJ][NQ], dm[NJ][NQ];
-    {
-        const float4 K0 = co[0], K1 = co[1];
-        const float detA = fmaf(K0.x, x, K0.w);
-        const float LA = K1.w + fmaf(K1.x, x, tx);
-#pragma unroll
-        for (int jj = 0; jj < NJ; ++jj) {
-            const float detB = fmaf(K0.y, y[jj], detA), LB = LA + fmaf(K1.y, y[jj], ty[jj]);
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const float det = fmaf(K0.z, z[q], detB), L = LB + fmaf(K1.z, z[q], tz[q]);
-                N[jj][q] = det * det; D[jj][q] = (L * L) * L; dm[jj][q] = det;
-            }
-        }
-    }
-    for (int t = 1; t < k; ++t) {
-        const float4 K0 = co[2 * t], K1 = co[2 * t + 1];
-        const float detA = fmaf(K0.x, x, K0.w);
-        const float LA = K1.w + fmaf(K1.x, x, tx);
-        float detB[NJ], LB[NJ];
-#pragma unroll
-        for (int jj = 0; jj < NJ; ++jj) { detB[jj] = fmaf(K0.y, y[jj], detA); LB[jj] = LA + fmaf(K1.y, y[jj], ty[jj]); }
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const float lz = fmaf(K1.z, z[q], tz[q]);
-#pragma unroll
-            for (int jj = 0; jj < NJ; ++jj) {
-                const float det = fmaf(K0.z, z[q], detB[jj]), L = LB[jj] + lz;
-                const float num = det * det, den = (L * L) * L;
-                if (num * D[jj][q] < N[jj][q] * den) { N[jj][q] = num; D[jj][q] = den; }
-                dm[jj][q] = fminf(dm[jj][q], det);
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-#pragma unroll
-        for (int jj = 0; jj < NJ; ++jj) {
-            const float key = dm[jj][q] < 0.f ? dm[jj][q] : N[jj][q] / D[jj][q];
-            const int idx = ci + 8 * (cj + 4 * (jbase + jj)) + 64 * q;
-            if (key > bk || (key == bk && idx < bi)) { bk = key; bi = idx; }
-        }
-    }
-}
-
-// ---- candidate filter of the tet search --------------------------------------------------------
-// The ring key of a candidate is a minimum over the ring's tets, so the minimum over any subset
-// of them bounds it from above. A level can only move the vertex to a candidate whose key
-// beats qLast, so a candidate whose key over a few tets is already below qLast can never be
-// chosen: the search evaluates the TET_CRIT tets with the smallest keys at the level's centre
-// for all 512 candidates, keeps the candidates that are not below qLast (with a relative
-// margin of 2^-14 that covers the rounding of the fraction comparisons), and evaluates the
-// full ring only for those, in the same operations and tet order as the plain search. The
-// winner, and whether the vertex moves, are the same as without the filter: every candidate
-// that beats qLast survives, and no discarded candidate can tie with or exceed one that does.
-#ifndef TET_CRIT_CFG
-#define TET_CRIT_CFG 6
-#endif
-constexpr int TET_CRIT = TET_CRIT_CFG;   // tets of the filter
-constexpr int TET_LIST = 256;    // survivors per warp evaluated from a list (more: full search)
-
 // (num, den, det) of tet t at (x, y, z): the operations of tet_key1
 __device__ __forceinline__ float tet_piece_key(const float4* __restrict__ co, int t, float x, float y, float z) {
     const float4 c0 = co[2 * t], c1 = co[2 * t + 1];
@@ -169,146 +77,11 @@ __device__ __forceinline__ float tet_piece_key(const float4* __restrict__ co, in
     return det < 0.f ? det : (det * det) / ((L * L) * L);
 }
 
-// The TET_CRIT tets of smallest key at (x, y, z), the same on all lanes. Any choice of tets gives
-// an exact filter (the key over any subset bounds the ring key from above), so the choice needs
-// no exact arithmetic: a ring of up to 32 tets keys each tet once on its lane (fast division),
-// orders the keys as unsigned integers whose low 5 bits are the tet index and takes the minimum
-// TET_CRIT times with one warp reduction each. Larger rings scan their tets per round.
+// a key's order as an unsigned integer, its low 5 bits replaced by the tet index
 __device__ __forceinline__ unsigned tet_order_key(float key, int t) {
     const unsigned b = __float_as_uint(key);
     const unsigned o = (b & 0x80000000u) ? ~b : (b | 0x80000000u);   // float order as unsigned order
     return (o & ~31u) | (unsigned)t;
-}
-
-__device__ __forceinline__ float tet_piece_key_fast(const float4* __restrict__ co, int t, float x, float y, float z) {
-    const float4 c0 = co[2 * t], c1 = co[2 * t + 1];
-    const float tx = (3.0f * x) * x, ty = (3.0f * y) * y, tz = (3.0f * z) * z;
-    const float det = fmaf(c0.z, z, fmaf(c0.y, y, fmaf(c0.x, x, c0.w)));
-    const float L = ((c1.w + fmaf(c1.x, x, tx)) + fmaf(c1.y, y, ty)) + fmaf(c1.z, z, tz);
-    return det < 0.f ? det : __fdividef(det * det, (L * L) * L);
-}
-
-__device__ __forceinline__ void tet_critical(const float4* __restrict__ co, int k, float x, float y, float z, int lane,
-                                             int (&crit)[TET_CRIT]) {
-    if (k <= 32) {
-        unsigned mine = lane < k ? tet_order_key(tet_piece_key_fast(co, lane, x, y, z), lane) : 0xffffffffu;
-#pragma unroll
-        for (int r = 0; r < TET_CRIT; ++r) {
-            const unsigned m = __reduce_min_sync(FULL, mine);
-            const int t = (int)(m & 31u);
-            crit[r] = t < k ? t : 0;
-            if (lane == t) mine = 0xffffffffu;
-        }
-        return;
-    }
-#pragma unroll
-    for (int r = 0; r < TET_CRIT; ++r) {
-        unsigned best = 0xffffffffu;
-        int bt = 0;
-        for (int t = lane; t < k; t += 32) {
-            bool used = false;
-#pragma unroll
-            for (int q = 0; q < r; ++q) used |= (crit[q] == t);
-            if (used) continue;
-            const unsigned kt = tet_order_key(tet_piece_key_fast(co, t, x, y, z), t & 31);
-            if (kt < best || (kt == best && t < bt)) { best = kt; bt = t; }
-        }
-        // the warp's smallest (key, tet) pair: reduce the key, then the tet among the lanes holding it
-        const unsigned m = __reduce_min_sync(FULL, best);
-        const unsigned tt = __reduce_min_sync(FULL, best == m ? (unsigned)bt : 0xffffffffu);
-        crit[r] = tt < (unsigned)k ? (int)tt : 0;
-    }
-}
-
-// the lane's 16 candidates (fixed x, y[2], z[8]) over the critical tets: bit jj * 8 + q set when
-// the candidate survives (its key over the subset is not below thr). Used when thr <= 0 (the
-// ring has an inverted tet, whose key is its det); tet_filter_pos covers thr > 0.
-#ifndef TET_FILTER_NEG_INLINE
-#define TET_FILTER_NEG_INLINE 1
-#endif
-#if TET_FILTER_NEG_INLINE
-__device__ __forceinline__
-#else
-__device__ __noinline__
-#endif
-unsigned tet_filter(const float4* __restrict__ co, const int (&crit)[TET_CRIT], int m,
-                                               float x, const float* y, const float* z, const float* tz, float thr) {
-    const float tx = (3.0f * x) * x;
-    const float ty[2] = { (3.0f * y[0]) * y[0], (3.0f * y[1]) * y[1] };
-    float N[2][NQ], D[2][NQ], dm[2][NQ];
-#pragma unroll
-    for (int r = 0; r < TET_CRIT; ++r) {
-        if (r >= m) break;
-        const int t = crit[r];
-        const float4 K0 = co[2 * t], K1 = co[2 * t + 1];
-        const float detA = fmaf(K0.x, x, K0.w);
-        const float LA = K1.w + fmaf(K1.x, x, tx);
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-            const float detB = fmaf(K0.y, y[jj], detA), LB = LA + fmaf(K1.y, y[jj], ty[jj]);
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const float det = fmaf(K0.z, z[q], detB), L = LB + fmaf(K1.z, z[q], tz[q]);
-                const float num = det * det, den = (L * L) * L;
-                if (r == 0) { N[jj][q] = num; D[jj][q] = den; dm[jj][q] = det; continue; }
-                if (num * D[jj][q] < N[jj][q] * den) { N[jj][q] = num; D[jj][q] = den; }
-                dm[jj][q] = fminf(dm[jj][q], det);
-            }
-        }
-    }
-    unsigned alive = 0;
-#pragma unroll
-    for (int jj = 0; jj < 2; ++jj)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            // key < thr, with the fraction compared by cross-multiplication (its rounding is
-            // far inside thr's margin)
-            const bool below = dm[jj][q] < 0.f ? dm[jj][q] < thr : N[jj][q] < thr * D[jj][q];
-            if (!below) alive |= 1u << (jj * 8 + q);
-        }
-    return alive;
-}
-
-// thr > 0: a candidate survives when every critical tet has det > 0 and det^2 >= thr L^3, tested
-// as min over the tets of min(det, det^2 - thr L^3) > 0 -- one running minimum instead of a
-// fraction and a det. det, det^2 and L^3 are the values the fraction would be formed from, and
-// the fma rounds det^2 - thr L^3 once, so a tet whose key det^2 / L^3 is at least the current
-// key (thr lies 2^-14 of it lower) gives a positive value: every candidate that can beat the
-// current key survives.
-__device__ __forceinline__ unsigned tet_filter_pos(const float4* __restrict__ co, const int (&crit)[TET_CRIT], int m,
-                                                   float x, const float* y, const float* z, const float* tz,
-                                                   float thr) {
-    const float tx = (3.0f * x) * x;
-    const float ty[2] = { (3.0f * y[0]) * y[0], (3.0f * y[1]) * y[1] };
-    float s[2][NQ];
-#pragma unroll
-    for (int r = 0; r < TET_CRIT; ++r) {
-        if (r >= m) break;
-        const int t = crit[r];
-        const float4 K0 = co[2 * t], K1 = co[2 * t + 1];
-        const float detA = fmaf(K0.x, x, K0.w);
-        const float LA = K1.w + fmaf(K1.x, x, tx);
-        float lz[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) lz[q] = fmaf(K1.z, z[q], tz[q]);
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-            const float detB = fmaf(K0.y, y[jj], detA), LB = LA + fmaf(K1.y, y[jj], ty[jj]);
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const float det = fmaf(K0.z, z[q], detB), L = LB + lz[q];
-                const float v = fminf(det, fmaf(-thr, (L * L) * L, det * det));
-                s[jj][q] = r == 0 ? v : fminf(s[jj][q], v);
-            }
-        }
-    }
-    unsigned alive = 0;
-#pragma unroll
-    for (int jj = 0; jj < 2; ++jj)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-            if (s[jj][q] > 0.f) alive |= 1u << (jj * 8 + q);
-    return alive;
 }
 
 // Ring key with the tets spread over the lanes and a warp minimum of the per-tet keys (det if
@@ -326,129 +99,71 @@ __device__ __forceinline__ float tet_key_min(const float4* __restrict__ co, int 
 
 // Setup of one tet vertex shared by the plain and the learned search: per-axis extent of the
 // ring (DMOTetImplCub.h:54-64), the exact power-of-two scale 2^ex and the element coefficients
-// in shared memory. Returns false when the ring is degenerate (the vertex is left alone).
-// KEEP: rings of up to 32 tets (all of a Kuhn cube's) keep their lane's corners in registers
-// between the extent and the coefficients; otherwise the corners are loaded again.
-template <bool KEEP>
-__device__ __forceinline__ bool tet_setup(const float4* __restrict__ pos, const int4* __restrict__ hf, int b, int k,
-                                          float4 c0, int lane, float4* co, float& sx, float& sy, float& sz, int& ex) {
-    float mdx = 0.f, mdy = 0.f, mdz = 0.f;
-    const bool one = KEEP && k <= 32;
-    float4 qa = c0, qb = c0, qc = c0;
-    if (one) {
-        if (lane < k) {
-            const int4 h = hf[b + lane];
-            qa = pos[h.x]; qb = pos[h.y]; qc = pos[h.z];
-        }
-        mdx = fmaxf(fabsf(qa.x - c0.x), fmaxf(fabsf(qb.x - c0.x), fabsf(qc.x - c0.x)));
-        mdy = fmaxf(fabsf(qa.y - c0.y), fmaxf(fabsf(qb.y - c0.y), fabsf(qc.y - c0.y)));
-        mdz = fmaxf(fabsf(qa.z - c0.z), fmaxf(fabsf(qb.z - c0.z), fabsf(qc.z - c0.z)));
-    } else {
+// in shared memory. Returns the number of tets, 0 when the vertex is left alone (an empty,
+// oversized or degenerate ring). scratch: 512 bytes of shared memory per warp.
+//
+// Rings of up to 32 tets and 32 vertices come from the ring table: one coalesced row of ring
+// vertices and one of 16-bit corner triples per vertex, so every ring position is loaded once
+// (14 instead of 72 gathers for a Kuhn vertex) and two dependent loads reach the positions
+// instead of three (row pointer, halffaces, positions). Larger rings read their halffaces twice.
+__device__ __forceinline__ int tet_setup(const float4* __restrict__ pos, const int* __restrict__ rowptr,
+                                         const int4* __restrict__ hf, const TetRingTable& ring, int v, int maxk,
+                                         float4 c0, int lane, float4* co, float4* scratch, float& sx, float& sy,
+                                         float& sz, int& ex) {
+    const size_t row = (size_t)(v - ring.base) * 32 + lane;
+    const unsigned corner = ring.corner[row];
+    const float4 q = pos[ring.nb[row]];
+    const unsigned has = __ballot_sync(FULL, corner != TetRingTable::NONE);
+    if (__any_sync(FULL, corner == TetRingTable::LARGE)) {
+        float mdx = 0.f, mdy = 0.f, mdz = 0.f;
+        const int b = rowptr[v], k = rowptr[v + 1] - b;
+        if (k <= 0 || k > maxk) return 0;
         for (int t = lane; t < k; t += 32) {
             const int4 h = hf[b + t];
             const float4 pa = pos[h.x], pb = pos[h.y], pc = pos[h.z];
-            mdx = fmaxf(mdx, fabsf(pa.x - c0.x)); mdy = fmaxf(mdy, fabsf(pa.y - c0.y)); mdz = fmaxf(mdz, fabsf(pa.z - c0.z));
-            mdx = fmaxf(mdx, fabsf(pb.x - c0.x)); mdy = fmaxf(mdy, fabsf(pb.y - c0.y)); mdz = fmaxf(mdz, fabsf(pb.z - c0.z));
-            mdx = fmaxf(mdx, fabsf(pc.x - c0.x)); mdy = fmaxf(mdy, fabsf(pc.y - c0.y)); mdz = fmaxf(mdz, fabsf(pc.z - c0.z));
+            mdx = fmaxf(mdx, fmaxf(fabsf(pa.x - c0.x), fmaxf(fabsf(pb.x - c0.x), fabsf(pc.x - c0.x))));
+            mdy = fmaxf(mdy, fmaxf(fabsf(pa.y - c0.y), fmaxf(fabsf(pb.y - c0.y), fabsf(pc.y - c0.y))));
+            mdz = fmaxf(mdz, fmaxf(fabsf(pa.z - c0.z), fmaxf(fabsf(pb.z - c0.z), fabsf(pc.z - c0.z))));
         }
+        mdx = redux_max(mdx); mdy = redux_max(mdy); mdz = redux_max(mdz);
+        const float mm = fmaxf(mdx, fmaxf(mdy, mdz));
+        if (!(mm > 0.f) || !(mm < FLT_MAX)) return 0;
+        (void)frexpf(mm, &ex);
+        const float p = exp2_exact(-ex);
+        for (int t = lane; t < k; t += 32) {
+            const int4 h = hf[b + t];
+            const float4 pa = pos[h.x], pb = pos[h.y], pc = pos[h.z];
+            tet_coeffs(scale2(pa.x - c0.x, p, -ex), scale2(pa.y - c0.y, p, -ex), scale2(pa.z - c0.z, p, -ex),
+                       scale2(pb.x - c0.x, p, -ex), scale2(pb.y - c0.y, p, -ex), scale2(pb.z - c0.z, p, -ex),
+                       scale2(pc.x - c0.x, p, -ex), scale2(pc.y - c0.y, p, -ex), scale2(pc.z - c0.z, p, -ex),
+                       co[2 * t], co[2 * t + 1]);
+        }
+        __syncwarp();
+        sx = scale2(mdx, p, -ex); sy = scale2(mdy, p, -ex); sz = scale2(mdz, p, -ex);
+        return k;
     }
-    mdx = warp_max(mdx); mdy = warp_max(mdy); mdz = warp_max(mdz);
+    const int k = __popc(has);   // the triples fill the row from its start
+    const float ux = q.x - c0.x, uy = q.y - c0.y, uz = q.z - c0.z;
+    const float mdx = redux_max(fabsf(ux)), mdy = redux_max(fabsf(uy)), mdz = redux_max(fabsf(uz));
     const float mm = fmaxf(mdx, fmaxf(mdy, mdz));
-    if (!(mm > 0.f) || !(mm < FLT_MAX)) return false;
+    if (k == 0 || !(mm > 0.f) || !(mm < FLT_MAX)) return 0;
     (void)frexpf(mm, &ex);
     const float p = exp2_exact(-ex);
-    for (int t = lane; t < k; t += 32) {
-        float4 pa = qa, pb = qb, pc = qc;
-        if (!one) {
-            const int4 h = hf[b + t];
-            pa = pos[h.x]; pb = pos[h.y]; pc = pos[h.z];
-        }
-        float4 K0, K1;
-        tet_coeffs(scale2(pa.x - c0.x, p, -ex), scale2(pa.y - c0.y, p, -ex), scale2(pa.z - c0.z, p, -ex),
-                   scale2(pb.x - c0.x, p, -ex), scale2(pb.y - c0.y, p, -ex), scale2(pb.z - c0.z, p, -ex),
-                   scale2(pc.x - c0.x, p, -ex), scale2(pc.y - c0.y, p, -ex), scale2(pc.z - c0.z, p, -ex), K0, K1);
-        co[2 * t] = K0;
-        co[2 * t + 1] = K1;
+    scratch[lane] = make_float4(scale2(ux, p, -ex), scale2(uy, p, -ex), scale2(uz, p, -ex), 0.f);
+    __syncwarp();
+    if (lane < k) {
+        const float4 a = scratch[corner & 31u], b = scratch[(corner >> 5) & 31u], c = scratch[corner >> 10];
+        tet_coeffs(a.x, a.y, a.z, b.x, b.y, b.z, c.x, c.y, c.z, co[2 * lane], co[2 * lane + 1]);
     }
     __syncwarp();
     sx = scale2(mdx, p, -ex); sy = scale2(mdy, p, -ex); sz = scale2(mdz, p, -ex);
-    return true;
+    return k;
 }
 
 // position c0 + (dx, dy, dz) 2^ex of a move found in scaled local coordinates
 __device__ __forceinline__ float4 tet_unscale(float4 c0, float dx, float dy, float dz, int ex) {
     const float p = exp2_exact(ex);
     return make_float4(c0.x + scale2(dx, p, ex), c0.y + scale2(dy, p, ex), c0.z + scale2(dz, p, ex), c0.w);
-}
-
-// The plain hierarchical search (DMOTetImplCub.h:66-136) from the local origin: depth levels
-// of 8 x 8 x 8 candidates, moving on strict improvement of the ring key qLast. Returns whether
-// the vertex moved; (dx, dy, dz) is the new position in scaled local coordinates.
-__device__ __forceinline__ bool tet_plain_search(const float4* __restrict__ co, int* __restrict__ list, int k, float sx,
-                                                 float sy, float sz, float grid_scale, int depth, int lane, float qLast,
-                                                 float& dx, float& dy, float& dz) {
-    const int ci = lane & 7, cj = lane >> 3;
-    const float oi = grid_offset(ci), oj0 = grid_offset(cj), oj1 = grid_offset(cj + 4);
-    dx = 0.f; dy = 0.f; dz = 0.f;
-    bool moved = false;
-    float ds = grid_scale;
-    for (int level = 0; level < depth; ++level) {
-        const float Sx = ds * sx, Sy = ds * sy, Sz = ds * sz;
-        const float x = fmaf(oi, Sx, dx);
-        const float y[2] = { fmaf(oj0, Sy, dy), fmaf(oj1, Sy, dy) };
-        float z[NQ], tz[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) { z[q] = fmaf(grid_offset(q), Sz, dz); tz[q] = (3.0f * z[q]) * z[q]; }
-        float bk = -FLT_MAX;
-        int bi = 1 << 30;
-        // filter: candidates already below qLast over the centre's critical tets are dropped
-        int crit[TET_CRIT];
-        tet_critical(co, k, dx, dy, dz, lane, crit);
-        const float thr = qLast - (fabsf(qLast) * 0x1p-14f + 1e-37f);
-        const unsigned alive = thr > 0.f ? tet_filter_pos(co, crit, min(TET_CRIT, k), x, y, z, tz, thr)
-                                         : tet_filter(co, crit, min(TET_CRIT, k), x, y, z, tz, thr);
-        const int cnt = __popc(alive);
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int n = __shfl_up_sync(FULL, incl, o);
-            if (lane >= o) incl += n;
-        }
-        const int total = __shfl_sync(FULL, incl, 31);
-        if (total > TET_LIST) {
-#if TET_SPLIT_Y
-            tet_lane_best<1>(co, k, x, &y[0], z, tz, ci, cj, 0, bk, bi);
-            tet_lane_best<1>(co, k, x, &y[1], z, tz, ci, cj, 1, bk, bi);
-#else
-            tet_lane_best<2>(co, k, x, y, z, tz, ci, cj, 0, bk, bi);
-#endif
-        } else if (total > 0) {
-            int at = incl - cnt;
-            for (unsigned a = alive; a; a &= a - 1) {
-                const int bit = __ffs(a) - 1;
-                list[at++] = ci + 8 * (cj + 4 * (bit >> 3)) + 64 * (bit & 7);
-            }
-            __syncwarp();
-            for (int j = lane; j < total; j += 32) {
-                const int idx = list[j];
-                const float key = tet_key1(co, k, fmaf(grid_offset(idx & 7), Sx, dx),
-                                           fmaf(grid_offset((idx >> 3) & 7), Sy, dy), fmaf(grid_offset(idx >> 6), Sz, dz));
-                if (key > bk || (key == bk && idx < bi)) { bk = key; bi = idx; }
-            }
-            __syncwarp();
-        }
-        warp_argmax(bk, bi);
-        if (bi < NQ * NQ * NQ && qLast < bk) {
-            const float nx = fmaf(grid_offset(bi & 7), Sx, dx);
-            const float ny = fmaf(grid_offset((bi >> 3) & 7), Sy, dy);
-            const float nz = fmaf(grid_offset(bi >> 6), Sz, dz);
-            dx = nx; dy = ny; dz = nz;
-            qLast = bk;
-            moved = true;
-        }
-        ds = ds * (2.0f / 7.0f);
-    }
-    return moved;
 }
 
 // Active set (optional, dirty != null): a vertex whose last search found no improvement and
@@ -466,7 +181,7 @@ __device__ __forceinline__ void tet_mark_ring(const int4* __restrict__ hf, int b
 
 __global__ void __launch_bounds__(TET_WARPS * 32, TET_MIN_BLOCKS)
 k_dmo_tet(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ hf,
-          int v0, int v1, float grid_scale, int depth, int maxk, uint8_t* __restrict__ dirty,
+          TetRingTable ring, int v0, int v1, float grid_scale, int depth, int maxk, uint8_t* __restrict__ dirty,
           unsigned long long* __restrict__ skipped) {
     extern __shared__ float4 smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -477,19 +192,18 @@ k_dmo_tet(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* 
         return;
     }
     float4* co = smem + (size_t)w * maxk * 2;
-    int* list = reinterpret_cast<int*>(smem + (size_t)TET_WARPS * maxk * 2) + w * TET_LIST;
-    const int b = rowptr[v], k = rowptr[v + 1] - b;
-    if (k <= 0 || k > maxk) return;
+    float* scratch = reinterpret_cast<float*>(smem + (size_t)TET_WARPS * maxk * 2) + w * (TS_WARP_BYTES / 4);
     const float4 c0 = pos[v];
     float sx, sy, sz;
     int ex;
-    if (!tet_setup<true>(pos, hf, b, k, c0, lane, co, sx, sy, sz, ex)) return;
-    const float qLast = tet_key_origin(co, k);
+    const int k = tet_setup(pos, rowptr, hf, ring, v, maxk, c0, lane, co, reinterpret_cast<float4*>(scratch), sx, sy, sz, ex);
+    if (k == 0) return;
+    const float qLast = tet_group_key(co, k, 0.f, 0.f, 0.f, 32, lane);
     float dx, dy, dz;
-    const bool moved = tet_plain_search(co, list, k, sx, sy, sz, grid_scale, depth, lane, qLast, dx, dy, dz);
+    const bool moved = tet_plain_search(co, scratch, k, sx, sy, sz, grid_scale, depth, lane, qLast, dx, dy, dz);
     if (moved && lane == 0) pos[v] = tet_unscale(c0, dx, dy, dz, ex);
     if (dirty) {
-        if (moved) tet_mark_ring(hf, b, k, lane, dirty);
+        if (moved) tet_mark_ring(hf, rowptr[v], k, lane, dirty);
         else if (lane == 0) dirty[v] = 0;
     }
 }
@@ -498,35 +212,33 @@ k_dmo_tet(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* 
 // warps stride over list[0 .. count[0]). The last warp to finish sets the queue back to empty
 // (count[0] = 0; count[1] counts the finished warps), so the next class's learned search
 // appends to an empty queue without a separate reset launch.
-#ifndef TET_LIST_MIN_BLOCKS
-#define TET_LIST_MIN_BLOCKS 4   // 128 registers: four blocks per SM (164 unconstrained, three blocks)
-#endif
+constexpr int TET_LIST_MIN_BLOCKS = 24;   // 80 registers
 __global__ void __launch_bounds__(TET_WARPS * 32, TET_LIST_MIN_BLOCKS)
 k_dmo_tet_list(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ hf,
-               const int* __restrict__ list, int* __restrict__ count, float grid_scale, int depth, int maxk,
+               TetRingTable ring, const int* __restrict__ list, int* __restrict__ count, float grid_scale, int depth, int maxk,
                uint8_t* __restrict__ dirty, unsigned long long* __restrict__ moved_count) {
     extern __shared__ float4 smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float4* co = smem + (size_t)w * maxk * 2;
-    int* slist = reinterpret_cast<int*>(smem + (size_t)TET_WARPS * maxk * 2) + w * TET_LIST;
+    float* scratch = reinterpret_cast<float*>(smem + (size_t)TET_WARPS * maxk * 2) + w * (TS_WARP_BYTES / 4);
     const int n = *count;
     for (int idx = blockIdx.x * TET_WARPS + w; idx < n; idx += gridDim.x * TET_WARPS) {
         const int v = list[idx];
-        const int b = rowptr[v], k = rowptr[v + 1] - b;
-        if (k <= 0 || k > maxk) continue;
         const float4 c0 = pos[v];
         float sx, sy, sz;
         int ex;
-        if (!tet_setup<true>(pos, hf, b, k, c0, lane, co, sx, sy, sz, ex)) continue;
-        const float qLast = tet_key_origin(co, k);
+        const int k = tet_setup(pos, rowptr, hf, ring, v, maxk, c0, lane, co, reinterpret_cast<float4*>(scratch), sx, sy,
+                                sz, ex);
+        if (k == 0) continue;
+        const float qLast = tet_group_key(co, k, 0.f, 0.f, 0.f, 32, lane);
         float dx, dy, dz;
-        const bool moved = tet_plain_search(co, slist, k, sx, sy, sz, grid_scale, depth, lane, qLast, dx, dy, dz);
+        const bool moved = tet_plain_search(co, scratch, k, sx, sy, sz, grid_scale, depth, lane, qLast, dx, dy, dz);
         if (moved && lane == 0) {
             pos[v] = tet_unscale(c0, dx, dy, dz, ex);
             atomicAdd(moved_count, 1ull);
         }
         if (dirty) {
-            if (moved) tet_mark_ring(hf, b, k, lane, dirty);
+            if (moved) tet_mark_ring(hf, rowptr[v], k, lane, dirty);
             else if (lane == 0) dirty[v] = 0;
         }
         __syncwarp();
@@ -544,27 +256,82 @@ k_dmo_tet_list(float4* __restrict__ pos, const int* __restrict__ rowptr, const i
 }
 
 // ---- learned proposal (tet) -------------------------------------------------------------------
-// Distinct ring vertices of every vertex in [v0, v1), in first-occurrence order of its
-// halfface row, at most 32 (the topology is fixed, so this runs once per optimiser):
-// nb [(v - v0) * 32 + a], nbn [v - v0].
-__global__ void k_tet_neighbours(const int* __restrict__ rowptr, const int4* __restrict__ hf, int v0, int v1,
-                                 int* __restrict__ nb, int* __restrict__ nbn) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < v1 - v0; i += gridDim.x * blockDim.x) {
+// Ring table of the vertices [v0, v1) (the topology is fixed, so it is built once per optimiser):
+// the distinct ring vertices of each in first-occurrence order of its halfface row, at most 32
+// (nb [(v - v0) * 32 + a], unused places hold v; nbn [v - v0] their number), and the corners of its
+// tets as indices into that row (corner [(v - v0) * 32 + t] = a | b << 5 | c << 10, NONE beyond the
+// ring; the first is LARGE for a ring of more than 32 tets or vertices). One warp per vertex.
+__global__ void __launch_bounds__(128)
+k_tet_rings(const int* __restrict__ rowptr, const int4* __restrict__ hf, int v0, int v1, int* __restrict__ nb,
+            int* __restrict__ nbn, uint16_t* __restrict__ corner) {
+    __shared__ int s_ids[4][96];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int* ids = s_ids[w];
+    for (int i = blockIdx.x * 4 + w; i < v1 - v0; i += gridDim.x * 4) {
         const int v = v0 + i;
         const int b = rowptr[v], k = rowptr[v + 1] - b;
         int* out = nb + (size_t)i * 32;
-        int n = 0;
-        for (int t = 0; t < k; ++t) {
-            const int4 h = hf[b + t];
-            const int u3[3] = { h.x, h.y, h.z };
+        if (k > 32) {
+            int n = 0;
+            if (lane == 0) {
+                for (int t = 0; t < k; ++t) {
+                    const int4 h = hf[b + t];
+                    const int u3[3] = { h.x, h.y, h.z };
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                bool seen = false;
-                for (int a = 0; a < n; ++a) seen |= out[a] == u3[j];
-                if (!seen && n < 32) out[n++] = u3[j];
+                    for (int j = 0; j < 3; ++j) {
+                        bool seen = false;
+                        for (int a = 0; a < n; ++a) seen |= ids[a] == u3[j];
+                        if (!seen && n < 32) ids[n++] = u3[j];
+                    }
+                }
+                nbn[i] = n;
             }
+            n = __shfl_sync(FULL, n, 0);
+            __syncwarp();
+            out[lane] = lane < n ? ids[lane] : v;
+            corner[(size_t)i * 32 + lane] = TetRingTable::LARGE;
+            __syncwarp();
+            continue;
         }
-        nbn[i] = n;
+        int u3[3] = { v, v, v };
+        if (lane < k) {
+            const int4 h = hf[b + lane];
+            u3[0] = h.x; u3[1] = h.y; u3[2] = h.z;
+            ids[3 * lane] = h.x; ids[3 * lane + 1] = h.y; ids[3 * lane + 2] = h.z;
+        }
+        __syncwarp();
+        // place of the first occurrence of each corner among the 3 k corners
+        int f3[3] = { 96, 96, 96 };
+        for (int q = 3 * k - 1; q >= 0; --q) {
+            const int u = ids[q];
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+                if (u == u3[j]) f3[j] = q;
+        }
+        unsigned first[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) first[j] = __ballot_sync(FULL, lane < k && f3[j] == 3 * lane + j);
+        const int n = __popc(first[0]) + __popc(first[1]) + __popc(first[2]);
+        unsigned code = 0;
+        int r3[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int tt = min(f3[j] / 3, 31), jj = f3[j] - 3 * (f3[j] / 3);
+            const unsigned lower = (1u << tt) - 1u;
+            int r = __popc(first[0] & lower) + __popc(first[1] & lower) + __popc(first[2] & lower);
+            if (jj > 0) r += (first[0] >> tt) & 1u;
+            if (jj > 1) r += (first[1] >> tt) & 1u;
+            r3[j] = r;
+            code |= (unsigned)(r & 31) << (5 * j);
+        }
+        __syncwarp();
+        if (lane >= n) out[lane] = v;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            if (((first[j] >> lane) & 1u) && r3[j] < 32) out[r3[j]] = u3[j];
+        if (lane == 0) nbn[i] = min(n, 32);
+        corner[(size_t)i * 32 + lane] = n > 32 ? TetRingTable::LARGE : lane < k ? (uint16_t)code : TetRingTable::NONE;
+        __syncwarp();
     }
 }
 
@@ -677,17 +444,10 @@ __device__ __forceinline__ float reduced_offset(int i, int n) { return (float)(n
 // accept and the minimum quality never decreases. counters: [0] reduced accepted,
 // [1] fallbacks, [2] fallbacks that moved, [3] skipped by the active set. rscale: first
 // reduced half-extent in units of grid_scale x the per-axis ring extent.
-// eight blocks per SM (64 registers, 16 bytes of spills) with the ring corners kept through the
-// setup: 2.3 % less time per learned iteration than seven blocks at 72 registers without
-#ifndef TET_LEARNED_MIN_BLOCKS
-#define TET_LEARNED_MIN_BLOCKS 8
-#endif
-#ifndef TET_LEARNED_KEEP
-#define TET_LEARNED_KEEP true
-#endif
+constexpr int TET_LEARNED_MIN_BLOCKS = 32;   // 64 registers (24 bytes of spills): 32 warps per SM
 __global__ void __launch_bounds__(TET_WARPS * 32, TET_LEARNED_MIN_BLOCKS)
-k_dmo_tet_learned(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ hf, int v0,
-                  int v1, float grid_scale, int maxk, const float* __restrict__ Y, int ldy, int rn, int rdepth,
+k_dmo_tet_learned(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ hf,
+                  TetRingTable ring, int v0, int v1, float grid_scale, int maxk, const float* __restrict__ Y, int ldy, int rn, int rdepth,
                   float rscale, unsigned long long* __restrict__ counters, uint8_t* __restrict__ dirty,
                   int* __restrict__ fb_list, int* __restrict__ fb_count) {
     extern __shared__ float4 smem[];
@@ -699,12 +459,12 @@ k_dmo_tet_learned(float4* __restrict__ pos, const int* __restrict__ rowptr, cons
         return;
     }
     float4* co = smem + (size_t)w * maxk * 2;
-    const int b = rowptr[v], k = rowptr[v + 1] - b;
-    if (k <= 0 || k > maxk) return;
     const float4 c0 = pos[v];
     float sx, sy, sz;
     int ex;
-    if (!tet_setup<TET_LEARNED_KEEP>(pos, hf, b, k, c0, lane, co, sx, sy, sz, ex)) return;
+    float4* scratch = smem + (size_t)TET_WARPS * maxk * 2 + w * 32;
+    const int k = tet_setup(pos, rowptr, hf, ring, v, maxk, c0, lane, co, scratch, sx, sy, sz, ex);
+    if (k == 0) return;
     const float q0 = tet_key_min(co, k, 0.f, 0.f, 0.f, lane);
     // proposal in scaled local coordinates (the features were divided by mm = max(sx, sy, sz) 2^ex)
     const float mms = fmaxf(sx, fmaxf(sy, sz));
@@ -789,7 +549,7 @@ k_dmo_tet_learned(float4* __restrict__ pos, const int* __restrict__ rowptr, cons
             pos[v] = tet_unscale(c0, cx, cy, cz, ex);
             atomicAdd(&counters[0], 1ull);
         }
-        if (dirty) tet_mark_ring(hf, b, k, lane, dirty);
+        if (dirty) tet_mark_ring(hf, rowptr[v], k, lane, dirty);
         return;
     }
     // the proposal did not raise the ring minimum: queue the vertex for the plain search
@@ -1310,8 +1070,8 @@ void launch_dmo_hex(const Mesh& m, const DmoLaunch& L, cudaStream_t s) {
     VSDMO_CHECK_LAUNCH();
 }
 
-// coefficients of every warp's ring, then every warp's survivor list
-size_t tet_smem_bytes(int maxk) { return (size_t)TET_WARPS * maxk * 2 * sizeof(float4) + (size_t)TET_WARPS * TET_LIST * sizeof(int); }
+// coefficients of every warp's ring, then every warp's search scratch
+size_t tet_smem_bytes(int maxk) { return (size_t)TET_WARPS * (maxk * 2 * sizeof(float4) + TS_WARP_BYTES); }
 
 // Raises the dynamic shared-memory limit of the grid-search kernels (called once per
 // optimiser, outside any stream capture, on the current device).
@@ -1320,7 +1080,7 @@ void prepare_dmo_kernels() {
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_tri2d, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     TRI_WARPS * TRI_MAX_RING * 2 * (int)sizeof(float4)));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_tet_learned, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    TET_WARPS * TET_MAX_RING * 2 * (int)sizeof(float4)));
+                                    TET_WARPS * (TET_MAX_RING * 2 + 32) * (int)sizeof(float4)));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_tet_list, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)tet_smem_bytes(TET_MAX_RING)));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_hex, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1329,14 +1089,14 @@ void prepare_dmo_kernels() {
 int dmo_tri2d_max_ring() { return TRI_MAX_RING; }
 int quality_stats_blocks() { return QS_BLOCKS; }
 
-void launch_dmo_tet(const Mesh& m, const DmoLaunch& L, cudaStream_t s, uint8_t* dirty,
+void launch_dmo_tet(const Mesh& m, const DmoLaunch& L, const TetRingTable& ring, cudaStream_t s, uint8_t* dirty,
                     unsigned long long* skipped) {
     const int n = L.v1 - L.v0;
     if (n <= 0) return;
     const int maxk = m.maxTets;
     const size_t smem = tet_smem_bytes(maxk);
     k_dmo_tet<<<(n + TET_WARPS - 1) / TET_WARPS, TET_WARPS * 32, smem, s>>>(
-        m.pos.p, m.hf_rowptr.p, m.hf.p, L.v0, L.v1, L.grid_scale, L.depth, maxk, dirty, skipped);
+        m.pos.p, m.hf_rowptr.p, m.hf.p, ring, L.v0, L.v1, L.grid_scale, L.depth, maxk, dirty, skipped);
     VSDMO_CHECK_LAUNCH();
 }
 
@@ -1358,9 +1118,9 @@ void launch_mark_rings(const Mesh& m, int v0, int v1, uint8_t* dirty, cudaStream
     VSDMO_CHECK_LAUNCH();
 }
 
-void launch_tet_neighbours(const Mesh& m, int v0, int v1, int* nb, int* nbn, cudaStream_t s) {
+void launch_tet_rings(const Mesh& m, int v0, int v1, int* nb, int* nbn, uint16_t* corner, cudaStream_t s) {
     if (v1 <= v0) return;
-    k_tet_neighbours<<<grid_for(v1 - v0, 128), 128, 0, s>>>(m.hf_rowptr.p, m.hf.p, v0, v1, nb, nbn);
+    k_tet_rings<<<grid_for(32L * (v1 - v0), 128), 128, 0, s>>>(m.hf_rowptr.p, m.hf.p, v0, v1, nb, nbn, corner);
     VSDMO_CHECK_LAUNCH();
 }
 
@@ -1378,21 +1138,21 @@ void launch_tet_targets(const Mesh& m, int v0, int v1, const float* scale, const
     VSDMO_CHECK_LAUNCH();
 }
 
-void launch_dmo_tet_learned(const Mesh& m, const DmoLaunch& L, const float* Y, int ldy, int rn, int rdepth,
-                            float rscale, unsigned long long* counters, uint8_t* dirty, int* fb_list, int* fb_count,
+void launch_dmo_tet_learned(const Mesh& m, const DmoLaunch& L, const TetRingTable& ring, const float* Y, int ldy,
+                            int rn, int rdepth, float rscale, unsigned long long* counters, uint8_t* dirty, int* fb_list, int* fb_count,
                             cudaStream_t s) {
     const int n = L.v1 - L.v0;
     if (n <= 0) return;
     const int maxk = m.maxTets;
-    const size_t smem = (size_t)TET_WARPS * maxk * 2 * sizeof(float4);
+    const size_t smem = (size_t)TET_WARPS * (maxk * 2 + 32) * sizeof(float4);
     k_dmo_tet_learned<<<(n + TET_WARPS - 1) / TET_WARPS, TET_WARPS * 32, smem, s>>>(
-        m.pos.p, m.hf_rowptr.p, m.hf.p, L.v0, L.v1, L.grid_scale, maxk, Y, ldy, rn, rdepth, rscale, counters, dirty,
+        m.pos.p, m.hf_rowptr.p, m.hf.p, ring, L.v0, L.v1, L.grid_scale, maxk, Y, ldy, rn, rdepth, rscale, counters, dirty,
         fb_list, fb_count);
     VSDMO_CHECK_LAUNCH();
     // fallback: the plain search over the queued vertices, a fixed grid striding over the list
-    const int blocks = std::min((n + TET_WARPS - 1) / TET_WARPS, 148 * 4);
-    k_dmo_tet_list<<<blocks, TET_WARPS * 32, tet_smem_bytes(maxk), s>>>(m.pos.p, m.hf_rowptr.p, m.hf.p, fb_list, fb_count,
-                                                                        L.grid_scale, L.depth, maxk, dirty, counters + 2);
+    const int blocks = std::min((n + TET_WARPS - 1) / TET_WARPS, 148 * TET_LIST_MIN_BLOCKS);
+    k_dmo_tet_list<<<blocks, TET_WARPS * 32, tet_smem_bytes(maxk), s>>>(m.pos.p, m.hf_rowptr.p, m.hf.p, ring, fb_list,
+                                                                        fb_count, L.grid_scale, L.depth, maxk, dirty, counters + 2);
     VSDMO_CHECK_LAUNCH();
 }
 

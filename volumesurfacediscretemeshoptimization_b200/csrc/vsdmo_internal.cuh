@@ -169,10 +169,17 @@ struct DmoLaunch {
     float grid_scale;
     int depth;
 };
+// Ring table of the inner vertices of a tet mesh (k_tet_rings), rows of 32 from vertex base on
+struct TetRingTable {
+    static constexpr uint16_t NONE = 0xffff, LARGE = 0xfffe;
+    const int* nb;            // distinct ring vertices, unused places hold the vertex itself
+    const uint16_t* corner;   // the tets' corners as places in that row: a | b << 5 | c << 10
+    int base;
+};
 // dirty (optional): active-set flags [nV], see k_dmo_tet; skipped (optional): skip counter
 void launch_mark_rings(const Mesh& m, int v0, int v1, uint8_t* dirty, cudaStream_t s);
-void launch_dmo_tet(const Mesh& m, const DmoLaunch& L, cudaStream_t s, uint8_t* dirty = nullptr,
-                    unsigned long long* skipped = nullptr);
+void launch_dmo_tet(const Mesh& m, const DmoLaunch& L, const TetRingTable& ring, cudaStream_t s,
+                    uint8_t* dirty = nullptr, unsigned long long* skipped = nullptr);
 void launch_dmo_tri2d(const Mesh& m, const DmoLaunch& L, cudaStream_t s);
 int dmo_tet_max_ring();      // largest halfface row the tet kernel accepts
 void launch_dmo_hex(const Mesh& m, const DmoLaunch& L, cudaStream_t s);
@@ -181,9 +188,9 @@ void prepare_dmo_kernels();
 int dmo_tri2d_max_ring();    // largest halfedge row the 2D kernel accepts
 
 // ---- learned proposal (tet; dmo_kernels.cu) ----------------------------------------------------
-// distinct ring vertices of [v0, v1) (first occurrence in the halfface row, at most 32):
-// nb [(v - v0) * 32 + a], nbn [v - v0]
-void launch_tet_neighbours(const Mesh& m, int v0, int v1, int* nb, int* nbn, cudaStream_t s);
+// ring table of [v0, v1): distinct ring vertices (first occurrence in the halfface row, at most 32)
+// nb [(v - v0) * 32 + a], their number nbn [v - v0], corner triples corner [(v - v0) * 32 + t]
+void launch_tet_rings(const Mesh& m, int v0, int v1, int* nb, int* nbn, uint16_t* corner, cudaStream_t s);
 // network inputs of vertices [v0, v1) from the neighbour table (whose first vertex is nb_base):
 // FP32 rows [n x 96] and / or BF16 packed operand rows, ring extent and old position per
 // vertex (any output may be null)
@@ -196,8 +203,8 @@ void launch_tet_targets(const Mesh& m, int v0, int v1, const float* scale, const
 // counters [4], dirty: optional active-set flags
 // fb_list [colour size] / fb_count [2]: the fallback queue (its length and a block counter,
 // both zero between launches: the fallback kernel leaves them so)
-void launch_dmo_tet_learned(const Mesh& m, const DmoLaunch& L, const float* Y, int ldy, int rn, int rdepth,
-                            float rscale, unsigned long long* counters, uint8_t* dirty, int* fb_list, int* fb_count,
+void launch_dmo_tet_learned(const Mesh& m, const DmoLaunch& L, const TetRingTable& ring, const float* Y, int ldy,
+                            int rn, int rdepth, float rscale, unsigned long long* counters, uint8_t* dirty, int* fb_list, int* fb_count,
                             cudaStream_t s);
 
 // ---- surface DMO (surf_kernels.cu) ----------------------------------------------------------
