@@ -29,7 +29,7 @@
 #include "tc_gemm.cuh"
 #include "angle_metrics.cuh"
 #include "tet_search.cuh"
-#include "hex_key.cuh"
+#include "hex_search.cuh"
 #include "hex_cond.cuh"
 #include "quad_cond.cuh"
 #include <cfloat>
@@ -562,155 +562,67 @@ k_dmo_tet_learned(float4* __restrict__ pos, const int* __restrict__ rowptr, cons
 
 // ---- hexahedra ------------------------------------------------------------------------------------
 // k_optimizeHierarchicalInnerHex<128> (dmo/DMOHexImplCub.h:21-137) with shapeMetricHex
-// (dmo/DMOQualityHex.h:54-71). With the candidate p as corner 0 of a halfhex, sub-tets 1, 2, 3
-// and 6 of the metric do not depend on p, and sub-tets 0, 4, 5, 7, 8 have a determinant affine
-// in p and a Frobenius term quadratic in p; each halfhex is staged as 43 coefficients (the
-// constant part's key and 5 x {g, c, m, C}). min_j cbrt(s^2) / A is compared through s^2 / A^3
-// as a fraction. The reference block's 128 threads of 4 candidates, whose maxima carry across
-// levels, are kept as one block of 128 threads per vertex: thread t takes candidates
-// 4t .. 4t+3 (x = 4 (t & 1) .. +3, y = (t >> 1) & 7, z = t >> 4). (The colour classes of a hex
-// mesh hold ~600-1,200 vertices: one warp per vertex left ~8 warps per SM.)
-constexpr int HEX_THREADS = 128;
+// (dmo/DMOQualityHex.h:54-71): one warp per vertex stages the halfhexes' coefficients (hex_key.cuh)
+// and runs the filtered search of hex_search.cuh. A block of 128 threads that judged all 512
+// candidates by the whole ring took 2.14 ms per iteration of the 32^3 cube (10 iterations), this one
+// takes 0.50 ms: 17 colour classes of up to 2,600 vertices, one wave each, bound by one search's latency.
 constexpr int HEX_MAX_RING = 64;
+constexpr int HEX_MIN_BLOCKS = 20;   // 96 registers
 
-__global__ void __launch_bounds__(HEX_THREADS)
+// coefficients, then the corners of the setup or the search's scratch and item list
+size_t hex_smem_bytes(int maxk) {
+    return (size_t)maxk * HEX_CO * sizeof(float) +
+           std::max((size_t)TS_WARP_BYTES + 6 * maxk * sizeof(unsigned short), (size_t)7 * maxk * sizeof(float4));
+}
+
+__global__ void __launch_bounds__(32, HEX_MIN_BLOCKS)
 k_dmo_hex(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ hh, int v0,
           float grid_scale, int depth, int maxk) {
     extern __shared__ float4 smem[];
-    __shared__ float red[6][HEX_THREADS / 32];
-    __shared__ float s_k[HEX_THREADS / 32];
-    __shared__ int s_i[HEX_THREADS / 32];
-    __shared__ float s_win[3];
-    __shared__ float s_qlast;
-    __shared__ int s_czero;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int lane = threadIdx.x;
     const int v = v0 + blockIdx.x;
     float* co = reinterpret_cast<float*>(smem);
+    float4* corner = smem + maxk * (HEX_CO / 4);
     const int b = rowptr[v], k = rowptr[v + 1] - b;
     if (k <= 0 || k > maxk) return;
     const float4 c0 = pos[v];
     // per-axis largest (scale) and smallest (grid extent, DMOHexImplCub.h:49-68) ring distance
     float mx0 = 0.f, mx1 = 0.f, mx2 = 0.f, mn0 = FLT_MAX, mn1 = FLT_MAX, mn2 = FLT_MAX;
-    for (int idx = t; idx < 7 * k; idx += HEX_THREADS) {
+    for (int idx = lane; idx < 7 * k; idx += 32) {
         const int h = idx / 7, c = idx % 7;
         const int4 q = hh[2 * (b + h) + (c >> 2)];
         const int cc = c & 3;
-        const int u = cc == 0 ? q.x : (cc == 1 ? q.y : (cc == 2 ? q.z : q.w));
-        const float4 p = pos[u];
-        const float d0 = fabsf(p.x - c0.x), d1 = fabsf(p.y - c0.y), d2 = fabsf(p.z - c0.z);
-        mx0 = fmaxf(mx0, d0); mx1 = fmaxf(mx1, d1); mx2 = fmaxf(mx2, d2);
-        mn0 = fminf(mn0, d0); mn1 = fminf(mn1, d1); mn2 = fminf(mn2, d2);
+        const float4 p = pos[cc == 0 ? q.x : (cc == 1 ? q.y : (cc == 2 ? q.z : q.w))];
+        const float4 d = make_float4(p.x - c0.x, p.y - c0.y, p.z - c0.z, 0.f);
+        corner[idx] = d;
+        mx0 = fmaxf(mx0, fabsf(d.x)); mx1 = fmaxf(mx1, fabsf(d.y)); mx2 = fmaxf(mx2, fabsf(d.z));
+        mn0 = fminf(mn0, fabsf(d.x)); mn1 = fminf(mn1, fabsf(d.y)); mn2 = fminf(mn2, fabsf(d.z));
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        mx0 = fmaxf(mx0, __shfl_xor_sync(FULL, mx0, o)); mx1 = fmaxf(mx1, __shfl_xor_sync(FULL, mx1, o));
-        mx2 = fmaxf(mx2, __shfl_xor_sync(FULL, mx2, o)); mn0 = fminf(mn0, __shfl_xor_sync(FULL, mn0, o));
-        mn1 = fminf(mn1, __shfl_xor_sync(FULL, mn1, o)); mn2 = fminf(mn2, __shfl_xor_sync(FULL, mn2, o));
-    }
-    if (lane == 0) { red[0][w] = mx0; red[1][w] = mx1; red[2][w] = mx2; red[3][w] = mn0; red[4][w] = mn1; red[5][w] = mn2; }
-    if (t == 0) s_czero = 0;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < HEX_THREADS / 32; ++i) {
-        mx0 = fmaxf(mx0, red[0][i]); mx1 = fmaxf(mx1, red[1][i]); mx2 = fmaxf(mx2, red[2][i]);
-        mn0 = fminf(mn0, red[3][i]); mn1 = fminf(mn1, red[4][i]); mn2 = fminf(mn2, red[5][i]);
-    }
+    mx0 = redux_max(mx0); mx1 = redux_max(mx1); mx2 = redux_max(mx2);
+    mn0 = redux_min(mn0); mn1 = redux_min(mn1); mn2 = redux_min(mn2);
     const float mm = fmaxf(mx0, fmaxf(mx1, mx2));
-    if (!(mm > 0.f) || !(mm < FLT_MAX)) return;   // uniform over the block
+    if (!(mm > 0.f) || !(mm < FLT_MAX)) return;
     int ex;
     (void)frexpf(mm, &ex);
     const float p2 = exp2_exact(-ex);
     const float es = ldexpf(HEX_EPS, -3 * ex), ea = ldexpf(HEX_EPS, -2 * ex);
-    for (int h = t; h < k; h += HEX_THREADS) {
-        const int4 qa = hh[2 * (b + h)], qb = hh[2 * (b + h) + 1];
-        const int us[7] = { qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z };
+    __syncwarp();
+    for (int h = lane; h < k; h += 32) {
         float r[7][3];
 #pragma unroll
         for (int c = 0; c < 7; ++c) {
-            const float4 p = pos[us[c]];
-            r[c][0] = scale2(p.x - c0.x, p2, -ex); r[c][1] = scale2(p.y - c0.y, p2, -ex); r[c][2] = scale2(p.z - c0.z, p2, -ex);
+            const float4 d = corner[7 * h + c];
+            r[c][0] = scale2(d.x, p2, -ex); r[c][1] = scale2(d.y, p2, -ex); r[c][2] = scale2(d.z, p2, -ex);
         }
         hex_coeffs(r, es, ea, co + HEX_CO * h);
-        if (co[HEX_CO * h + 2] != 0.f) s_czero = 1;
     }
-    __syncthreads();
-    const float sx = scale2(mn0, p2, -ex), sy = scale2(mn1, p2, -ex), sz = scale2(mn2, p2, -ex);
-    // ring-wide: any constant part zero makes every candidate's key zero
-    const bool czero = s_czero != 0;
-    const int ci = 4 * (t & 1), cj = (t >> 1) & 7, ck = t >> 4;
-    float qMax = -FLT_MAX, pX = 0.f, pY = 0.f, pZ = 0.f;
-    float dx = 0.f, dy = 0.f, dz = 0.f;
-    float ds = grid_scale;
-    float qWin = -FLT_MAX;
-    for (int level = 0; level < depth; ++level) {
-        const float Sx = ds * sx, Sy = ds * sy, Sz = ds * sz;
-        // the key at the current position: one warp computes it while the others search
-        if (w == 0) {
-            const float q = hex_key1(co, k, dx, dy, dz, es, ea);
-            if (lane == 0) s_qlast = q;
-        }
-        const float z = fmaf(grid_offset(ck), Sz, dz);
-        const float y = fmaf(grid_offset(cj), Sy, dy);
-        float x[4], t1x[4], t3x[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { x[i] = fmaf(grid_offset(ci + i), Sx, dx); t1x[i] = x[i] * x[i]; t3x[i] = (3.f * x[i]) * x[i]; }
-        const float t1z = z * z, t3z = (3.f * z) * z;
-        const float t1y = y * y, t3y = (3.f * y) * y;
-        float N[4], D[4];
-        bool zr[4];
-        {
-            const float n0 = co[0], d0 = co[1];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { N[i] = n0; D[i] = d0; zr[i] = czero; }
-        }
-        for (int h = 0; h < k; ++h) {
-            const float* c = co + HEX_CO * h;
-            if (h > 0) {
-                const float cn = c[0], cd = c[1];
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (cn * D[i] < N[i] * cd) { N[i] = cn; D[i] = cd; }
-            }
-#pragma unroll
-            for (int j = 0; j < 5; ++j) {
-                const float* q = c + 3 + 8 * j;
-                const bool a3 = (j == 1 || j == 4);
-                const float sY = fmaf(q[1], y, fmaf(q[2], z, q[3]));
-                const float aY = (q[7] + fmaf(q[6], z, a3 ? t3z : t1z)) + fmaf(q[5], y, a3 ? t3y : t1y);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float sd = fmaf(q[0], x[i], sY);
-                    const float A = aY + fmaf(q[4], x[i], a3 ? t3x[i] : t1x[i]);
-                    if (sd < es || A < ea) { zr[i] = true; continue; }
-                    const float num = sd * sd, den = (A * A) * A;
-                    if (num * D[i] < N[i] * den) { N[i] = num; D[i] = den; }
-                }
-            }
-        }
-        // the thread's maximum carries across levels (candidates in index order, strict >)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float key = zr[i] ? 0.f : N[i] / D[i];
-            if (key > qMax) { qMax = key; pX = x[i]; pY = y; pZ = z; }
-        }
-        // block arg-max, the lowest thread on ties
-        float bk = qMax;
-        int bi = t;
-        warp_argmax(bk, bi);
-        if (lane == 0) { s_k[w] = bk; s_i[w] = bi; }
-        __syncthreads();
-        bk = s_k[0]; bi = s_i[0];
-#pragma unroll
-        for (int i = 1; i < HEX_THREADS / 32; ++i)
-            if (s_k[i] > bk || (s_k[i] == bk && s_i[i] < bi)) { bk = s_k[i]; bi = s_i[i]; }
-        if (t == bi) { s_win[0] = pX; s_win[1] = pY; s_win[2] = pZ; }
-        __syncthreads();
-        if (s_qlast < bk) { dx = s_win[0]; dy = s_win[1]; dz = s_win[2]; }
-        qWin = bk;
-        ds = ds * (2.0f / 7.0f);
-        __syncthreads();   // s_k / s_win are rewritten by the next level
-    }
-    if (t == 0 && hex_key1(co, k, 0.f, 0.f, 0.f, es, ea) < qWin) pos[v] = tet_unscale(c0, dx, dy, dz, ex);
+    __syncwarp();
+    const HexItems ring{co, k, es, ea, nullptr, 0};
+    float* scratch = reinterpret_cast<float*>(corner);
+    float dx, dy, dz;
+    const bool moved = hex_plain_search(ring, scratch, reinterpret_cast<unsigned short*>(scratch + TS_WARP_BYTES / 4), scale2(mn0, p2, -ex), scale2(mn1, p2, -ex),
+                                        scale2(mn2, p2, -ex), grid_scale, depth, lane, dx, dy, dz);
+    if (moved && lane == 0) pos[v] = tet_unscale(c0, dx, dy, dz, ex);
 }
 
 // ---- flat triangles ---------------------------------------------------------------------------
@@ -1065,8 +977,7 @@ void launch_dmo_hex(const Mesh& m, const DmoLaunch& L, cudaStream_t s) {
     const int n = L.v1 - L.v0;
     if (n <= 0) return;
     const int maxk = m.maxTets;
-    const size_t smem = (size_t)maxk * HEX_CO * sizeof(float);
-    k_dmo_hex<<<n, HEX_THREADS, smem, s>>>(m.pos.p, m.hf_rowptr.p, m.hh.p, L.v0, L.grid_scale, L.depth, maxk);
+    k_dmo_hex<<<n, 32, hex_smem_bytes(maxk), s>>>(m.pos.p, m.hf_rowptr.p, m.hh.p, L.v0, L.grid_scale, L.depth, maxk);
     VSDMO_CHECK_LAUNCH();
 }
 
@@ -1084,7 +995,7 @@ void prepare_dmo_kernels() {
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_tet_list, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)tet_smem_bytes(TET_MAX_RING)));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_hex, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    HEX_MAX_RING * HEX_CO * (int)sizeof(float)));
+                                    (int)hex_smem_bytes(HEX_MAX_RING)));
 }
 int dmo_tri2d_max_ring() { return TRI_MAX_RING; }
 int quality_stats_blocks() { return QS_BLOCKS; }
