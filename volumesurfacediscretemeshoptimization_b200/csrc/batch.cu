@@ -14,13 +14,14 @@
 //     vertices at a time) -- chosen per size bucket by the autotuner below;
 //   * positions of vertices other warps may have moved during the launch are read through L2
 //     (__ldcg); moves are published with __threadfence before the completion count;
-//   * a second kernel reduces each mesh's element qualities (min, sum, monotonicity count).
-// One iteration = memset of the counters + the two kernels, captured once as a CUDA graph and
+//   * two more reduce each mesh's element qualities (min, sum, monotonicity count), first per chunk.
+// One iteration = memset of the counters + these kernels, captured once as a CUDA graph and
 // replayed. The grid search is the 2D search of k_optimizeHierarchical2DFlat
 // (dmo/DMOTriFlatImplCub.h:24-152) generalised to N candidates per axis (oracle/or_flat.c
 // restates it); with N = 8, 3 levels it is the reference kernel.
 #include "vsdmo_internal.cuh"
 #include "batch.cuh"
+#include "flat_search.cuh"
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -31,8 +32,12 @@ namespace vsdmo {
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int BCO = 9;                 // coefficient floats per ring element
 constexpr int BATCH_WARPS = 8;
+// vertices of a colour class from which on four vertices share a warp: below, a warp per vertex is the
+// shorter chain and fits in one wave (flat triangles / quads, ms per iteration, packed against not:
+// 64^2 (classes of 550) 0.049 / 0.064 : 0.042 / 0.063; 128^2 (2,300) 0.053 / 0.065 : 0.057 / 0.079; 500^2
+// (35,000) 0.167 / 0.199 : 0.407 / 0.575)
+constexpr int FLAT_PACKED_MIN = 2048;
 constexpr unsigned long long BWAIT_NS = 1000000000ull;
 // limit of a colour-class wait: BWAIT_NS unless the test-only vsdmo_debug_set_wait_limit_ns
 // lowered it to make waits expire
@@ -43,69 +48,6 @@ __device__ __forceinline__ unsigned long long bnow() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-
-__device__ __forceinline__ float bexp2(int e) { return (e >= -126 && e <= 127) ? __int_as_float((e + 127) << 23) : 0.f; }
-__device__ __forceinline__ float bscale(float x, float p, int e) { return p != 0.f ? x * p : ldexpf(x, e); }
-
-template <bool COHERENT>
-__device__ __forceinline__ float4 ldpos(const float4* p) {
-    if (COHERENT) return __ldcg(p);
-    return *p;
-}
-
-// triangle (p, a, b): A = K0 x + K1 y + K2, L = K5 + K3 x + K4 y + 2 |p|^2
-__device__ __forceinline__ void btri_co(float ax, float ay, float bx, float by, float* K) {
-    const float ux = bx - ax, uy = by - ay;
-    K[0] = -uy; K[1] = ux;
-    K[2] = ax * uy - ay * ux;
-    K[3] = -2.0f * (ax + bx); K[4] = -2.0f * (ay + by);
-    K[5] = ((ax * ax + ay * ay) + (bx * bx + by * by)) + (ux * ux + uy * uy);
-}
-
-// quad (p, a, b, c): corner cross products c1 = K0 x + K1 y + K2, c2 = K3 x + K4 y + K5,
-// edge sum l = K8 + K6 x + K7 y + 2 |p|^2
-__device__ __forceinline__ void bquad_co(float ax, float ay, float bx, float by, float cx, float cy, float* K) {
-    const float e1x = bx - ax, e1y = by - ay;
-    const float fx = bx - cx, fy = by - cy;
-    const float gx = cx - bx, gy = cy - by;
-    K[0] = -e1y; K[1] = e1x; K[2] = e1y * ax - e1x * ay;
-    K[3] = fy; K[4] = -fx; K[5] = cy * fx - cx * fy;
-    K[6] = -2.0f * (ax + cx); K[7] = -2.0f * (ay + cy);
-    K[8] = (((ax * ax + ay * ay) + (e1x * e1x + e1y * e1y)) + (gx * gx + gy * gy)) + (cx * cx + cy * cy);
-}
-
-template <int FK>
-__device__ __forceinline__ float bkey(const float* co, int k, float x, float y) {
-    const float tx = (2.0f * x) * x, ty = (2.0f * y) * y;
-    float N = 0.f, D = 1.f;
-    if (FK == 3) {
-        float amin = 0.f;
-        for (int t = 0; t < k; ++t) {
-            const float* c = co + BCO * t;
-            const float A = fmaf(c[1], y, fmaf(c[0], x, c[2]));
-            const float L = (c[5] + fmaf(c[3], x, tx)) + fmaf(c[4], y, ty);
-            if (t == 0) { N = A; D = L; amin = A; continue; }
-            if (A * D < N * L) { N = A; D = L; }
-            amin = fminf(amin, A);
-        }
-        return amin < 0.f ? amin : N / D;
-    } else {
-        bool neg = false;
-        for (int t = 0; t < k; ++t) {
-            const float* c = co + BCO * t;
-            const float c1 = fmaf(c[1], y, fmaf(c[0], x, c[2]));
-            const float c2 = fmaf(c[4], y, fmaf(c[3], x, c[5]));
-            const float l = (c[8] + fmaf(c[6], x, tx)) + fmaf(c[7], y, ty);
-            neg |= (c1 < 0.f || c2 < 0.f);
-            const float num = c1 + c2;
-            if (t == 0) { N = num; D = l; continue; }
-            if (num * D < N * l) { N = num; D = l; }
-        }
-        return neg ? -1.f : N / D;
-    }
-}
-
-__device__ __forceinline__ float boffset(int i, int n) { return (float)(n - 1 - 2 * i) / (float)(n - 1); }
 
 // One vertex searched by a group of L lanes (gl = lane in group, gbase = first lane of the
 // group in the warp). co: the group's shared-memory coefficient buffer (maxk x BCO floats).
@@ -201,15 +143,39 @@ k_dmo_flat(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4*
     flat_vertex<FK, false>(pos, rowptr, he, v, gs, nq, depth, co, maxk, gl, L, gmask);
 }
 
+// the same for four vertices per warp (8 x 8 candidates, rings of up to F8_MAX_RING)
+constexpr int F8_WARPS = 4;
+template <int FK>
+__global__ void __launch_bounds__(F8_WARPS * 32)
+k_dmo_flat8(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ he, int v0, int v1,
+            float gs, int depth, int maxk) {
+    extern __shared__ float4 f8sm[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 3;
+    float* sm = reinterpret_cast<float*>(f8sm) + (size_t)(w * 4 + g) * f8_group_floats(maxk);
+    const int base = v0 + (blockIdx.x * F8_WARPS + w) * 4;
+    if (base >= v1) return;
+    flat_search8<FK, false>(pos, rowptr, he, base + g, base + g < v1, gs, depth, sm, maxk, lane);
+}
+
 // ---- the persistent batched iteration -----------------------------------------------------------
-__global__ void __launch_bounds__(BATCH_WARPS * 32)
+// floats of shared memory per warp: up to 4 groups of either search
+__host__ __device__ constexpr int batch_warp_floats(int maxk) {
+    return maxk > F8_MAX_RING || maxk * BCO > f8_group_floats(maxk) ? 4 * maxk * BCO : 4 * f8_group_floats(maxk);
+}
+
+// PACKED: every mesh is searched four vertices per warp (the other search stays out of the kernel:
+// with both in one, half the stalls were instruction fetches)
+// Registers: four blocks per SM at 64 (48 bytes of spills) against three at 80 and two at 96: 2.28 / 2.33
+// / 2.80 ms per iteration of 256 meshes.
+template <bool PACKED>
+__global__ void __launch_bounds__(BATCH_WARPS * 32, 4)
 k_batch_iter(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ he,
              const BatchItem* __restrict__ items, int n_items, const BatchMeshDev* __restrict__ meshes,
              const int* __restrict__ csize, int* __restrict__ done, int* __restrict__ head, int maxk, float gs,
              int* __restrict__ err) {
-    extern __shared__ float bsm[];
+    extern __shared__ float4 bsm4[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float* wco = bsm + (size_t)w * 4 * maxk * BCO;   // up to 4 groups per warp
+    float* wco = reinterpret_cast<float*>(bsm4) + (size_t)w * batch_warp_floats(maxk);
     while (true) {
         int idx = 0;
         if (lane == 0) idx = atomicAdd(head, 1);
@@ -242,14 +208,23 @@ k_batch_iter(float4* __restrict__ pos, const int* __restrict__ rowptr, const int
                 continue;
             }
         }
-        const int L = mh.lanes, groups = 32 / L, g = lane / L, gl = lane % L;
-        const unsigned gmask = L == 32 ? FULL : (((1u << L) - 1u) << (g * L));
-        float* co = wco + (size_t)g * maxk * BCO;
-        for (int base = it.v0; base < it.v1; base += groups) {
-            const int v = base + g;
-            if (v < it.v1) {
-                if (mh.fk == 3) flat_vertex<3, true>(pos, rowptr, he, v, gs, mh.nq, mh.depth, co, maxk, gl, L, gmask);
-                else flat_vertex<4, true>(pos, rowptr, he, v, gs, mh.nq, mh.depth, co, maxk, gl, L, gmask);
+        if (PACKED || mh.packed) {
+            float* sm = wco + (size_t)(lane >> 3) * f8_group_floats(maxk);
+            for (int base = it.v0; base < it.v1; base += 4) {
+                const int v = base + (lane >> 3);
+                if (mh.fk == 3) flat_search8<3, true>(pos, rowptr, he, v, v < it.v1, gs, mh.depth, sm, maxk, lane);
+                else flat_search8<4, true>(pos, rowptr, he, v, v < it.v1, gs, mh.depth, sm, maxk, lane);
+            }
+        } else if constexpr (!PACKED) {
+            const int L = mh.lanes, groups = 32 / L, g = lane / L, gl = lane % L;
+            const unsigned gmask = L == 32 ? FULL : (((1u << L) - 1u) << (g * L));
+            float* co = wco + (size_t)g * maxk * BCO;
+            for (int base = it.v0; base < it.v1; base += groups) {
+                const int v = base + g;
+                if (v < it.v1) {
+                    if (mh.fk == 3) flat_vertex<3, true>(pos, rowptr, he, v, gs, mh.nq, mh.depth, co, maxk, gl, L, gmask);
+                    else flat_vertex<4, true>(pos, rowptr, he, v, gs, mh.nq, mh.depth, co, maxk, gl, L, gmask);
+                }
             }
         }
         // publish: every writer fences its moves before lane 0 counts the chunk as done
@@ -279,21 +254,27 @@ __device__ __forceinline__ float bq_quad(float4 p0, float4 p1, float4 p2, float4
     return (2.f * (c1 + c2)) / l;
 }
 
+// chunk c: elements [first, first + QCHUNK) of one mesh; one block per chunk, a mesh's partials are
+// folded in chunk order by k_batch_quality_fold (one block per mesh took 410 us for meshes of up to
+// 100,000 elements)
+constexpr int QCHUNK = 2048;
+
 __global__ void __launch_bounds__(256)
 k_batch_quality(const float4* __restrict__ pos, const int* __restrict__ el, const BatchMeshDev* __restrict__ meshes,
-                BatchStats* __restrict__ stats, int n_meshes, int* __restrict__ iter, int init) {
+                const int2* __restrict__ chunks, const BatchStats* __restrict__ stats, int n_meshes,
+                const int* __restrict__ iter, int init, BatchStats* __restrict__ part) {
     __shared__ float smin[8];
     __shared__ double ssum[8];
     __shared__ int sfail[8];
-    const int m = blockIdx.x;
-    const BatchMeshDev mh = meshes[m];
-    const int it = *iter;
-    const float last = init ? -FLT_MAX : stats[(size_t)it * n_meshes + m].min_q;
+    const int2 ch = chunks[blockIdx.x];
+    const BatchMeshDev mh = meshes[ch.x];
+    const float last = init ? -FLT_MAX : stats[(size_t)*iter * n_meshes + ch.x].min_q;
     const float tol = 1e-6f * fmaxf(fabsf(last), 1e-30f);
     float mn = FLT_MAX;
     double sm = 0.0;
     int fl = 0;
-    for (int e = threadIdx.x; e < mh.n_elems; e += 256) {
+    const int end = min(ch.y + QCHUNK, mh.n_elems);
+    for (int e = ch.y + threadIdx.x; e < end; e += 256) {
         const int* t = el + mh.el_off + (long)mh.fk * e;
         const float q = mh.fk == 3 ? bq_tri(pos[t[0]], pos[t[1]], pos[t[2]]) : bq_quad(pos[t[0]], pos[t[1]], pos[t[2]], pos[t[3]]);
         mn = fminf(mn, q);
@@ -314,13 +295,29 @@ k_batch_quality(const float4* __restrict__ pos, const int* __restrict__ el, cons
         double s = ssum[0];
         int f = sfail[0];
         for (int i = 1; i < 8; ++i) { a = fminf(a, smin[i]); s += ssum[i]; f += sfail[i]; }
-        const int slot = init ? 0 : it + 1;
-        BatchStats& o = stats[(size_t)slot * n_meshes + m];
+        BatchStats o;
         o.min_q = a; o.sum_q = s; o.fail_count = f;
+        part[blockIdx.x] = o;
     }
 }
 
-__global__ void k_batch_iter_advance(int* iter) { *iter += 1; }
+// one thread per mesh; mesh m's chunks are [first[m], first[m + 1]). A single block, so that the
+// iteration count advances after every thread has read it.
+__global__ void __launch_bounds__(1024)
+k_batch_quality_fold(const BatchStats* __restrict__ part, const int* __restrict__ first, BatchStats* __restrict__ stats,
+                     int n_meshes, int* __restrict__ iter, int init, int advance) {
+    const int it = *iter;
+    for (int m = threadIdx.x; m < n_meshes; m += 1024) {
+        float a = FLT_MAX;
+        double s = 0.0;
+        int f = 0;
+        for (int c = first[m]; c < first[m + 1]; ++c) { a = fminf(a, part[c].min_q); s += part[c].sum_q; f += part[c].fail_count; }
+        BatchStats& o = stats[(size_t)(init ? 0 : it + 1) * n_meshes + m];
+        o.min_q = a; o.sum_q = s; o.fail_count = f;
+    }
+    __syncthreads();
+    if (advance && threadIdx.x == 0) *iter = it + 1;
+}
 
 // positions in the input numbering <-> batch numbering
 __global__ void k_batch_pack(const float4* __restrict__ pos, const int* __restrict__ map, long n, float* __restrict__ out) {
@@ -353,6 +350,8 @@ __global__ void k_batch_concat_int(const int* in, int n, int off, int* out) {
 
 // ---- host ---------------------------------------------------------------------------------------------
 size_t flat_smem(int maxk, int groups) { return (size_t)BATCH_WARPS * groups * maxk * BCO * sizeof(float); }
+size_t flat8_smem(int maxk) { return (size_t)F8_WARPS * 4 * f8_group_floats(maxk) * sizeof(float); }
+size_t batch_smem(int maxk) { return (size_t)BATCH_WARPS * batch_warp_floats(maxk) * sizeof(float); }
 
 int flat_max_ring() { return 64; }
 
@@ -360,9 +359,13 @@ void prepare_flat_kernels() {
     static bool done = false;
     if (done) return;
     const int mx = (int)flat_smem(flat_max_ring(), 4);
+    const int bmx = (int)std::max(batch_smem(flat_max_ring()), batch_smem(F8_MAX_RING));
+    VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat8<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)flat8_smem(F8_MAX_RING)));
+    VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat8<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)flat8_smem(F8_MAX_RING)));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    VSDMO_CUDA(cudaFuncSetAttribute(k_batch_iter, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    VSDMO_CUDA(cudaFuncSetAttribute(k_batch_iter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bmx));
+    VSDMO_CUDA(cudaFuncSetAttribute(k_batch_iter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bmx));
     done = true;
 }
 
@@ -382,6 +385,21 @@ void launch_dmo_flat(const Mesh& m, const DmoLaunch& L, int nq, int lanes, cudaS
         k_dmo_flat<3><<<blocks, BATCH_WARPS * 32, flat_smem(maxk, groups), s>>>(m.pos.p, m.he_rowptr.p, m.he.p, L.v0, L.v1,
                                                                                 L.grid_scale, nq, L.depth, lanes, maxk);
     VSDMO_CHECK_LAUNCH();
+}
+
+bool launch_dmo_flat_packed(const Mesh& m, const DmoLaunch& L, cudaStream_t s) {
+    const int n = L.v1 - L.v0, maxk = std::max(m.maxHE, 1);
+    if (n < FLAT_PACKED_MIN || maxk > F8_MAX_RING) return false;
+    prepare_flat_kernels();
+    const int blocks = (n + 4 * F8_WARPS - 1) / (4 * F8_WARPS);
+    if (m.fk == 4)
+        k_dmo_flat8<4><<<blocks, F8_WARPS * 32, flat8_smem(maxk), s>>>(m.pos.p, m.he_rowptr.p, m.he.p, L.v0, L.v1, L.grid_scale,
+                                                                       L.depth, maxk);
+    else
+        k_dmo_flat8<3><<<blocks, F8_WARPS * 32, flat8_smem(maxk), s>>>(m.pos.p, m.he_rowptr.p, m.he.p, L.v0, L.v1, L.grid_scale,
+                                                                       L.depth, maxk);
+    VSDMO_CHECK_LAUNCH();
+    return true;
 }
 
 Batch::~Batch() {
@@ -467,6 +485,18 @@ void Batch::build(const std::vector<MeshInput>& inputs, uint32_t seed) {
     err.zero();
     d_iter.alloc(1, stream);
     d_iter.zero();
+    std::vector<int2> ch;
+    std::vector<int> cf(M + 1, 0);
+    for (int i = 0; i < M; ++i) {
+        for (int e = 0; e < hm[i].nE; e += QCHUNK) ch.push_back(make_int2(i, e));
+        cf[i + 1] = (int)ch.size();
+    }
+    n_qchunks = (int)ch.size();
+    qchunks.alloc(ch.size(), stream);
+    qfirst.alloc(cf.size(), stream);
+    qpart.alloc(ch.size(), stream);
+    VSDMO_CUDA(cudaMemcpyAsync(qchunks.p, ch.data(), sizeof(int2) * ch.size(), cudaMemcpyHostToDevice, stream));
+    VSDMO_CUDA(cudaMemcpyAsync(qfirst.p, cf.data(), sizeof(int) * cf.size(), cudaMemcpyHostToDevice, stream));
     cfg.assign(M, BatchConfig{8, 3, 32});
     d_meshes.alloc(std::max(M, 1), stream);
     upload_meshes();
@@ -475,13 +505,37 @@ void Batch::build(const std::vector<MeshInput>& inputs, uint32_t seed) {
 
 int Batch::n_colors_total() const { return (int)csize.n; }
 
-void Batch::upload_meshes() {
+// Meshes searched four vertices per warp: 8 x 8 grids whose rings fit, where the caller asks for 8 lanes
+// per vertex or the colour classes of the meshes in `sel` (all when empty) together fill the device.
+void Batch::choose_packed(const std::vector<int>& sel) {
+    std::vector<int> ms = sel;
+    if (ms.empty())
+        for (int i = 0; i < (int)hm.size(); ++i) ms.push_back(i);
+    long free_v = 0;
+    int maxc = 1;
+    for (int i : ms) {
+        if (!hm[i].col.empty()) free_v += hm[i].col.back() - hm[i].col.front();
+        maxc = std::max(maxc, hm[i].n_colors);
+    }
+    const bool fills = free_v / maxc >= FLAT_PACKED_MIN;
+    all_packed = true;
+    for (int i : ms) {
+        hm[i].packed = cfg[i].nq == 8 && maxk <= F8_MAX_RING && (fills || cfg[i].lanes == 8);
+        all_packed = all_packed && hm[i].packed;
+    }
+}
+
+int Batch::chunk(int i) const { return 8 * (hm[i].packed ? 4 : 32 / cfg[i].lanes); }
+
+void Batch::upload_meshes(const std::vector<int>& sel) {
+    choose_packed(sel);
     std::vector<BatchMeshDev> dm(hm.size());
     for (size_t i = 0; i < hm.size(); ++i) {
         dm[i].fk = hm[i].fk;
         dm[i].nq = cfg[i].nq;
         dm[i].depth = cfg[i].depth;
         dm[i].lanes = cfg[i].lanes;
+        dm[i].packed = hm[i].packed ? 1 : 0;
         dm[i].col_base = hm[i].col_base;
         dm[i].n_elems = hm[i].nE;
         dm[i].el_off = hm[i].el_off;
@@ -509,7 +563,7 @@ void Batch::invalidate_graph() {
 }
 
 // Work items of the meshes in `sel` (all when empty) in colour-major order: every mesh's colour
-// c before any mesh's colour c + 1. A chunk is 8 steps of one warp (8 x the vertices a warp
+// c before any mesh's colour c + 1. An item is a chunk of 8 steps of one warp (8 x the vertices a warp
 // searches at once).
 std::vector<BatchItem> Batch::make_items(const std::vector<int>& sel) const {
     std::vector<int> ms = sel;
@@ -523,8 +577,8 @@ std::vector<BatchItem> Batch::make_items(const std::vector<int>& sel) const {
             const BatchMeshHost& h = hm[i];
             if (c >= h.n_colors) continue;
             const int v0 = h.v_off + h.col[c], v1 = h.v_off + h.col[c + 1];
-            const int chunk = 8 * (32 / cfg[i].lanes);
-            for (int a = v0; a < v1; a += chunk) items.push_back(BatchItem{i, c, a, std::min(v1, a + chunk)});
+            const int step = chunk(i);
+            for (int a = v0; a < v1; a += step) items.push_back(BatchItem{i, c, a, std::min(v1, a + step)});
         }
     return items;
 }
@@ -545,27 +599,26 @@ void Batch::ensure_launch_setup() {
     int dev = 0, sms = 148, per = 1;
     VSDMO_CUDA(cudaGetDevice(&dev));
     VSDMO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    VSDMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_iter, BATCH_WARPS * 32, flat_smem(maxk, 4)));
+    VSDMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_iter<false>, BATCH_WARPS * 32, batch_smem(maxk)));
     blocks = sms * std::max(per, 1);
 }
 
-void Batch::quality(BatchStats* out, int* d_it, int init, cudaStream_t s) const {
+void Batch::quality(BatchStats* out, int* d_it, int init, int advance, cudaStream_t s) {
     const int M = (int)hm.size();
-    k_batch_quality<<<M, 256, 0, s>>>(pos.p, el.p, d_meshes.p, out, M, d_it, init);
+    k_batch_quality<<<n_qchunks, 256, 0, s>>>(pos.p, el.p, d_meshes.p, qchunks.p, out, M, d_it, init, qpart.p);
+    VSDMO_CHECK_LAUNCH();
+    k_batch_quality_fold<<<1, 1024, 0, s>>>(qpart.p, qfirst.p, out, M, d_it, init, advance);
     VSDMO_CHECK_LAUNCH();
 }
 
 void Batch::launch_iteration(const BatchItem* d_it, int n, bool with_stats, cudaStream_t s) {
     VSDMO_CUDA(cudaMemsetAsync(done.p, 0, sizeof(int) * done.n, s));
     VSDMO_CUDA(cudaMemsetAsync(head.p, 0, sizeof(int), s));
-    k_batch_iter<<<blocks, BATCH_WARPS * 32, flat_smem(maxk, 4), s>>>(pos.p, rowptr.p, he.p, d_it, n, d_meshes.p, csize.p,
-                                                                     done.p, head.p, maxk, grid_scale, err.p);
+    const auto kernel = all_packed ? k_batch_iter<true> : k_batch_iter<false>;
+    kernel<<<blocks, BATCH_WARPS * 32, batch_smem(maxk), s>>>(pos.p, rowptr.p, he.p, d_it, n, d_meshes.p, csize.p, done.p,
+                                                              head.p, maxk, grid_scale, err.p);
     VSDMO_CHECK_LAUNCH();
-    if (with_stats) {
-        quality(stats.p, d_iter.p, 0, s);
-        k_batch_iter_advance<<<1, 1, 0, s>>>(d_iter.p);
-        VSDMO_CHECK_LAUNCH();
-    }
+    if (with_stats) quality(stats.p, d_iter.p, 0, 1, s);
 }
 
 void Batch::ensure_stats(int iters) {
@@ -583,7 +636,7 @@ void Batch::restart() {
     iters_done = 0;
     ensure_stats(16);
     d_iter.zero();
-    quality(stats.p, d_iter.p, 1, stream);
+    quality(stats.p, d_iter.p, 1, 0, stream);
     VSDMO_CUDA(cudaStreamSynchronize(stream));
 }
 
@@ -684,7 +737,7 @@ std::vector<std::string> Batch::autotune(int probe_iters) {
             for (size_t ci = 0; ci < cands.size(); ++ci) {
                 const BatchConfig c = cands[ci];
                 for (int i : bm) cfg[i] = c;
-                upload_meshes();
+                upload_meshes(bm);
                 const std::vector<BatchItem> it = make_items(bm);
                 DBuf<BatchItem> dit(it.size(), stream);
                 VSDMO_CUDA(cudaMemcpyAsync(dit.p, it.data(), sizeof(BatchItem) * it.size(), cudaMemcpyHostToDevice, stream));
@@ -699,7 +752,7 @@ std::vector<std::string> Batch::autotune(int probe_iters) {
                     VSDMO_CUDA(cudaEventRecord(e0, stream));
                     launch_iteration(dit.p, (int)it.size(), false, stream);
                     VSDMO_CUDA(cudaEventRecord(e1, stream));
-                    quality(qs.p, qit.p, 1, stream);
+                    quality(qs.p, qit.p, 1, 0, stream);
                     std::vector<BatchStats> st(M);
                     VSDMO_CUDA(cudaMemcpyAsync(st.data(), qs.p, sizeof(BatchStats) * M, cudaMemcpyDeviceToHost, stream));
                     VSDMO_CUDA(cudaStreamSynchronize(stream));

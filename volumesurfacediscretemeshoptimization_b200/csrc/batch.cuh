@@ -18,6 +18,7 @@ struct BatchMeshDev {
     int nq;        // candidates per axis (4 or 8)
     int depth;     // refinement levels (1..4)
     int lanes;     // lanes per vertex (8, 16 or 32)
+    int packed;    // four vertices per warp (flat_search.cuh) instead
     int col_base;  // first entry of this mesh in the per-(mesh, colour) arrays
     int n_elems;
     long el_off;   // first element index (x fk) in the concatenated element array
@@ -38,6 +39,7 @@ struct BatchMeshHost {
     int v_off = 0, he_off = 0, col_base = 0, n_colors = 0;
     long el_off = 0;
     std::vector<int> col;          // colour offsets of the free vertices, mesh-local ids
+    bool packed = false;           // searched four vertices per warp
 };
 
 // one input mesh: device arrays xyz [nV x 3], elems [nE x k] with mesh-local vertex ids
@@ -49,6 +51,8 @@ struct MeshInput {
 
 // single-mesh flat search (triangles or quads, N candidates per axis, `lanes` lanes per vertex)
 void launch_dmo_flat(const Mesh& m, const DmoLaunch& L, int nq, int lanes, cudaStream_t s);
+// the same for the 8 x 8 grid with four vertices per warp, where that is the faster search; false: not taken
+bool launch_dmo_flat_packed(const Mesh& m, const DmoLaunch& L, cudaStream_t s);
 int flat_max_ring();
 void prepare_flat_kernels();
 
@@ -69,6 +73,11 @@ struct Batch {
     DBuf<BatchMeshDev> d_meshes;
     DBuf<BatchItem> d_items;
     DBuf<BatchStats> stats;      // [(iterations + 1) x meshes]
+    DBuf<int2> qchunks;          // quality chunks: mesh, first element
+    DBuf<int> qfirst;            // [meshes + 1] first chunk of each mesh
+    DBuf<BatchStats> qpart;      // per-chunk partials
+    int n_qchunks = 0;
+    bool all_packed = false;
     int n_items = 0;
     bool items_dirty = true;
     int blocks = 0;
@@ -87,16 +96,18 @@ struct Batch {
     void get_positions(float* d_xyz_out) const;        // input numbering, [nV x 3]
     void set_positions(const float* d_xyz_in);
     int n_colors_total() const;
+    int chunk(int i) const;       // vertices of one work item of mesh i
 
    private:
-    void upload_meshes();
+    void choose_packed(const std::vector<int>& sel);
+    void upload_meshes(const std::vector<int>& sel = {});
     void invalidate_graph();
     std::vector<BatchItem> make_items(const std::vector<int>& sel) const;
     void ensure_items();
     void ensure_stats(int iters);
     void ensure_launch_setup();
     void launch_iteration(const BatchItem* d_it, int n, bool with_stats, cudaStream_t s);
-    void quality(BatchStats* out, int* d_it, int init, cudaStream_t s) const;
+    void quality(BatchStats* out, int* d_it, int init, int advance, cudaStream_t s);
 };
 
 // limit of the colour-class waits of the batched iteration on the current device (test-only lowering)

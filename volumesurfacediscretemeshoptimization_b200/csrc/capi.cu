@@ -70,8 +70,11 @@ void launch_color(vsdmo_opt_s* o, int c, cudaStream_t s) {
         if (o->kind == MK_HEX_COND) launch_dmo_hex_cond(m, L, s);
         else launch_dmo_hex(m, L, s);
     }
-    else if (o->mode == MODE_TRI2D) launch_dmo_tri2d(m, L, s);
-    else if (o->mode == MODE_FLAT) launch_dmo_flat(m, L, o->p.grid_n, 32, s);
+    else if (o->mode == MODE_TRI2D || o->mode == MODE_FLAT) {
+        if (o->p.grid_n == 8 && launch_dmo_flat_packed(m, L, s)) return;
+        if (o->mode == MODE_TRI2D) launch_dmo_tri2d(m, L, s);
+        else launch_dmo_flat(m, L, o->p.grid_n, 32, s);
+    }
     else if (o->mode == MODE_ANGLE) launch_dmo_angle(m, L, o->p.quality == VSDMO_MAX_ANGLE, s);
     else {
         SectorSurfaces sec{o->srow.p, o->stab.p, o->FS.p, o->Xs.p};

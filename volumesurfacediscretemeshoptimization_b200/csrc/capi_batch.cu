@@ -187,7 +187,7 @@ VSDMO_API long vsdmo_batch_info(vsdmo_batch_t batch, int which) {
     case 2: {
         long n = 0;
         for (size_t i = 0; i < b.hm.size(); ++i) {
-            const int chunk = 8 * (32 / b.cfg[i].lanes);
+            const int chunk = b.chunk((int)i);
             for (int c = 0; c < b.hm[i].n_colors; ++c) n += (b.hm[i].col[c + 1] - b.hm[i].col[c] + chunk - 1) / chunk;
         }
         return n;

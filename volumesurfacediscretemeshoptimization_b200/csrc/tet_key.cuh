@@ -14,7 +14,9 @@ namespace vsdmo {
 // 2^e as a float when it is a normal number, else 0. Multiplying by it is exactly ldexpf(x, e)
 // (both are the correctly rounded value of x 2^e), at the cost of one multiply.
 static __device__ __forceinline__ float exp2_exact(int e) { return (e >= -126 && e <= 127) ? __int_as_float((e + 127) << 23) : 0.f; }
-static __device__ __forceinline__ float scale2(float x, float p, int e) { return p != 0.f ? x * p : ldexpf(x, e); }
+// x 2^e when 2^e is no normal number: kept out of line (its code at every use crowds the instruction cache)
+static __device__ __noinline__ float scale2_far(float x, int e) { return ldexpf(x, e); }
+static __device__ __forceinline__ float scale2(float x, float p, int e) { return p != 0.f ? x * p : scale2_far(x, e); }
 
 // coefficients of tet (p, a, b, c) in scaled local coordinates
 static __device__ __forceinline__ void tet_coeffs(float ax, float ay, float az, float bx, float by, float bz,
