@@ -107,6 +107,7 @@ inline vsdmo_status guarded(F&& f) {
 struct vsdmo_model_s {
     mlp::Model m;
     mlp::Workspace ws;
+    mlp::TrainBuffers tb;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
 };

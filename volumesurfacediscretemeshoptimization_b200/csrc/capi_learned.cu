@@ -126,12 +126,17 @@ VSDMO_API vsdmo_status vsdmo_model_gradients(vsdmo_model_t m, const float* feats
         DBuf<float> f, t;
         copy_in_rows(f, feats, (size_t)n * mlp::IN, VSDMO_HOST, s);
         copy_in_rows(t, targets, (size_t)n * mlp::OUT, VSDMO_HOST, s);
-        m->ws.ensure(n, true, s);
-        m->m.gather(m->ws, f.p, t.p, nullptr, n, n, true, s);
-        m->m.forward(m->ws, n, true, s);
-        m->m.backward(m->ws, n, s);
+        const bool fused = mlp::fused_tiles(n) > 0;
+        if (fused) {
+            m->m.gradients_fused(m->tb, f.p, t.p, n, s);
+        } else {
+            m->ws.ensure(n, true, s);
+            m->m.gather(m->ws, f.p, t.p, nullptr, n, n, true, s);
+            m->m.forward(m->ws, n, true, s);
+            m->m.backward(m->ws, n, s);
+        }
         m->m.check(s);
-        if (loss) *loss = read_scalar(m->ws.loss.p, s) / (3.f * (float)n);
+        if (loss) *loss = read_scalar(fused ? m->tb.loss.p : m->ws.loss.p, s) / (3.f * (float)n);
         if (grads) {
             VSDMO_CUDA(cudaMemcpyAsync(grads, m->m.grads.p, sizeof(float) * mlp::N_PARAMS, cudaMemcpyDeviceToHost, s));
             VSDMO_CUDA(cudaStreamSynchronize(s));
@@ -156,13 +161,15 @@ VSDMO_API vsdmo_status vsdmo_model_train(vsdmo_model_t m, const float* feats, co
             df = fh.p;
             dt = th.p;
         }
-        m->ws.ensure(batch, true, s);
         DBuf<float> hist(std::max(steps, 1), s);
+        const bool fused = mlp::fused_tiles(batch) > 0 && n_rows <= (long)INT32_MAX;
+        if (fused) m->m.train_fused(m->tb, df, dt, n_rows, steps, batch, lr, seed, hist.p, s);
+        else m->ws.ensure(batch, true, s);
         std::mt19937_64 g(seed);
         std::uniform_int_distribution<long> pick(0, n_rows - 1);
         std::vector<int> idx(batch);
         DBuf<int> didx[2] = { DBuf<int>(batch, s), DBuf<int>(batch, s) };
-        for (int it = 0; it < steps; ++it) {
+        for (int it = 0; it < (fused ? 0 : steps); ++it) {
             for (int i = 0; i < batch; ++i) idx[i] = (int)pick(g);
             DBuf<int>& d = didx[it & 1];
             VSDMO_CUDA(cudaMemcpyAsync(d.p, idx.data(), sizeof(int) * batch, cudaMemcpyHostToDevice, s));

@@ -350,7 +350,8 @@ k_mlp_tet_infer(const float4* __restrict__ pos, const int* __restrict__ nb, cons
         tc::bulk_g2s(sb + FI_W3, W3p, 4 * 8192, bar_w);
         for (int c = 0; c < 4; ++c) tc::bulk_g2s(sb + FI_W4 + 1024u * c, W4p + (size_t)c * 8192, 1024, bar_w);
     }
-    bool weights = tc::mbar_wait_reported(bar_w, 0);
+    const unsigned long long limit = tc::wait_limit();
+    bool weights = tc::mbar_wait_within(bar_w, 0, limit);
     if (!weights && lane == 0) {
         atomicExch(err, tc::TC_TIMEOUT_LOAD);
         s_wfail = 1;
@@ -426,7 +427,7 @@ k_mlp_tet_infer(const float4* __restrict__ pos, const int* __restrict__ nb, cons
                 else fi_layer_issue(tmem, sbuf, sb + FI_W4, HID, 1024u, id16, bar_m);
             }
             pending = true;
-            if (!tc::mbar_wait_reported(bar_m, phase)) {
+            if (!tc::mbar_wait_within(bar_m, phase, limit)) {
                 if (lane == 0) {
                     atomicExch(err, tc::TC_TIMEOUT_MMA);
                     s_fail[g][step & 1] = 1;
@@ -587,15 +588,12 @@ void Workspace::ensure(long rows, bool training, cudaStream_t s) {
     }
 }
 
-namespace {
-// split-K parts for the weight-gradient GEMMs (batch as K)
 int wgrad_parts(int B) {
     const int chunks = B / 32;
     int parts = std::min(MAX_PARTS, std::max(1, chunks / 4));
     while (chunks % parts) --parts;
     return parts;
 }
-}  // namespace
 
 void Model::forward(Workspace& w, int n, bool training, cudaStream_t s) {
     const int tiles = (n + 127) / 128;
@@ -723,6 +721,7 @@ void Model::check(cudaStream_t s) {
 void set_wait_limit(unsigned long long ns) {
     VSDMO_CUDA(cudaDeviceSynchronize());
     VSDMO_CUDA(cudaMemcpyToSymbol(tc::g_wait_limit_ns, &ns, sizeof(ns)));
+    set_train_wait_limit(ns);
     VSDMO_CUDA(cudaDeviceSynchronize());
 }
 
@@ -741,6 +740,7 @@ void prepare(cudaStream_t s) {
     cfg((const void*)k_gemm<32, EPI_RAW>, tc::gemm_smem_bytes<32>());
     cfg((const void*)k_gemm<64, EPI_RAW>, tc::gemm_smem_bytes<64>());
     cfg((const void*)k_mlp_tet_infer, FI_SMEM);
+    prepare_train();
 }
 
 // D [M x N] = A [M x K] . B [N x K]^T for the GEMM test entry point (FP32 in, BF16 operands)

@@ -1,6 +1,7 @@
 // mlp.cuh -- host-side view of the learned proposal network (mlp.cu).
 #pragma once
 #include "vsdmo_internal.cuh"
+#include <algorithm>
 
 namespace vsdmo {
 namespace mlp {
@@ -11,6 +12,12 @@ constexpr int OUT = 3;
 constexpr int OUTP = 16;    // output padded to the smallest tensor-core N
 constexpr int MAX_NB = 32;
 constexpr int MAX_PARTS = 64;
+constexpr int TRAIN_PART = 128 * OUTP + 2 * 128 * HID + 128 * IN;   // floats of one weight-gradient partial
+
+// split-K parts of the weight gradients of a batch (the batch is K)
+int wgrad_parts(int B);
+// tiles of 128 rows per part when the parts of the batch are whole tiles, else 0
+int fused_tiles(int B);
 
 constexpr int OFF_W1 = 0;
 constexpr int OFF_B1 = OFF_W1 + HID * IN;
@@ -36,6 +43,14 @@ struct Workspace {
     void ensure(long rows, bool training, cudaStream_t s);
 };
 
+// buffers of the two-launch training step (mlp_train.cu)
+struct TrainBuffers {
+    int rows = 0, cap_parts = 0;
+    DBuf<float> part, ws, loss_rows, loss;
+    DBuf<int> idx;
+    void ensure(int B, cudaStream_t s);
+};
+
 struct Model {
     cudaStream_t stream = nullptr;
     DBuf<float> params, grads, adam_m, adam_v;     // flat FP32 [N_PARAMS]
@@ -56,6 +71,14 @@ struct Model {
     // rows idx (or 0..n_valid-1) of feats [*, 96] / targets [*, 3] -> w.X (+ w.XT, w.T)
     void gather(Workspace& w, const float* feats, const float* targets, const int* idx, int B, int n_valid,
                 bool training, cudaStream_t s);
+    // whole training steps in two launches each (batches with fused_tiles(B) > 0); d_hist [steps]: sums of
+    // the row losses. gradients_fused: the gradients alone into grads, the loss sum into w.loss.
+    void train_fused(TrainBuffers& w, const float* feats, const float* targets, long n_rows, int steps, int B, float lr,
+                     uint64_t seed, float* d_hist, cudaStream_t s);
+    void gradients_fused(TrainBuffers& w, const float* feats, const float* targets, int B, cudaStream_t s);
+    void train_tile(TrainBuffers& w, const float* feats, const float* targets, const int* idx, int B,
+                    unsigned long long* mt, int* next, long n_rows, bool rows_only, bool chained, cudaStream_t s);
+    void train_update(TrainBuffers& w, int B, const float* bias_corr, float lr, float* loss, cudaStream_t s);
     void check(cudaStream_t s);
     // fused inference for tet vertices [v0, v0 + n): ring features from the neighbour table
     // (nb / nbn index vertices from nb_base) -> network -> Y [n x ldy] (first 3 columns)
@@ -64,6 +87,8 @@ struct Model {
 };
 
 void prepare(cudaStream_t s);
+void prepare_train();
+void set_train_wait_limit(unsigned long long ns);
 void debug_gemm(const float* hA, const float* hB, int M, int N, int K, float* hD, cudaStream_t s);
 // limit of the reported tensor-core waits on the current device (test-only lowering)
 void set_wait_limit(unsigned long long ns);

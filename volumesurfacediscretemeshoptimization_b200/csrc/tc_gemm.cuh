@@ -105,9 +105,13 @@ __device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, uns
 static __device__ unsigned long long g_wait_limit_ns = WAIT_NS;
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return mbar_wait_for(bar, parity, WAIT_NS); }
-__device__ __forceinline__ bool mbar_wait_reported(uint32_t bar, uint32_t parity) {
-    const unsigned long long lim = *(volatile unsigned long long*)&g_wait_limit_ns;
+__device__ __forceinline__ unsigned long long wait_limit() { return *(volatile unsigned long long*)&g_wait_limit_ns; }
+// reported wait under a limit that the kernel read once (a read before every wait is an L2 round trip each)
+__device__ __forceinline__ bool mbar_wait_within(uint32_t bar, uint32_t parity, unsigned long long lim) {
     return lim != 0 && mbar_wait_for(bar, parity, lim);
+}
+__device__ __forceinline__ bool mbar_wait_reported(uint32_t bar, uint32_t parity) {
+    return mbar_wait_within(bar, parity, wait_limit());
 }
 
 // global -> shared bulk copy, completion counted on an mbarrier (no multicast)
