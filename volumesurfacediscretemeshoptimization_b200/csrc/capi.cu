@@ -8,6 +8,7 @@
 // positions, the local surfaces and the nearest-neighbour map, and their iteration adds the
 // nearest-neighbour walk and the normal update after the colour launches.
 #include "capi_internal.cuh"
+#include <cfloat>
 #include <cstring>
 #include <cmath>
 #include <algorithm>
@@ -848,20 +849,16 @@ VSDMO_API vsdmo_status vsdmo_opt_element_qualities(vsdmo_opt_t o, float* out, in
 
 VSDMO_API vsdmo_status vsdmo_opt_find_min_quality(vsdmo_opt_t o, float* min_q, double* mean_q) {
     if (!o) return fail(VSDMO_E_ARG, "null optimiser");
-    std::vector<float> q;
-    vsdmo_status st = guarded([&] {
+    // the iterations' own reduction, into a slot of its own (reading every element's quality back and
+    // summing it on one host core took 0.6 ms for 664 k tets)
+    return guarded([&] {
         const Mesh& m = o->mesh->m;
-        DBuf<float> t(m.nE, m.stream);
-        launch_element_qualities(m, o->kind, t.p, m.stream);
-        q = t.to_host();
+        DBuf<IterStats> t(1, m.stream);
+        launch_quality_stats(m, o->kind, t.p, o->d_iter.p, o->pmin.p, o->psum.p, o->pfail.p, o->done.p, -1, m.stream);
+        const IterStats r = read_scalar(t.p, m.stream);
+        if (min_q) *min_q = r.min_q == FLT_MAX ? INFINITY : r.min_q;   // no element has a quality (all NaN)
+        if (mean_q) *mean_q = r.sum_q / (double)m.nE;
     });
-    if (st != VSDMO_OK) return st;
-    float mn = INFINITY;
-    double sm = 0.0;
-    for (float x : q) { mn = std::min(mn, x); sm += x; }
-    if (min_q) *min_q = mn;
-    if (mean_q) *mean_q = q.empty() ? 0.0 : sm / (double)q.size();
-    return VSDMO_OK;
 }
 
 VSDMO_API vsdmo_status vsdmo_opt_quality_histogram(vsdmo_opt_t o, int32_t* host_counts, int n_cols) {
