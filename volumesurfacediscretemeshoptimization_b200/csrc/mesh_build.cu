@@ -55,18 +55,24 @@ __device__ __forceinline__ uint32_t priority(uint32_t i, uint32_t seed, uint32_t
 #define GRID_STRIDE(i, n) for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (long)gridDim.x * blockDim.x)
 constexpr unsigned FULL = 0xffffffffu;
 
-__global__ void k_count_keys_u32(const uint32_t* keys, long n, int* counts) { GRID_STRIDE(i, n) atomicAdd(&counts[keys[i]], 1); }
-
-__global__ void k_input(const float* xyz, int nV, const int* elems, long nIdx, float4* pos, int* err, int* nonzero_z) {
+// copies the input, checks it and counts each vertex's elements; slot: the place of an element corner
+// among its vertex's (-1: index out of range). The counter's old value is that place, so one pass of
+// atomics serves the whole vertex-to-element table.
+__global__ void k_input(const float* xyz, int nV, const int* elems, long nIdx, float4* pos, int* orig, int* cur,
+                        int* out, int* counts, int* slot, int* err, int* nonzero_z) {
     GRID_STRIDE(i, nV) {
         float x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
         if (!isfinite(x) || !isfinite(y) || !isfinite(z)) atomicMax(err, BE_NAN);
         if (z != 0.f) *nonzero_z = 1;
         pos[i] = make_float4(x, y, z, 0.f);
+        orig[i] = cur[i] = (int)i;
     }
     GRID_STRIDE(i, nIdx) {
         int v = elems[i];
-        if (v < 0 || v >= nV) atomicMax(err, BE_INDEX);
+        out[i] = v;
+        const bool bad = v < 0 || v >= nV;
+        if (bad) atomicMax(err, BE_INDEX);
+        slot[i] = bad ? -1 : atomicAdd(&counts[v], 1);
     }
 }
 
@@ -86,76 +92,112 @@ __device__ __forceinline__ void smallest_first(int a, int b, int c, uint32_t* o)
     else { o[0] = c; o[1] = a; o[2] = b; }
 }
 
-__global__ void k_tet_faces(const int* tets, int nT, uint32_t* f0, uint32_t* f1, uint32_t* f2) {
-    GRID_STRIDE(t, nT) {
-        const int* v = tets + 4 * t;
-        uint32_t o[3];
-        smallest_first(v[2], v[1], v[0], o); f0[4 * t] = o[0]; f1[4 * t] = o[1]; f2[4 * t] = o[2];
-        smallest_first(v[0], v[1], v[3], o); f0[4 * t + 1] = o[0]; f1[4 * t + 1] = o[1]; f2[4 * t + 1] = o[2];
-        smallest_first(v[1], v[2], v[3], o); f0[4 * t + 2] = o[0]; f1[4 * t + 2] = o[1]; f2[4 * t + 2] = o[2];
-        smallest_first(v[0], v[3], v[2], o); f0[4 * t + 3] = o[0]; f1[4 * t + 3] = o[1]; f2[4 * t + 3] = o[2];
-    }
-}
-
-// faces bucketed by their first vertex: row f0 holds (f1 << 32 | f2) of every face (f0, f1, f2)
-__global__ void k_face_bucket(const uint32_t* f0, const uint32_t* f1, const uint32_t* f2, long nF, int* cursor,
-                              unsigned long long* out) {
-    GRID_STRIDE(i, nF) out[atomicAdd(&cursor[f0[i]], 1)] = ((unsigned long long)f1[i] << 32) | f2[i];
-}
-
-// one warp per row a (grid-stride over rows): face (a, b, c) is a boundary face unless the row
-// also holds its twin (a, c, b) (k_markDuplicateTris, mesh/MeshGPUCommon.cu:56-74); an exact
-// repeat is a non-manifold input. The boundary faces get their place among the row's boundary
-// faces in (b, c) order, so rows in vertex order give the lexicographic order of a sort.
-__global__ void k_face_rows(const int* rs, const unsigned long long* fb, long K, uint8_t* bnd, int* rank, int* u,
-                            int* err) {
-    const int lane = threadIdx.x & 31;
-    const long nw = ((long)gridDim.x * blockDim.x) >> 5;
-    for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < K; r += nw) {
-        const int b0 = rs[r], n = rs[r + 1] - b0;
-        for (int i = lane; i < n; i += 32) {
-            const unsigned long long x = fb[b0 + i], twin = (x << 32) | (x >> 32);
-            bool paired = false, repeat = false;
-            for (int j = 0; j < n; ++j) {
-                if (j == i) continue;
-                const unsigned long long y = fb[b0 + j];
-                repeat |= y == x;
-                paired |= y == twin;
+// One warp per vertex a (grid-stride): the faces whose first vertex is a, from the tets around a
+// (rs, inc: element corners 4 t + j by vertex). Corner j of tet t owns the faces of t that
+// smallest_first starts at j, so every face is looked at once. Face (a, b, c) is a boundary face
+// unless the row also holds its twin (a, c, b) (k_markDuplicateTris, mesh/MeshGPUCommon.cu:56-74); an
+// exact repeat is a non-manifold input. A boundary face takes its place among the row's boundary faces in
+// (b, c) order, so rows in vertex order give the lexicographic order of a sort; rec collects
+// them in any order as (b << 32 | c, a << 32 | place) and u counts them per row.
+// Bound by the latency of the gathers. The rows live in shared memory (faces of up to FACE_CAP; longer
+// ones in their own part of spill). Five passes over lists of all faces in global memory before: 260 us
+// for 663,552 tets, 30 us now.
+constexpr int FACE_CAP = 160;
+constexpr int FACE_WARPS = 4;
+__global__ void __launch_bounds__(FACE_WARPS * 32)
+k_tet_boundary(const int* __restrict__ rs, const uint32_t* __restrict__ inc, const int4* __restrict__ tets, long K,
+               const int* input_err, unsigned long long* spill, uint8_t* spill_flag, int* spill_used, int* u,
+               ulonglong2* rec, int* nrec, uint8_t* isB2, int* err, int* longest) {
+    __shared__ unsigned long long sf[FACE_WARPS][FACE_CAP];
+    __shared__ uint8_t sb[FACE_WARPS][FACE_CAP];
+    if (*input_err != BE_OK) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const long nw = (long)gridDim.x * FACE_WARPS;
+    for (long r = (long)blockIdx.x * FACE_WARPS + warp; r < K; r += nw) {
+        const int b0 = rs[r], m = 3 * (rs[r + 1] - b0);
+        unsigned long long* f = sf[warp];
+        uint8_t* bnd = sb[warp];
+        int n = 0;
+        for (int pass = 0; pass < 2; ++pass) {
+            n = 0;
+            for (int i0 = 0; i0 < m; i0 += 32) {
+                const int i = i0 + lane;
+                bool own = false;
+                uint32_t o[3];
+                if (i < m) {
+                    const uint32_t e = inc[b0 + i / 3];
+                    const int j = e & 3;
+                    const int4 t = tets[e >> 2];
+                    // the faces of corner j: all but the one opposite
+                    const int skip = j == 0 ? 2 : (j == 1 ? 3 : (j == 2 ? 1 : 0));
+                    const int face = i % 3 + (i % 3 >= skip ? 1 : 0);
+                    // corners of the face in order, two bits each
+                    const unsigned F = face == 0 ? (2u | 1u << 2 | 0u << 4) : face == 1 ? (0u | 1u << 2 | 3u << 4)
+                                     : face == 2 ? (1u | 2u << 2 | 3u << 4) : (0u | 3u << 2 | 2u << 4);
+                    const int p0 = F & 3, p1 = (F >> 2) & 3, p2 = F >> 4;
+                    const int a = p0 == 0 ? t.x : (p0 == 1 ? t.y : t.z), b = p1 == 1 ? t.y : (p1 == 2 ? t.z : t.w),
+                              c = p2 == 0 ? t.x : (p2 == 2 ? t.z : t.w);
+                    smallest_first(a, b, c, o);
+                    own = j == (a < b && a < c ? p0 : (b < a && b < c ? p1 : p2));
+                }
+                const unsigned mask = __ballot_sync(FULL, own);
+                const int at = n + __popc(mask & lt);
+                if (own && (pass == 1 || at < FACE_CAP)) f[at] = ((unsigned long long)o[1] << 32) | o[2];
+                n += __popc(mask);
             }
-            if (repeat) atomicMax(err, BE_NONMANIFOLD);
-            bnd[b0 + i] = paired ? 0 : 1;
+            if (pass == 1 || n <= FACE_CAP || n > SHORT_ROW_MAX) break;
+            int at = 0;
+            if (lane == 0) at = atomicAdd(spill_used, n);
+            at = __shfl_sync(FULL, at, 0);
+            f = spill + at;
+            bnd = spill_flag + at;
+        }
+        if (n > SHORT_ROW_MAX) {
+            if (lane == 0) atomicMax(longest, n);
+            continue;
         }
         __syncwarp();
         int cnt = 0;
         for (int i = lane; i < n; i += 32) {
-            if (!bnd[b0 + i]) continue;
-            const unsigned long long x = fb[b0 + i];
-            int k = 0;
-            for (int j = 0; j < n; ++j) k += (bnd[b0 + j] && fb[b0 + j] < x) ? 1 : 0;
-            rank[b0 + i] = k;
-            ++cnt;
+            const unsigned long long x = f[i], twin = (x << 32) | (x >> 32);
+            bool paired = false, repeat = false;
+            for (int j = 0; j < n; ++j) {
+                const unsigned long long y = f[j];
+                repeat |= y == x && j != i;
+                paired |= y == twin && j != i;
+            }
+            if (repeat) atomicMax(err, BE_NONMANIFOLD);
+            bnd[i] = paired ? 0 : 1;
+            cnt += paired ? 0 : 1;
         }
         cnt = __reduce_add_sync(FULL, cnt);
         if (lane == 0) u[r] = cnt;
+        if (cnt) {
+            __syncwarp();
+            int at = 0;
+            if (lane == 0) at = atomicAdd(nrec, cnt);
+            at = __shfl_sync(FULL, at, 0);
+            for (int i = lane; i < n; i += 32) {
+                if (!bnd[i]) continue;
+                const unsigned long long x = f[i];
+                int k = 0;
+                for (int j = 0; j < n; ++j) k += (bnd[j] && f[j] < x) ? 1 : 0;
+                // a repeat leaves two faces on one place: the build ends in an error, the list stays in bounds
+                rec[at + k] = make_ulonglong2(x, ((unsigned long long)r << 32) | (unsigned)k);
+                isB2[r] = 1; isB2[x >> 32] = 1; isB2[x & 0xffffffffull] = 1;
+            }
+        }
         __syncwarp();
     }
 }
 
-// one warp per row: the row's boundary faces to tris[offs[a] + rank], their vertices flagged
-__global__ void k_face_emit(const int* rs, const unsigned long long* fb, const uint8_t* bnd, const int* rank,
-                            const int* offs, long K, int* tris, uint8_t* isB2) {
-    const int lane = threadIdx.x & 31;
-    const long nw = ((long)gridDim.x * blockDim.x) >> 5;
-    for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < K; r += nw) {
-        const int b0 = rs[r], n = rs[r + 1] - b0;
-        for (int i = lane; i < n; i += 32) {
-            if (!bnd[b0 + i]) continue;
-            const long p = offs[r] + rank[b0 + i];
-            const unsigned long long x = fb[b0 + i];
-            const int b = (int)(x >> 32), c = (int)(x & 0xffffffffu);
-            tris[3 * p] = (int)r; tris[3 * p + 1] = b; tris[3 * p + 2] = c;
-            isB2[r] = 1; isB2[b] = 1; isB2[c] = 1;
-        }
+__global__ void k_face_emit(const ulonglong2* rec, int nB, const int* offs, int* tris) {
+    GRID_STRIDE(i, nB) {
+        const ulonglong2 x = rec[i];
+        const int a = (int)(x.y >> 32);
+        const long p = (long)offs[a] + (int)(x.y & 0xffffffffull);
+        tris[3 * p] = a; tris[3 * p + 1] = (int)(x.x >> 32); tris[3 * p + 2] = (int)(x.x & 0xffffffffull);
     }
 }
 
@@ -218,172 +260,184 @@ __global__ void k_emit_boundary_quads(const int* idx, int nB, const uint32_t* s0
     }
 }
 
-// every vertex pair of a hexahedron within [lo, lo+num) (mesh/MeshGPUCommon.cu:936-1037)
-__global__ void k_hex_pairs(const int* hexes, int nH, int lo, int num, uint32_t* ks, uint32_t* vs, int* counter) {
-    GRID_STRIDE(t, nH) {
-        const int* v = hexes + 8 * t;
-        for (int i = 0; i < 7; ++i)
-            for (int j = i + 1; j < 8; ++j) {
-                const int a = v[i] - lo, b = v[j] - lo;
-                if (a >= 0 && a < num && b >= 0 && b < num) {
-                    const int p = atomicAdd(counter, 2);
-                    ks[p] = a; vs[p] = b; ks[p + 1] = b; vs[p + 1] = a;
-                }
-            }
-    }
-}
-
 // halfhex of corner j: the other seven corners (k_constructHalfhexesNew, mesh/MeshGPUCommon.cu:1334-1368),
 // two int4 per halfhex (the eighth value is -1)
-__global__ void k_halfhexes(const uint32_t* order, long nHH, const int* hexes, int4* hh) {
+// the rows of inc (element corners by original vertex) in the final vertex order: row i is that of vertex orig[i]
+__global__ void k_halfhexes(const int* rs, const uint32_t* inc, const int* orig, const int* rowptr, int nV,
+                            const int* hexes, int4* hh) {
     const int H[8][7] = { {1, 2, 3, 4, 5, 6, 7}, {5, 6, 2, 0, 4, 7, 3}, {6, 7, 3, 1, 5, 4, 0}, {7, 4, 0, 2, 6, 5, 1},
                           {0, 3, 7, 5, 1, 2, 6}, {4, 7, 6, 1, 0, 3, 2}, {5, 4, 7, 2, 1, 0, 3}, {6, 5, 4, 3, 2, 1, 0} };
-    GRID_STRIDE(i, nHH) {
-        const int e = (int)order[i], t = e >> 3, j = e & 7;
-        const int* v = hexes + 8L * t;
-        hh[2 * i] = make_int4(v[H[j][0]], v[H[j][1]], v[H[j][2]], v[H[j][3]]);
-        hh[2 * i + 1] = make_int4(v[H[j][4]], v[H[j][5]], v[H[j][6]], -1);
+    const int lane = threadIdx.x & 7;
+    const long nw = ((long)gridDim.x * blockDim.x) >> 3;
+    for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 3; r < nV; r += nw) {
+        const int src = rs[orig[r]], dst = rowptr[r], n = rowptr[r + 1] - dst;
+        for (int q = lane; q < n; q += 8) {
+            const int e = (int)inc[src + q], t = e >> 3, j = e & 7;
+            const int* v = hexes + 8L * t;
+            const long i = dst + q;
+            hh[2 * i] = make_int4(v[H[j][0]], v[H[j][1]], v[H[j][2]], v[H[j][3]]);
+            hh[2 * i + 1] = make_int4(v[H[j][4]], v[H[j][5]], v[H[j][6]], -1);
+        }
     }
 }
 
 __global__ void k_not(const uint8_t* f, uint8_t* o, long n) { GRID_STRIDE(i, n) o[i] = f[i] ? 0 : 1; }
 
 // ---- permutations -----------------------------------------------------------------------
-// full-size maps from a range order: new_of_old / old_of_new are identity outside [start, start+num)
-__global__ void k_range_maps(const int* order_local, int start, int num, int nTot, int* old_of_new, int* new_of_old) {
+// New vertex order: position start + i comes from start + order[i] for i < num, the others stay. One pass moves the
+// positions, the original indices with their inverse and up to two flag arrays (of nf0 / nf1
+// vertices) and leaves the map for the remap of index arrays.
+__global__ void k_permute(const int* order, int start, int num, int nTot, const float4* pin, float4* pout,
+                          const int* oin, int* oout, int* cur_of_orig, int* new_of_old, const uint8_t* f0, uint8_t* g0, int nf0,
+                          const uint8_t* f1, uint8_t* g1, int nf1) {
     GRID_STRIDE(i, nTot) {
-        if (i < start || i >= start + num) { old_of_new[i] = (int)i; new_of_old[i] = (int)i; }
-    }
-    GRID_STRIDE(i, num) {
-        int o = start + order_local[i];
-        old_of_new[start + i] = o;
-        new_of_old[o] = start + (int)i;
-    }
-}
-
-__global__ void k_permute_verts(const int* old_of_new, int nTot, const float4* pin, float4* pout, const int* oin, int* oout) {
-    GRID_STRIDE(i, nTot) {
-        int o = old_of_new[i];
+        const int o = i >= start && i < start + num ? start + order[i - start] : (int)i;
         pout[i] = pin[o];
-        oout[i] = oin[o];
+        const int og = oin[o];
+        oout[i] = og;
+        cur_of_orig[og] = (int)i;
+        new_of_old[o] = (int)i;
+        if (i < nf0) g0[i] = f0[o];
+        if (i < nf1) g1[i] = f1[o];
     }
 }
 
-__global__ void k_permute_u8(const int* old_of_new, int n, const uint8_t* in, uint8_t* out) {
-    GRID_STRIDE(i, n) out[i] = in[old_of_new[i]];
-}
-
-__global__ void k_remap(int* idx, long n, const int* new_of_old, int limit) {
-    GRID_STRIDE(i, n) {
-        int v = idx[i];
-        if (v >= 0 && v < limit) idx[i] = new_of_old[v];
-    }
-}
-
-// ---- adjacency pairs ---------------------------------------------------------------------
-__global__ void k_tet_edge_pairs(const int* tets, int nT, int lo, int num, uint32_t* ks, uint32_t* vs, int* counter) {
-    const int E[6][2] = { {0, 1}, {0, 2}, {0, 3}, {1, 2}, {1, 3}, {2, 3} };
-    GRID_STRIDE(t, nT) {
-        const int* v = tets + 4 * t;
-#pragma unroll
-        for (int e = 0; e < 6; ++e) {
-            int a = v[E[e][0]] - lo, b = v[E[e][1]] - lo;
-            if (a >= 0 && a < num && b >= 0 && b < num) {
-                int p = atomicAdd(counter, 2);
-                ks[p] = a; vs[p] = b; ks[p + 1] = b; vs[p + 1] = a;
-            }
-        }
-    }
-}
-
-__global__ void k_tri_edge_pairs(const int* tris, int nTris, int lo, int num, uint32_t* ks, uint32_t* vs, int* counter) {
-    const int E[3][2] = { {0, 1}, {0, 2}, {1, 2} };
-    GRID_STRIDE(t, nTris) {
-        const int* v = tris + 3 * t;
-#pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            int a = v[E[e][0]] - lo, b = v[E[e][1]] - lo;
-            if (a >= 0 && a < num && b >= 0 && b < num) {
-                int p = atomicAdd(counter, 2);
-                ks[p] = a; vs[p] = b; ks[p + 1] = b; vs[p + 1] = a;
-            }
-        }
-    }
-}
-
-// quad edges and both diagonals
-__global__ void k_quad_edge_pairs(const int* quads, int nQ, int lo, int num, uint32_t* ks, uint32_t* vs, int* counter) {
-    const int E[6][2] = { {0, 1}, {1, 2}, {2, 3}, {3, 0}, {0, 2}, {1, 3} };
-    GRID_STRIDE(t, nQ) {
-        const int* v = quads + 4 * t;
-#pragma unroll
-        for (int e = 0; e < 6; ++e) {
-            int a = v[E[e][0]] - lo, b = v[E[e][1]] - lo;
-            if (a >= 0 && a < num && b >= 0 && b < num) {
-                int p = atomicAdd(counter, 2);
-                ks[p] = a; vs[p] = b; ks[p + 1] = b; vs[p + 1] = a;
-            }
-        }
-    }
+__global__ void k_remap(int* idx, long n, const int* new_of_old) {
+    GRID_STRIDE(i, n) idx[i] = new_of_old[idx[i]];
 }
 
 // ---- JPL colouring ---------------------------------------------------------------------------
-__global__ void k_fill_int(int* a, long n, int v) { GRID_STRIDE(i, n) a[i] = v; }
-
-// One JPL round c: an uncoloured vertex is coloured iff its priority beats every neighbour that
-// is uncoloured or coloured in this round (rnd: the round each vertex was coloured in, -1 before).
-// Its colour is c (round colours), or with first_fit the smallest colour none of its coloured
-// neighbours has: those all have higher priorities and earlier rounds (two neighbours are never
-// coloured in the same round), so the colours are the greedy colouring in priority order.
-// prev: the previous round's count of uncoloured vertices in the same host read (null for the
-// first round of one); when it is 0 every vertex has its colour and the round has nothing to do.
-// maxc collects the largest first-fit colour.
-__global__ void k_jpl_round(int n, const int* rowptr, const int* col, uint32_t seed, int c, int first_fit, int* colors,
-                            int* rnd, int* remaining, const int* prev, int* maxc) {
-    if (prev && *prev == 0) return;
-    GRID_STRIDE(i, n) {
-        if (rnd[i] != -1) continue;
-        const uint32_t pi = priority((uint32_t)i, seed, (uint32_t)n);
-        bool f = true;
-        for (int e = rowptr[i]; e < rowptr[i + 1]; ++e) {
-            const int j = col[e];
-            const int jr = rnd[j];
-            if ((jr != -1 && jr != c) || (int)i == j) continue;
-            if (pi <= priority((uint32_t)j, seed, (uint32_t)n)) { f = false; break; }
-        }
-        if (!f) {
-            atomicAdd(remaining, 1);
-            continue;
-        }
-        int colour = c;
-        if (first_fit) {
-            // smallest colour not taken by a neighbour coloured in an earlier round
-            unsigned long long used = 0ull;
-            for (int e = rowptr[i]; e < rowptr[i + 1]; ++e) {
-                const int j = col[e];
-                const int jr = rnd[j];
-                if (jr == -1 || jr == c || (int)i == j) continue;
-                const int cj = colors[j];
-                if (cj < 64) used |= 1ull << cj;
+// The vertices of [lo, lo + num) that share an element are neighbours, and every vertex waits for its
+// neighbours of higher priority only: its colour is the smallest one none of them has (first fit), or
+// 1 + the largest of them (round colours: the JPL round it would be coloured in). Both are
+// functions of those neighbours' colours alone, so a vertex may be coloured as soon as they are,
+// in any order and without rounds, and the colours are those of the round-by-round rule.
+//
+// k_wait_lists: one warp per vertex, its higher-priority neighbours (places in the range) from the
+// elements around it to list[(k - 1) * rs[original vertex]], their number beside the row start in
+// info. Neighbours seen more than once are dropped by a small table that keeps the last value of
+// each hash; the few it lets through twice change nothing. Bound by the latency of its gathers
+// (25 us for the 103,823 inner vertices of 663,552 tets); writing, bucketing, deduplicating and copying all
+// neighbour pairs as a CSR before: 450 us.
+constexpr int WAIT_TABLE = 128;
+template <int KC>
+__global__ void __launch_bounds__(128)
+k_wait_lists(const int* __restrict__ rs, const uint32_t* __restrict__ inc, const int* __restrict__ elems,
+             const int* __restrict__ orig_of_cur, const int* __restrict__ cur_of_orig, int lo, int num, uint32_t seed,
+             int* list, int2* info, int* colors) {
+    __shared__ int table[4][WAIT_TABLE];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const long nw = (long)gridDim.x * 4;
+    for (long v = (long)blockIdx.x * 4 + warp; v < num; v += nw) {
+        for (int j = lane; j < WAIT_TABLE; j += 32) table[warp][j] = -1;
+        const int o = orig_of_cur[lo + v], b0 = rs[o], m = (KC - 1) * (rs[o + 1] - b0);
+        int* out = list + (long)(KC - 1) * b0;
+        const uint32_t pv = priority((uint32_t)v, seed, (uint32_t)num);
+        int n = 0;
+        __syncwarp();
+        for (int i0 = 0; i0 < m; i0 += 32) {
+            const int i = i0 + lane;
+            bool take = false;
+            int w = 0;
+            if (i < m) {
+                const uint32_t e = inc[b0 + i / (KC - 1)];
+                const uint32_t j = e % KC, c = (j + 1 + i % (KC - 1)) % KC;
+                w = cur_of_orig[elems[e - j + c]] - lo;
+                if (w >= 0 && w < num && w != (int)v && priority((uint32_t)w, seed, (uint32_t)num) >= pv)
+                    take = atomicExch(&table[warp][(w * 0x9E3779B1u) >> 25], w) != w;
             }
-            if (~used) {
+            const unsigned mask = __ballot_sync(FULL, take);
+            if (take) out[n + __popc(mask & lt)] = w;
+            n += __popc(mask);
+        }
+        if (lane == 0) {
+            info[v] = make_int2(b0, n);
+            colors[v] = -1;
+        }
+        __syncwarp();
+    }
+}
+
+// One thread per vertex: looks COLOUR_TRIES times whether the vertices it waits for have their
+// colours (going on from the first one that had none) and then takes its own. What is left after
+// the tries is counted in *remaining and taken up by the next launch; prev: the count of the launch
+// before (null for the first); when it is 0 nothing is left. A launch always colours the uncoloured vertex
+// of highest priority, so the launches end whatever the order the blocks run in. hist counts
+// the colours below 256, maxc collects the largest. Chains of waiting vertices pass within one
+// launch at the latency of a read through L2 (27 us for 103,823 vertices); a launch per
+// round before: 32 launches of up to 14 us.
+constexpr int COLOUR_TRIES = 32;
+__global__ void __launch_bounds__(256)
+k_colour(int num, const int* __restrict__ list, int per_slot, const int2* __restrict__ info, int first_fit, int* colors, int* remaining,
+         const int* prev, int* maxc, int* hist) {
+    if (prev && *prev == 0) return;
+    const long v = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    volatile int* col = colors;
+    bool todo = v < num && col[v] < 0;
+    int colour = -1;
+    if (__any_sync(FULL, todo)) {
+        const int* p = nullptr;
+        int n = 0, at = 0, mx = -1;
+        unsigned long long used = 0ull;
+        if (todo) {
+            const int2 w = info[v];
+            p = list + (long)per_slot * w.x;
+            n = w.y;
+        }
+        for (int t = 0; t < COLOUR_TRIES && __any_sync(FULL, todo && colour < 0); ++t) {
+            if (!todo || colour >= 0) continue;
+            while (at < n) {
+                int c[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) c[j] = at + j < n ? col[p[at + j]] : -2;
+                int j = 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (j != q || c[q] < 0) continue;
+                    if (c[q] < 64) used |= 1ull << c[q];
+                    mx = max(mx, c[q]);
+                    ++j;
+                }
+                at += j;
+                if (j < 4) break;
+            }
+            if (at < n) continue;
+            if (!first_fit) {
+                colour = mx + 1;
+            } else if (~used) {
                 colour = __ffsll((long long)~used) - 1;
             } else {
                 for (colour = 64;; ++colour) {
                     bool taken = false;
-                    for (int e = rowptr[i]; e < rowptr[i + 1] && !taken; ++e) {
-                        const int j = col[e];
-                        const int jr = rnd[j];
-                        taken = jr != -1 && jr != c && (int)i != j && colors[j] == colour;
-                    }
+                    for (int e = 0; e < n && !taken; ++e) taken = col[p[e]] == colour;
                     if (!taken) break;
                 }
             }
-            atomicMax(maxc, colour);
+            col[v] = colour;
         }
-        colors[i] = colour;
-        rnd[i] = c;
+        __syncwarp();
     }
+    const unsigned left = __ballot_sync(FULL, todo && colour < 0);
+    const int lane = threadIdx.x & 31;
+    if (left && lane == 0) atomicAdd(remaining, __popc(left));
+    const unsigned same = __match_any_sync(FULL, colour);
+    if (colour >= 0 && lane == __ffs(same) - 1) {
+        if (colour < 256) atomicAdd(&hist[colour], __popc(same));
+        if (colour > *(volatile int*)maxc) atomicMax(maxc, colour);
+    }
+}
+
+// offs[c] = lo + the vertices of the colours below c (nc <= 256 colours; one block of 256 threads)
+__global__ void k_colour_offsets(const int* hist, int nc, int lo, int* offs) {
+    __shared__ int h[256];
+    const int t = threadIdx.x;
+    h[t] = t < nc ? hist[t] : 0;
+    __syncthreads();
+    int s = lo;
+    for (int i = 0; i < t; ++i) s += h[i];
+    if (t < nc) offs[t] = s;
+    if (t == nc - 1) offs[nc] = s + h[t];
 }
 
 __global__ void k_add_const(int* a, long n, int v) { GRID_STRIDE(i, n) a[i] += v; }
@@ -416,7 +470,9 @@ __global__ void k_he_records(const uint32_t* order, long nHE, const int* tris, i
 }
 
 // opposite = last halfedge of the target's row that points back to the source
-__global__ void k_opposite(const uint32_t* srcs, int4* he, long nHE, const int* rowptr) {
+// (longest: the rows' maximum; above SHORT_ROW_MAX the build ends in an error and nothing is searched)
+__global__ void k_opposite(const uint32_t* srcs, int4* he, long nHE, const int* rowptr, const int* longest) {
+    if (*longest > SHORT_ROW_MAX) return;
     GRID_STRIDE(i, nHE) {
         int src = (int)srcs[i], dst = he[i].x, opp = -1;
         for (int q = rowptr[dst]; q < rowptr[dst + 1]; ++q) if (he[q].x == src) opp = q;
@@ -425,11 +481,13 @@ __global__ void k_opposite(const uint32_t* srcs, int4* he, long nHE, const int* 
 }
 
 __global__ void k_flags_b1_feat(const uint32_t* srcs, const int4* he, long nHE, const float* fn, uint8_t* isB1,
-                                uint8_t* isFeat, int flat) {
+                                uint8_t* isFeat, int flat, int* nOpen, const int* longest) {
+    if (*longest > SHORT_ROW_MAX) return;
     GRID_STRIDE(i, nHE) {
         int src = (int)srcs[i];
         int4 h = he[i];
         if (h.y == -1) {
+            atomicAdd(nOpen, 1);
             isB1[src] = 1;
             if (!flat) { isFeat[src] = 1; isFeat[h.x] = 1; }
             continue;
@@ -476,7 +534,8 @@ __device__ __forceinline__ int third_vertex_quad(const int* q, int dst) {
 }
 
 __global__ void k_ccw(int nS, const int* rowptr, const int4* in, int4* out, const uint8_t* isB1, const uint8_t* isFeat,
-                      const int* tris, int fk, int* err) {
+                      const int* tris, int fk, int* err, const int* longest) {
+    if (*longest > SHORT_ROW_MAX) return;
     GRID_STRIDE(src, nS) {
         const int start = rowptr[src], n = rowptr[src + 1] - start;
         if (n == 0) { atomicMax(err, BE_FAN); continue; }
@@ -523,7 +582,8 @@ __global__ void k_ccw(int nS, const int* rowptr, const int4* in, int4* out, cons
     }
 }
 
-__global__ void k_opp_next(int nS, const int* rowptr, int4* he) {
+__global__ void k_opp_next(int nS, const int* rowptr, int4* he, const int* err, const int* longest) {
+    if (*err != BE_OK || *longest > SHORT_ROW_MAX) return;
     GRID_STRIDE(v, nS) {
         for (int i = rowptr[v]; i < rowptr[v + 1]; ++i) {
             int4 h = he[i];
@@ -536,10 +596,6 @@ __global__ void k_opp_next(int nS, const int* rowptr, int4* he) {
             he[i].y = opp; he[i].w = nxt;
         }
     }
-}
-
-__global__ void k_max_row(const int* rowptr, int n, int* mx) {
-    GRID_STRIDE(i, n) atomicMax(mx, rowptr[i + 1] - rowptr[i]);
 }
 
 __global__ void k_vertex_normals(int nS, const int* rowptr, const int4* he, const float* fn, float* vn) {
@@ -555,27 +611,35 @@ __global__ void k_vertex_normals(int nS, const int* rowptr, const int4* he, cons
 }
 
 // ---- halffaces ------------------------------------------------------------------------------------
-__global__ void k_halffaces(const uint32_t* order, long nH, const int* tets, int4* hf) {
-    GRID_STRIDE(i, nH) {
-        int e = (int)order[i], t = e >> 2, j = e & 3;
-        const int* v = tets + 4 * (long)t;
-        int4 o;
-        if (j == 0) o = make_int4(v[1], v[2], v[3], t);
-        else if (j == 1) o = make_int4(v[0], v[3], v[2], t);
-        else if (j == 2) o = make_int4(v[0], v[1], v[3], t);
-        else o = make_int4(v[0], v[2], v[1], t);
-        hf[i] = o;
+// the rows of inc (element corners by original vertex) in the final vertex order: row i is that of vertex orig[i]
+__global__ void k_halffaces(const int* rs, const uint32_t* inc, const int* orig, const int* rowptr, int nV,
+                            const int4* tets, int4* hf) {
+    const int lane = threadIdx.x & 7;
+    const long nw = ((long)gridDim.x * blockDim.x) >> 3;
+    for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 3; r < nV; r += nw) {
+        const int src = rs[orig[r]], dst = rowptr[r], n = rowptr[r + 1] - dst;
+        for (int q = lane; q < n; q += 8) {
+            const uint32_t e = inc[src + q];
+            const int t = e >> 2, j = e & 3;
+            const int4 v = tets[t];
+            int4 o;
+            if (j == 0) o = make_int4(v.y, v.z, v.w, t);
+            else if (j == 1) o = make_int4(v.x, v.w, v.z, t);
+            else if (j == 2) o = make_int4(v.x, v.y, v.w, t);
+            else o = make_int4(v.x, v.z, v.y, t);
+            hf[dst + q] = o;
+        }
     }
 }
 
-__global__ void k_final_perm(const int* orig_of_cur, int nV, int* new_of_old) {
-    GRID_STRIDE(i, nV) new_of_old[orig_of_cur[i]] = (int)i;
+// row lengths in the final vertex order
+__global__ void k_row_lengths(const int* rs, const int* orig, int nV, int* len) {
+    GRID_STRIDE(i, nV) len[i] = rs[orig[i] + 1] - rs[orig[i]];
 }
 
 inline int G(long n) { return grid_for(n, 256); }
 
-void check_err(const DBuf<int>& err, cudaStream_t s, const char* stage) {
-    int e = read_scalar(err.p, s);
+void check_err(int e, const char* stage) {
     switch (e) {
     case BE_OK: return;
     case BE_INDEX: throw Error(VSDMO_E_ARG, std::string(stage) + ": element index out of range");
@@ -588,139 +652,154 @@ void check_err(const DBuf<int>& err, cudaStream_t s, const char* stage) {
     }
 }
 
+// what the build's kernels report, read by the host a few times in one piece
+struct BuildStatus {
+    int input_err;       // BE_* of the input
+    int nonzero_z;
+    int longest_elems;   // elements around one vertex
+    int face_err, face_rows, spill, nB, nS;   // boundary faces: error, longest refused row, ..., faces, boundary vertices
+    int surf_err, longest_he, nOpen, nFree;   // faces: error; halfedges of one vertex; boundary halfedges; free vertices
+    int fan_err, longest_full;                // fans: error, halfedges of one vertex with the dummies
+};
+struct ColourStatus {
+    int remaining[4];
+    int maxc;
+    int hist[256];
+};
+
 // Shared state of one build.
 struct Builder {
     Mesh& m;
     cudaStream_t s;
-    DBuf<int> orig_of_cur;
-    DBuf<int> err;
+    DBuf<int> orig_of_cur, cur_of_orig;
+    DBuf<int> inc_rs;                 // elements around each vertex (original numbering): rows and
+    DBuf<uint32_t> inc;               // element corners k e + j
+    DBuf<BuildStatus> st;
     explicit Builder(Mesh& mm) : m(mm), s(mm.stream) {}
 
-    // apply a permutation of range [start, start+num) given as order_local (new -> old, local)
-    void permute_range(const int* order_local, int start, int num, std::vector<DBuf<uint8_t>*> flags,
-                       std::vector<std::pair<int*, long>> elem_arrays, int remap_limit) {
+    BuildStatus status() { return read_scalar(st.p, s); }
+    int* at(int BuildStatus::* f) { return &(st.p->*f); }
+
+    // apply a permutation of range [start, start+num) given as order_local (new -> old, local) to the vertices and the
+    // surface; the elements keep the original numbering until finish_elems()
+    void permute_range(const int* order_local, int start, int num, std::vector<DBuf<uint8_t>*> flags) {
         const int nTot = m.nV;
-        DBuf<int> oon(nTot, s), noo(nTot, s);
-        k_range_maps<<<G(nTot), 256, 0, s>>>(order_local, start, num, nTot, oon.p, noo.p);
-        VSDMO_CHECK_LAUNCH();
+        DBuf<int> noo(nTot, s), o2(nTot, s);
         DBuf<float4> p2(nTot, s);
-        DBuf<int> o2(nTot, s);
-        k_permute_verts<<<G(nTot), 256, 0, s>>>(oon.p, nTot, m.pos.p, p2.p, orig_of_cur.p, o2.p);
+        DBuf<uint8_t> g[2];
+        const uint8_t* f[2] = { nullptr, nullptr };
+        for (size_t i = 0; i < flags.size(); ++i) {
+            if (!flags[i]->p) continue;
+            f[i] = flags[i]->p;
+            g[i].alloc(flags[i]->n, s);
+        }
+        k_permute<<<G(nTot), 256, 0, s>>>(order_local, start, num, nTot, m.pos.p, p2.p, orig_of_cur.p, o2.p, cur_of_orig.p, noo.p,
+                                          f[0], g[0].p, (int)g[0].n, f[1], g[1].p, (int)g[1].n);
         VSDMO_CHECK_LAUNCH();
         m.pos = std::move(p2);
         orig_of_cur = std::move(o2);
-        for (DBuf<uint8_t>* f : flags) {
-            if (!f->p) continue;
-            long n = (long)f->n;
-            DBuf<uint8_t> f2(n, s);
-            k_permute_u8<<<G(n), 256, 0, s>>>(oon.p, (int)n, f->p, f2.p);
-            VSDMO_CHECK_LAUNCH();
-            *f = std::move(f2);
-        }
-        for (auto& ea : elem_arrays) {
-            if (!ea.first || ea.second == 0) continue;
-            k_remap<<<G(ea.second), 256, 0, s>>>(ea.first, ea.second, noo.p, remap_limit);
+        for (size_t i = 0; i < flags.size(); ++i)
+            if (f[i]) *flags[i] = std::move(g[i]);
+        const long nt = m.tris.p ? (long)m.fk * m.nTris : 0;
+        if (nt > 0) {
+            k_remap<<<G(nt), 256, 0, s>>>(m.tris.p, nt, noo.p);
             VSDMO_CHECK_LAUNCH();
         }
     }
 
-    // stable partition of [0, n): flag == first_value first; returns the number of those
-    int stable_partition(const uint8_t* d_flags, int n, int first_value, DBuf<int>& order) {
-        order.alloc(n, s);
-        return stable_partition_flags(d_flags, n, first_value, order.p, s);
-    }
-
-    // colour the range [lo, lo+num) given its adjacency pairs; sort it by colour
-    int color_range(int lo, int num, DBuf<uint32_t>& ks, DBuf<uint32_t>& vs, int npairs, std::vector<int>& offs_host,
-                    DBuf<int>& offs_dev, std::vector<DBuf<uint8_t>*> flags, std::vector<std::pair<int*, long>> elems) {
-        // adjacency CSR with sorted unique rows
-        DBuf<int> rowptr(num + 1, s);
-        DBuf<int> col;
-        if (npairs > 0) {
-            col.alloc(npairs, s);
-            csr_unique_from_pairs(ks.p, vs.p, npairs, num, rowptr.p, col.p, s);
-        } else {
-            rowptr.zero();
-            col.alloc(1, s);
-        }
-        // JPL rounds, CH per host read: round c leaves remaining[c % CH] uncoloured vertices; the
-        // rounds after the last one find nobody uncoloured and change nothing; remaining[CH]
-        // collects the largest first-fit colour
-        constexpr int CH = 16;
+    // colour the range [lo, lo+num), sort it by colour; returns the number of colours
+    int color_range(int lo, int num, std::vector<int>& offs_host, DBuf<int>& offs_dev, std::vector<DBuf<uint8_t>*> flags) {
         const int first_fit = m.seed != VSDMO_COLOR_REFERENCE && !(m.seed & VSDMO_COLOR_ROUNDS) ? 1 : 0;
-        DBuf<int> colors(num, s), rnd(num, s), remaining(CH + 1, s);
-        k_fill_int<<<G(num), 256, 0, s>>>(rnd.p, num, -1);
+        DBuf<int> colors(num, s), list(std::max<size_t>((size_t)(m.k - 1) * inc.n, 1), s);
+        DBuf<int2> info(num, s);
+        DBuf<ColourStatus> cs(1, s);
+        cs.zero();
+        auto lists = m.k == 3 ? k_wait_lists<3> : m.k == 4 ? k_wait_lists<4> : k_wait_lists<8>;
+        lists<<<grid_for(32L * num, 128), 128, 0, s>>>(inc_rs.p, inc.p, m.elems.p, orig_of_cur.p, cur_of_orig.p, lo, num, m.seed,
+                                                       list.p, info.p, colors.p);
         VSDMO_CHECK_LAUNCH();
-        remaining.zero();
-        int nc = -1;
-        std::vector<int> left;
-        for (int c0 = 0; nc < 0; c0 += CH) {
-            if (c0 > num + 1) throw Error(VSDMO_E_CUDA, "colouring did not terminate");
-            VSDMO_CUDA(cudaMemsetAsync(remaining.p, 0, sizeof(int) * CH, s));
+        constexpr int CH = 4;
+        ColourStatus h;
+        for (long c0 = 0;; c0 += CH) {
+            if (c0 > (long)num + CH) throw Error(VSDMO_E_CUDA, "colouring did not terminate");
+            if (c0) VSDMO_CUDA(cudaMemsetAsync(cs.p->remaining, 0, sizeof(h.remaining), s));
             for (int i = 0; i < CH; ++i) {
-                k_jpl_round<<<G(num), 256, 0, s>>>(num, rowptr.p, col.p, m.seed, c0 + i, first_fit, colors.p, rnd.p,
-                                                   remaining.p + i, i > 0 ? remaining.p + i - 1 : nullptr,
-                                                   remaining.p + CH);
+                k_colour<<<(num + 255) / 256, 256, 0, s>>>(num, list.p, m.k - 1, info.p, first_fit, colors.p, cs.p->remaining + i,
+                                                           i > 0 ? cs.p->remaining + i - 1 : nullptr, &cs.p->maxc,
+                                                           cs.p->hist);
                 VSDMO_CHECK_LAUNCH();
             }
-            left = remaining.to_host();
-            for (int i = 0; i < CH && nc < 0; ++i)
-                if (left[i] == 0) nc = c0 + i + 1;
+            h = read_scalar(cs.p, s);
+            if (h.remaining[CH - 1] == 0) break;
         }
-        if (first_fit) nc = left[CH] + 1;
-        // the colours are dense: every round colours the top-priority vertex left, and a
-        // first-fit colour k has neighbours of every colour below k
+        // the colours are dense: a first-fit colour k has neighbours of every colour below k, a round colour k
+        // one of colour k - 1
+        const int nc = h.maxc + 1;
         // stable sort of the range by colour
-        DBuf<uint32_t> ck(num, s), order(num, s);
-        VSDMO_CUDA(cudaMemcpyAsync(ck.p, colors.p, sizeof(int) * num, cudaMemcpyDeviceToDevice, s));
+        DBuf<uint32_t> order(num, s);
         k_iota<<<G(num), 256, 0, s>>>(order.p, num);
         VSDMO_CHECK_LAUNCH();
-        radix_sort_pairs(ck.p, order.p, num, bits_for((uint32_t)(nc > 1 ? nc - 1 : 1)), s);
+        radix_sort_pairs((uint32_t*)colors.p, order.p, num, bits_for((uint32_t)(nc > 1 ? nc - 1 : 1)), s);
         offs_dev.alloc(nc + 1, s);
-        rowptr_from_sorted(ck.p, num, nc, offs_dev.p, s);
-        k_add_const<<<G(nc + 1), 256, 0, s>>>(offs_dev.p, nc + 1, lo);
-        VSDMO_CHECK_LAUNCH();
-        offs_host = offs_dev.to_host();
-        permute_range((const int*)order.p, lo, num, flags, elems, m.nV);
+        if (nc <= 256) {
+            k_colour_offsets<<<1, 256, 0, s>>>(cs.p->hist, nc, lo, offs_dev.p);
+            VSDMO_CHECK_LAUNCH();
+            offs_host.assign(1, lo);
+            for (int c = 0; c < nc; ++c) offs_host.push_back(offs_host.back() + h.hist[c]);
+        } else {
+            rowptr_from_sorted((uint32_t*)colors.p, num, nc, offs_dev.p, s);
+            k_add_const<<<G(nc + 1), 256, 0, s>>>(offs_dev.p, nc + 1, lo);
+            VSDMO_CHECK_LAUNCH();
+            offs_host = offs_dev.to_host();
+        }
+        permute_range((const int*)order.p, lo, num, flags);
         return nc;
+    }
+
+    // halfedges of the triangles / quads by source vertex; keys: the sources
+    void halfedges(DBuf<uint32_t>& keys, DBuf<int>& rowptr, DBuf<int4>& he, int* longest) {
+        const int nS = m.nSurf;
+        const long n = (long)m.fk * m.nTris;
+        DBuf<uint32_t> order(n, s);
+        keys.alloc(n, s);
+        VSDMO_CUDA(cudaMemcpyAsync(keys.p, m.tris.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
+        rowptr.alloc(nS + 1, s);
+        sort_short_rows(keys.p, order.p, n, nS, rowptr.p, longest, s);
+        he.alloc(n, s);
+        k_he_records<<<G(n), 256, 0, s>>>(order.p, n, m.tris.p, m.fk, he.p);
+        VSDMO_CHECK_LAUNCH();
+        k_opposite<<<G(n), 256, 0, s>>>(keys.p, he.p, n, rowptr.p, longest);
+        VSDMO_CHECK_LAUNCH();
     }
 
     void surface_init() {
         const int nS = m.nSurf;
         const long nHE1 = (long)m.fk * m.nTris;
         m.fn.alloc(3L * m.nTris, s);
-        err.zero();
-        k_face_normals<<<G(m.nTris), 256, 0, s>>>(m.tris.p, m.fk, m.nTris, m.pos.p, m.fn.p, err.p);
+        k_face_normals<<<G(m.nTris), 256, 0, s>>>(m.tris.p, m.fk, m.nTris, m.pos.p, m.fn.p, at(&BuildStatus::surf_err));
         VSDMO_CHECK_LAUNCH();
-        check_err(err, s, "surface");
-        // first-pass halfedges
+        BuildStatus h;
+        // first-pass halfedges; free vertices first, feature vertices last
         {
-            DBuf<uint32_t> keys(nHE1, s), order(nHE1, s);
-            VSDMO_CUDA(cudaMemcpyAsync(keys.p, m.tris.p, sizeof(int) * nHE1, cudaMemcpyDeviceToDevice, s));
-            DBuf<int> rowptr(nS + 1, s);
-            if (stable_sort_short_rows(keys.p, order.p, nHE1, nS, rowptr.p, s) > SHORT_ROW_MAX) throw_long_fan();
-            DBuf<int4> he(nHE1, s);
-            k_he_records<<<G(nHE1), 256, 0, s>>>(order.p, nHE1, m.tris.p, m.fk, he.p);
-            VSDMO_CHECK_LAUNCH();
-            k_opposite<<<G(nHE1), 256, 0, s>>>(keys.p, he.p, nHE1, rowptr.p);
-            VSDMO_CHECK_LAUNCH();
+            DBuf<uint32_t> keys;
+            DBuf<int> rowptr, order(nS, s);
+            DBuf<int4> he;
+            halfedges(keys, rowptr, he, at(&BuildStatus::longest_he));
             m.isB1.alloc(nS, s); m.isB1.zero();
             m.isFeat.alloc(nS, s); m.isFeat.zero();
-            k_flags_b1_feat<<<G(nHE1), 256, 0, s>>>(keys.p, he.p, nHE1, m.fn.p, m.isB1.p, m.isFeat.p, m.isFlat);
+            k_flags_b1_feat<<<G(nHE1), 256, 0, s>>>(keys.p, he.p, nHE1, m.fn.p, m.isB1.p, m.isFeat.p, m.isFlat,
+                                                    at(&BuildStatus::nOpen), at(&BuildStatus::longest_he));
             VSDMO_CHECK_LAUNCH();
             if (m.isFlat) {
                 k_copy_u8<<<G(nS), 256, 0, s>>>(m.isB1.p, m.isFeat.p, nS);
                 VSDMO_CHECK_LAUNCH();
             }
-        }
-        // free first, feature last
-        {
-            DBuf<int> order;
-            int nFree = stable_partition(m.isFeat.p, nS, 0, order);
-            std::vector<std::pair<int*, long>> el = { {m.tris.p, (long)m.fk * m.nTris} };
-            if (m.type == VSDMO_TET || m.type == VSDMO_HEX) el.push_back({m.elems.p, (long)m.k * m.nE});
-            permute_range(order.p, 0, nS, {&m.isB1, &m.isFeat}, el, nS);
-            m.nFeature = nS - nFree;
+            partition_flags(m.isFeat.p, nS, 0, order.p, at(&BuildStatus::nFree), s);
+            h = status();
+            check_err(h.surf_err, "surface");
+            if (h.longest_he > SHORT_ROW_MAX) throw_long_fan();
+            permute_range(order.p, 0, nS, {&m.isB1, &m.isFeat});
+            m.nFeature = nS - h.nFree;
         }
         const int nFree = nS - m.nFeature;
         for (int part = 0; part < 2; ++part) {
@@ -735,106 +814,89 @@ struct Builder {
                 nc = 0;
                 continue;
             }
-            long cap = m.type == VSDMO_TET ? 12L * m.nE : m.type == VSDMO_HEX ? 56L * m.nE : (m.fk == 4 ? 12L : 6L) * m.nTris;
-            DBuf<uint32_t> ks(cap, s), vs(cap, s);
-            DBuf<int> cnt(1, s);
-            cnt.zero();
-            if (m.type == VSDMO_HEX)
-                k_hex_pairs<<<G(m.nE), 256, 0, s>>>(m.elems.p, m.nE, lo, num, ks.p, vs.p, cnt.p);
-            else if (m.type == VSDMO_TET)
-                k_tet_edge_pairs<<<G(m.nE), 256, 0, s>>>(m.elems.p, m.nE, lo, num, ks.p, vs.p, cnt.p);
-            else if (m.fk == 4)
-                k_quad_edge_pairs<<<G(m.nTris), 256, 0, s>>>(m.tris.p, m.nTris, lo, num, ks.p, vs.p, cnt.p);
-            else
-                k_tri_edge_pairs<<<G(m.nTris), 256, 0, s>>>(m.tris.p, m.nTris, lo, num, ks.p, vs.p, cnt.p);
-            VSDMO_CHECK_LAUNCH();
-            int np = read_scalar(cnt.p, s);
-            std::vector<std::pair<int*, long>> el = { {m.tris.p, (long)m.fk * m.nTris} };
-            if (m.type == VSDMO_TET || m.type == VSDMO_HEX) el.push_back({m.elems.p, (long)m.k * m.nE});
-            nc = color_range(lo, num, ks, vs, np, oh, od, {&m.isB1, &m.isFeat}, el);
+            nc = color_range(lo, num, oh, od, {&m.isB1, &m.isFeat});
         }
-        final_halfedges();
+        final_halfedges(h.nOpen);
         m.vn.alloc(3L * nS, s);
         k_vertex_normals<<<G(nS), 256, 0, s>>>(nS, m.he_rowptr.p, m.he.p, m.fn.p, m.vn.p);
         VSDMO_CHECK_LAUNCH();
     }
 
-    void final_halfedges() {
+    // nD: the boundary halfedges, each of which gets a dummy twin
+    void final_halfedges(int nD) {
         const int nS = m.nSurf;
         const long nHE1 = (long)m.fk * m.nTris;
-        DBuf<uint32_t> keys(nHE1, s), order(nHE1, s);
-        VSDMO_CUDA(cudaMemcpyAsync(keys.p, m.tris.p, sizeof(int) * nHE1, cudaMemcpyDeviceToDevice, s));
-        DBuf<int> rowptr1(nS + 1, s);
-        if (stable_sort_short_rows(keys.p, order.p, nHE1, nS, rowptr1.p, s) > SHORT_ROW_MAX) throw_long_fan();
-        DBuf<int4> he1(nHE1, s);
-        k_he_records<<<G(nHE1), 256, 0, s>>>(order.p, nHE1, m.tris.p, m.fk, he1.p);
-        VSDMO_CHECK_LAUNCH();
-        k_opposite<<<G(nHE1), 256, 0, s>>>(keys.p, he1.p, nHE1, rowptr1.p);
-        VSDMO_CHECK_LAUNCH();
+        DBuf<uint32_t> keys;
+        DBuf<int> rowptr1;
+        DBuf<int4> he1;
+        halfedges(keys, rowptr1, he1, at(&BuildStatus::longest_he));
         DBuf<uint8_t> df(nHE1, s);
         k_dummy_flags<<<G(nHE1), 256, 0, s>>>(he1.p, nHE1, df.p);
         VSDMO_CHECK_LAUNCH();
         DBuf<int> didx(nHE1, s);
-        const int nD = compact_flags(df.p, nHE1, didx.p, s);
+        compact_flags(df.p, nHE1, didx.p, nullptr, s);
         const long nHE = nHE1 + nD;
         DBuf<uint32_t> k2(nHE, s), o2(nHE, s);
         DBuf<int4> rec(nHE, s);
         k_with_dummies<<<G(nHE), 256, 0, s>>>(keys.p, he1.p, nHE1, didx.p, nD, k2.p, rec.p);
         VSDMO_CHECK_LAUNCH();
         m.he_rowptr.alloc(nS + 1, s);
-        if (stable_sort_short_rows(k2.p, o2.p, nHE, nS, m.he_rowptr.p, s) > SHORT_ROW_MAX) throw_long_fan();
+        int* longest = at(&BuildStatus::longest_full);
+        int* err = at(&BuildStatus::fan_err);
+        sort_short_rows(k2.p, o2.p, nHE, nS, m.he_rowptr.p, longest, s);
         DBuf<int4> in(nHE, s);
         k_gather<int4><<<G(nHE), 256, 0, s>>>(rec.p, o2.p, in.p, nHE);
         VSDMO_CHECK_LAUNCH();
-        k_opposite<<<G(nHE), 256, 0, s>>>(k2.p, in.p, nHE, m.he_rowptr.p);
+        k_opposite<<<G(nHE), 256, 0, s>>>(k2.p, in.p, nHE, m.he_rowptr.p, longest);
         VSDMO_CHECK_LAUNCH();
         m.he.alloc(nHE, s);
-        err.zero();
-        k_ccw<<<G(nS), 256, 0, s>>>(nS, m.he_rowptr.p, in.p, m.he.p, m.isB1.p, m.isFeat.p, m.tris.p, m.fk, err.p);
+        k_ccw<<<G(nS), 256, 0, s>>>(nS, m.he_rowptr.p, in.p, m.he.p, m.isB1.p, m.isFeat.p, m.tris.p, m.fk, err, longest);
         VSDMO_CHECK_LAUNCH();
-        check_err(err, s, "halfedges");
-        k_opp_next<<<G(nS), 256, 0, s>>>(nS, m.he_rowptr.p, m.he.p);
+        k_opp_next<<<G(nS), 256, 0, s>>>(nS, m.he_rowptr.p, m.he.p, err, longest);
         VSDMO_CHECK_LAUNCH();
-        DBuf<int> mx(1, s);
-        mx.zero();
-        k_max_row<<<G(nS), 256, 0, s>>>(m.he_rowptr.p, nS, mx.p);
-        VSDMO_CHECK_LAUNCH();
-        m.maxHE = read_scalar(mx.p, s);
+        const BuildStatus h = status();
+        if (h.longest_full > SHORT_ROW_MAX) throw_long_fan();
+        check_err(h.fan_err, "halfedges");
+        m.maxHE = h.longest_full;
         m.nHE = (int)nHE;
     }
 
-    void tet_boundary() {
-        const int nT = m.nE, nV = m.nV;
-        const long nF = 4L * nT;
-        DBuf<uint32_t> f0(nF, s), f1(nF, s), f2(nF, s);
-        k_tet_faces<<<G(nT), 256, 0, s>>>(m.elems.p, nT, f0.p, f1.p, f2.p);
+    // boundary triangles and boundary vertices of a tet mesh; the vertices' order, boundary first
+    int tet_boundary(DBuf<int>& order) {
+        const int nV = m.nV;
+        const long nF = 4L * m.nE;
+        DBuf<int> u(nV, s), offs((long)nV + 1, s);
+        DBuf<unsigned long long> spill(nF, s);
+        DBuf<uint8_t> spill_flag(nF, s);
+        DBuf<ulonglong2> rec(nF, s);
+        m.isB2.alloc(nV, s);
+        m.isB2.zero();
+        u.zero();
+        k_tet_boundary<<<grid_for(32L * nV, FACE_WARPS * 32), FACE_WARPS * 32, 0, s>>>(
+            inc_rs.p, inc.p, (const int4*)m.elems.p, nV, at(&BuildStatus::input_err), spill.p, spill_flag.p, at(&BuildStatus::spill), u.p,
+            rec.p, at(&BuildStatus::nB), m.isB2.p, at(&BuildStatus::face_err), at(&BuildStatus::face_rows));
         VSDMO_CHECK_LAUNCH();
-        // bucket the faces by first vertex (counting sort), then pair each row's faces in place
-        DBuf<int> counts(nV, s), rs((long)nV + 1, s), cursor(nV, s), u(nV, s), offs((long)nV + 1, s), rank(nF, s);
-        DBuf<unsigned long long> fb(nF, s);
-        DBuf<uint8_t> bnd(nF, s);
-        counts.zero();
-        k_count_keys_u32<<<G(nF), 256, 0, s>>>(f0.p, nF, counts.p);
-        VSDMO_CHECK_LAUNCH();
-        exclusive_scan(counts.p, rs.p, nV, rs.p + nV, s);
-        if (longest_row(rs.p, nV, s) > SHORT_ROW_MAX)
+        exclusive_scan(u.p, offs.p, nV, offs.p + nV, s);
+        order.alloc(nV, s);
+        partition_flags(m.isB2.p, nV, 1, order.p, at(&BuildStatus::nS), s);
+        const BuildStatus h = status();
+        check_err(h.input_err, "input");
+        if (h.face_rows > SHORT_ROW_MAX)
             throw Error(VSDMO_E_VALENCE, "a vertex is the first corner of more than " + std::to_string(SHORT_ROW_MAX) +
                                              " tetrahedron faces (more than ~1365 tetrahedra around one vertex)");
-        VSDMO_CUDA(cudaMemcpyAsync(cursor.p, rs.p, sizeof(int) * nV, cudaMemcpyDeviceToDevice, s));
-        k_face_bucket<<<G(nF), 256, 0, s>>>(f0.p, f1.p, f2.p, nF, cursor.p, fb.p);
+        check_err(h.face_err, "boundary faces");
+        m.nTris = h.nB;
+        m.tris.alloc(3L * h.nB, s);
+        k_face_emit<<<G(h.nB), 256, 0, s>>>(rec.p, h.nB, offs.p, m.tris.p);
         VSDMO_CHECK_LAUNCH();
-        err.zero();
-        k_face_rows<<<G(32L * nV), 256, 0, s>>>(rs.p, fb.p, nV, bnd.p, rank.p, u.p, err.p);
-        VSDMO_CHECK_LAUNCH();
-        check_err(err, s, "boundary faces");
-        exclusive_scan(u.p, offs.p, nV, offs.p + nV, s);
-        const int nB = read_scalar(offs.p + nV, s);
-        m.nTris = nB;
-        m.tris.alloc(3L * nB, s);
-        m.isB2.alloc(m.nV, s);
-        m.isB2.zero();
-        k_face_emit<<<G(32L * nV), 256, 0, s>>>(rs.p, fb.p, bnd.p, rank.p, offs.p, nV, m.tris.p, m.isB2.p);
-        VSDMO_CHECK_LAUNCH();
+        order_elem_rows(h);
+        return h.nS;
+    }
+
+    // the rows of the vertex-to-element table longer than one warp orders (the others are)
+    void order_elem_rows(const BuildStatus& h) {
+        m.maxTets = h.longest_elems;
+        if (h.longest_elems > SHORT_ROW_MAX) sort_long_rows((const uint32_t*)m.elems.p, inc.p, (long)inc.n, m.nV, s);
     }
 
     void hex_boundary() {
@@ -860,75 +922,93 @@ struct Builder {
         VSDMO_CHECK_LAUNCH();
         DBuf<uint8_t> paired(nF, s), unpaired(nF, s);
         paired.zero();
-        err.zero();
-        k_pair_quads<<<G(nF), 256, 0, s>>>(s0.p, s1.p, s2.p, s3.p, nF, paired.p, err.p);
+        k_pair_quads<<<G(nF), 256, 0, s>>>(s0.p, s1.p, s2.p, s3.p, nF, paired.p, at(&BuildStatus::face_err));
         VSDMO_CHECK_LAUNCH();
-        check_err(err, s, "boundary faces");
         k_not<<<G(nF), 256, 0, s>>>(paired.p, unpaired.p, nF);
         VSDMO_CHECK_LAUNCH();
         DBuf<int> bidx(nF, s);
-        const int nB = compact_flags(unpaired.p, nF, bidx.p, s);
+        compact_flags(unpaired.p, nF, bidx.p, at(&BuildStatus::nB), s);
+        const BuildStatus h = status();
+        check_err(h.face_err, "boundary faces");
+        const int nB = h.nB;
         m.nTris = nB;
         m.tris.alloc(4L * nB, s);
         m.isB2.alloc(m.nV, s);
         m.isB2.zero();
         k_emit_boundary_quads<<<G(nB), 256, 0, s>>>(bidx.p, nB, s0.p, s1.p, s2.p, s3.p, m.tris.p, m.isB2.p);
         VSDMO_CHECK_LAUNCH();
+        order_elem_rows(h);
     }
 
-    void hex_halfhexes() {
-        const long nHH = 8L * m.nE;
-        DBuf<uint32_t> keys(nHH, s), order(nHH, s);
-        VSDMO_CUDA(cudaMemcpyAsync(keys.p, m.elems.p, sizeof(int) * nHH, cudaMemcpyDeviceToDevice, s));
-        k_iota<<<G(nHH), 256, 0, s>>>(order.p, nHH);
+    // the elements in the final vertex numbering and the halffaces / halfhexes, rows in element order
+    void finish_elems() {
+        const long n = (long)m.k * m.nE;
+        k_remap<<<G(n), 256, 0, s>>>(m.elems.p, n, cur_of_orig.p);
         VSDMO_CHECK_LAUNCH();
-        radix_sort_pairs(keys.p, order.p, nHH, bits_for((uint32_t)(m.nV - 1)), s);
         m.hf_rowptr.alloc(m.nV + 1, s);
-        rowptr_from_sorted(keys.p, nHH, m.nV, m.hf_rowptr.p, s);
-        m.hh.alloc(2 * nHH, s);
-        k_halfhexes<<<G(nHH), 256, 0, s>>>(order.p, nHH, m.elems.p, m.hh.p);
+        DBuf<int> len(m.nV, s);
+        k_row_lengths<<<G(m.nV), 256, 0, s>>>(inc_rs.p, orig_of_cur.p, m.nV, len.p);
         VSDMO_CHECK_LAUNCH();
-        DBuf<int> mx(1, s);
-        mx.zero();
-        k_max_row<<<G(m.nV), 256, 0, s>>>(m.hf_rowptr.p, m.nV, mx.p);
+        exclusive_scan(len.p, m.hf_rowptr.p, m.nV, m.hf_rowptr.p + m.nV, s);
+        if (m.type == VSDMO_HEX) {
+            m.hh.alloc(2 * n, s);
+            k_halfhexes<<<G(8L * m.nV), 256, 0, s>>>(inc_rs.p, inc.p, orig_of_cur.p, m.hf_rowptr.p, m.nV, m.elems.p, m.hh.p);
+        } else {
+            m.hf.alloc(n, s);
+            k_halffaces<<<G(8L * m.nV), 256, 0, s>>>(inc_rs.p, inc.p, orig_of_cur.p, m.hf_rowptr.p, m.nV,
+                                                     (const int4*)m.elems.p, m.hf.p);
+        }
         VSDMO_CHECK_LAUNCH();
-        m.maxTets = read_scalar(mx.p, s);
     }
 
-    void tet_halffaces() {
-        const long nH = 4L * m.nE;
-        DBuf<uint32_t> keys(nH, s), order(nH, s);
-        VSDMO_CUDA(cudaMemcpyAsync(keys.p, m.elems.p, sizeof(int) * nH, cudaMemcpyDeviceToDevice, s));
-        m.hf_rowptr.alloc(m.nV + 1, s);
-        stable_sort_short_rows(keys.p, order.p, nH, m.nV, m.hf_rowptr.p, s);
-        m.hf.alloc(nH, s);
-        k_halffaces<<<G(nH), 256, 0, s>>>(order.p, nH, m.elems.p, m.hf.p);
-        VSDMO_CHECK_LAUNCH();
-        DBuf<int> mx(1, s);
-        mx.zero();
-        k_max_row<<<G(m.nV), 256, 0, s>>>(m.hf_rowptr.p, m.nV, mx.p);
-        VSDMO_CHECK_LAUNCH();
-        m.maxTets = read_scalar(mx.p, s);
+    // boundary vertices first, the inner ones coloured and sorted, then the surface
+    void volume(const int* order, int nS) {
+        permute_range(order, 0, m.nV, {&m.isB2});
+        m.nSurf = nS;
+        const int nI = m.nV - nS;
+        if (nI > 0) {
+            m.nColInner = color_range(nS, nI, m.col_inner, m.d_col_inner, {&m.isB2});
+        } else {
+            m.nColInner = 0;
+            m.col_inner.assign(1, nS);
+            m.d_col_inner.alloc(1, s);
+            VSDMO_CUDA(cudaMemcpyAsync(m.d_col_inner.p, m.col_inner.data(), sizeof(int), cudaMemcpyHostToDevice, s));
+        }
+        if (nS > 0) surface_init();
+        finish_elems();
     }
 
     void run(const float* d_xyz, const int* d_elems) {
         const long nIdx = (long)m.nE * m.k;
         m.pos.alloc(m.nV, s);
         m.elems.alloc(nIdx, s);
-        VSDMO_CUDA(cudaMemcpyAsync(m.elems.p, d_elems, sizeof(int) * nIdx, cudaMemcpyDeviceToDevice, s));
-        err.alloc(1, s);
-        err.zero();
-        DBuf<int> nz(1, s);
-        nz.zero();
-        k_input<<<G(std::max<long>(m.nV, nIdx)), 256, 0, s>>>(d_xyz, m.nV, m.elems.p, nIdx, m.pos.p, err.p, nz.p);
-        VSDMO_CHECK_LAUNCH();
-        check_err(err, s, "input");
         orig_of_cur.alloc(m.nV, s);
-        k_iota<<<G(m.nV), 256, 0, s>>>((uint32_t*)orig_of_cur.p, m.nV);
-        VSDMO_CHECK_LAUNCH();
-        if (m.type == VSDMO_TRI || m.type == VSDMO_QUAD) {
+        cur_of_orig.alloc(m.nV, s);
+        st.alloc(1, s);
+        st.zero();
+        const bool volume_mesh = m.type != VSDMO_TRI && m.type != VSDMO_QUAD;
+        inc_rs.alloc((long)m.nV + 1, s);
+        inc.alloc(nIdx, s);
+        {
+            DBuf<int> counts(m.nV, s), slot(nIdx, s);
+            counts.zero();
+            k_input<<<G(std::max<long>(m.nV, nIdx)), 256, 0, s>>>(d_xyz, m.nV, d_elems, nIdx, m.pos.p, orig_of_cur.p, cur_of_orig.p,
+                                                                  m.elems.p, counts.p, slot.p, at(&BuildStatus::input_err),
+                                                                  at(&BuildStatus::nonzero_z));
+            VSDMO_CHECK_LAUNCH();
+            if (volume_mesh) {
+                DBuf<uint32_t> rows(nIdx, s);
+                rows_from_slots((const uint32_t*)m.elems.p, slot.p, counts.p, nIdx, m.nV, inc_rs.p, rows.p, s);
+                order_short_rows(inc_rs.p, rows.p, m.nV, inc.p, nullptr, at(&BuildStatus::longest_elems), s);
+            } else {
+                rows_from_slots((const uint32_t*)m.elems.p, slot.p, counts.p, nIdx, m.nV, inc_rs.p, inc.p, s);
+            }
+        }
+        if (!volume_mesh) {
+            const BuildStatus h = status();
+            check_err(h.input_err, "input");
             m.fk = m.k;
-            m.isFlat = read_scalar(nz.p, s) ? 0 : 1;
+            m.isFlat = h.nonzero_z ? 0 : 1;
             m.nSurf = m.nV;
             m.nTris = m.nE;
             m.tris.alloc(nIdx, s);
@@ -941,63 +1021,19 @@ struct Builder {
         } else if (m.type == VSDMO_TET) {
             m.fk = 3;
             m.isFlat = 0;
-            tet_boundary();
-            {
-                DBuf<int> order;
-                int nS = stable_partition(m.isB2.p, m.nV, 1, order);
-                permute_range(order.p, 0, m.nV, {&m.isB2}, { {m.tris.p, 3L * m.nTris}, {m.elems.p, 4L * m.nE} }, m.nV);
-                m.nSurf = nS;
-            }
-            const int nI = m.nV - m.nSurf;
-            if (nI > 0) {
-                DBuf<uint32_t> ks(12L * m.nE, s), vs(12L * m.nE, s);
-                DBuf<int> cnt(1, s);
-                cnt.zero();
-                k_tet_edge_pairs<<<G(m.nE), 256, 0, s>>>(m.elems.p, m.nE, m.nSurf, nI, ks.p, vs.p, cnt.p);
-                VSDMO_CHECK_LAUNCH();
-                int np = read_scalar(cnt.p, s);
-                m.nColInner = color_range(m.nSurf, nI, ks, vs, np, m.col_inner, m.d_col_inner, {&m.isB2},
-                                          { {m.tris.p, 3L * m.nTris}, {m.elems.p, 4L * m.nE} });
-            } else {
-                m.nColInner = 0;
-                m.col_inner.assign(1, m.nSurf);
-                m.d_col_inner.alloc(1, s);
-                VSDMO_CUDA(cudaMemcpyAsync(m.d_col_inner.p, m.col_inner.data(), sizeof(int), cudaMemcpyHostToDevice, s));
-            }
-            if (m.nSurf > 0) surface_init();
-            tet_halffaces();
+            DBuf<int> order;
+            const int nS = tet_boundary(order);
+            volume(order.p, nS);
         } else {  // VSDMO_HEX (MeshHexGPU::init, mesh/MeshHexGPU.cu:35-43)
             m.fk = 4;
             m.isFlat = 0;
+            check_err(status().input_err, "input");
             hex_boundary();
-            {
-                DBuf<int> order;
-                int nS = stable_partition(m.isB2.p, m.nV, 1, order);
-                permute_range(order.p, 0, m.nV, {&m.isB2}, { {m.tris.p, 4L * m.nTris}, {m.elems.p, 8L * m.nE} }, m.nV);
-                m.nSurf = nS;
-            }
-            const int nI = m.nV - m.nSurf;
-            if (nI > 0) {
-                DBuf<uint32_t> ks(56L * m.nE, s), vs(56L * m.nE, s);
-                DBuf<int> cnt(1, s);
-                cnt.zero();
-                k_hex_pairs<<<G(m.nE), 256, 0, s>>>(m.elems.p, m.nE, m.nSurf, nI, ks.p, vs.p, cnt.p);
-                VSDMO_CHECK_LAUNCH();
-                int np = read_scalar(cnt.p, s);
-                m.nColInner = color_range(m.nSurf, nI, ks, vs, np, m.col_inner, m.d_col_inner, {&m.isB2},
-                                          { {m.tris.p, 4L * m.nTris}, {m.elems.p, 8L * m.nE} });
-            } else {
-                m.nColInner = 0;
-                m.col_inner.assign(1, m.nSurf);
-                m.d_col_inner.alloc(1, s);
-                VSDMO_CUDA(cudaMemcpyAsync(m.d_col_inner.p, m.col_inner.data(), sizeof(int), cudaMemcpyHostToDevice, s));
-            }
-            if (m.nSurf > 0) surface_init();
-            hex_halfhexes();
+            DBuf<int> order(m.nV, s);
+            partition_flags(m.isB2.p, m.nV, 1, order.p, at(&BuildStatus::nS), s);
+            volume(order.p, status().nS);
         }
-        m.new_of_old.alloc(m.nV, s);
-        k_final_perm<<<G(m.nV), 256, 0, s>>>(orig_of_cur.p, m.nV, m.new_of_old.p);
-        VSDMO_CHECK_LAUNCH();
+        m.new_of_old = std::move(cur_of_orig);
         m.sync();
     }
 };

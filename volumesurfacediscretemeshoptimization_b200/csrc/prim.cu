@@ -183,85 +183,47 @@ __global__ void k_count_keys(const uint32_t* keys, long n, int* counts) {
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
         atomicAdd(&counts[keys[i]], 1);
 }
-// ---- CSR of the distinct pairs ------------------------------------------------------------------
-// bucket the values by key: each pair takes the next free slot of its key's row (the order
-// inside a row is arbitrary; k_row_unique makes the row canonical)
-__global__ void k_bucket_scatter(const uint32_t* keys, const uint32_t* vals, long n, int* cursor, uint32_t* out) {
+
+// counts per key; slot[i] is the place the counter gave to i within its row, so that the scatter
+// after the scan needs no atomics of its own
+__global__ void k_count_slots(const uint32_t* keys, long n, int* counts, int* slot) {
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        out[atomicAdd(&cursor[keys[i]], 1)] = vals[i];
+        slot[i] = atomicAdd(&counts[keys[i]], 1);
 }
 
-// one warp per row (grid-stride over rows): the row's distinct values in ascending order to
-// out[rs[r] ...] and their number to u[r]. A value is kept at its first occurrence in the row,
-// and its place is the number of kept values below it. Rows are short (the edges of one
-// vertex's ring), so the quadratic scans cost less than sorting the rows.
-__global__ void k_row_unique(const int* rs, const uint32_t* v, long K, uint8_t* keep, uint32_t* out, int* u) {
+__global__ void k_scatter_slots(const uint32_t* keys, const int* slot, const int* rs, long n, uint32_t* out) {
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+        if (slot[i] >= 0) out[rs[keys[i]] + slot[i]] = (uint32_t)i;
+}
+
+// one warp per row (grid-stride): the row's indices in ascending order (each placed by the number
+// of smaller indices in the row: they are distinct), the row's key beside each (keys may be null),
+// the longest row to *longest. Rows of more than SHORT_ROW_MAX indices are copied as they are.
+__global__ void k_row_order(const int* rs, const uint32_t* idx, long K, uint32_t* order, uint32_t* keys, int* longest) {
     const int lane = threadIdx.x & 31;
     const long nw = ((long)gridDim.x * blockDim.x) >> 5;
+    int mx = 0;
     for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < K; r += nw) {
         const int b = rs[r], n = rs[r + 1] - b;
-        for (int i = lane; i < n; i += 32) {
-            const uint32_t x = v[b + i];
-            bool first = true;
-            for (int j = 0; j < i && first; ++j) first = v[b + j] != x;
-            keep[b + i] = first ? 1 : 0;
-        }
-        __syncwarp();
-        int cnt = 0;
-        for (int i = lane; i < n; i += 32) {
-            if (!keep[b + i]) continue;
-            const uint32_t x = v[b + i];
-            int rank = 0;
-            for (int j = 0; j < n; ++j) rank += (keep[b + j] && v[b + j] < x) ? 1 : 0;
-            out[b + rank] = x;
-            ++cnt;
-        }
-        cnt = __reduce_add_sync(FULL, cnt);
-        if (lane == 0) u[r] = cnt;
-        __syncwarp();
-    }
-}
-
-// one warp per row: the distinct values of row r to col[rowptr[r] ...]
-__global__ void k_row_copy(const int* rs, const int* rowptr, const uint32_t* src, long K, int* col) {
-    const int lane = threadIdx.x & 31;
-    const long nw = ((long)gridDim.x * blockDim.x) >> 5;
-    for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < K; r += nw) {
-        const int b = rs[r], o = rowptr[r], n = rowptr[r + 1] - o;
-        for (int j = lane; j < n; j += 32) col[o + j] = (int)src[b + j];
-    }
-}
-
-// bucket the indices [0, n) by key (arbitrary order inside a row)
-__global__ void k_bucket_index(const uint32_t* keys, long n, int* cursor, uint32_t* out) {
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        out[atomicAdd(&cursor[keys[i]], 1)] = (uint32_t)i;
-}
-
-// one warp per row (grid-stride): the row's indices in ascending order (each placed by the
-// number of smaller indices in the row: they are distinct), and the row's key beside each
-__global__ void k_row_order(const int* rs, const uint32_t* idx, long K, uint32_t* order, uint32_t* keys) {
-    const int lane = threadIdx.x & 31;
-    const long nw = ((long)gridDim.x * blockDim.x) >> 5;
-    for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < K; r += nw) {
-        const int b = rs[r], n = rs[r + 1] - b;
-        for (int i = lane; i < n; i += 32) {
-            const uint32_t x = idx[b + i];
+        mx = max(mx, n);
+        for (int i0 = 0; i0 < n; i0 += 32) {
+            const int i = i0 + lane;
+            const uint32_t x = i < n ? idx[b + i] : 0u;
             int k = 0;
-            for (int j = 0; j < n; ++j) k += idx[b + j] < x ? 1 : 0;
-            order[b + k] = x;
-            keys[b + i] = (uint32_t)r;
+            if (n <= 32) {
+                for (int j = 0; j < n; ++j) k += __shfl_sync(FULL, x, j) < x ? 1 : 0;
+            } else if (n <= SHORT_ROW_MAX) {
+                for (int j = 0; j < n; ++j) k += idx[b + j] < x ? 1 : 0;
+            } else {
+                k = i;
+            }
+            if (i < n) {
+                order[b + k] = x;
+                if (keys) keys[b + i] = (uint32_t)r;
+            }
         }
     }
-}
-
-// the longest row of a CSR row pointer rs[0..K] to *out (atomic maximum; *out starts at 0)
-__global__ void k_longest_row(const int* rs, long K, int* out) {
-    int m = 0;
-    for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < K; r += (long)gridDim.x * blockDim.x)
-        m = max(m, rs[r + 1] - rs[r]);
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(out, m);
+    if (lane == 0 && mx > *(volatile int*)longest) atomicMax(longest, mx);
 }
 
 __global__ void k_iota_u32(uint32_t* a, long n) {
@@ -269,30 +231,7 @@ __global__ void k_iota_u32(uint32_t* a, long n) {
         a[i] = (uint32_t)i;
 }
 
-// in (key, value)-sorted pairs: 1 where a pair differs from the one before it, counted per key
-__global__ void k_flag_distinct(const uint32_t* k, const uint32_t* v, long n, uint8_t* flag, int* per_key) {
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const bool d = i == 0 || k[i] != k[i - 1] || v[i] != v[i - 1];
-        flag[i] = d ? 1 : 0;
-        if (d) atomicAdd(&per_key[k[i]], 1);
-    }
-}
-
-__global__ void k_gather_col(const uint32_t* v, const int* idx, long n, int* col) {
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        col[i] = (int)v[idx[i]];
-}
-
 }  // namespace
-
-int longest_row(const int* d_rowptr, long K, cudaStream_t s) {
-    if (K <= 0) return 0;
-    DBuf<int> m(1, s);
-    m.zero();
-    k_longest_row<<<grid_for(K, 256), 256, 0, s>>>(d_rowptr, K, m.p);
-    VSDMO_CHECK_LAUNCH();
-    return read_scalar(m.p, s);
-}
 
 int bits_for(uint32_t maxval) {
     int b = 1;
@@ -340,26 +279,30 @@ void radix_sort_pairs(uint32_t* keys, uint32_t* vals, long n, int bits, cudaStre
     }
 }
 
-int compact_flags(const uint8_t* d_flags, long n, int* d_out_index, cudaStream_t s) {
-    if (n <= 0) return 0;
-    DBuf<int> pos(n, s), tot(1, s);
+void compact_flags(const uint8_t* d_flags, long n, int* d_out_index, int* d_total, cudaStream_t s) {
+    if (n <= 0) {
+        if (d_total) VSDMO_CUDA(cudaMemsetAsync(d_total, 0, sizeof(int), s));
+        return;
+    }
+    DBuf<int> pos(n, s);
     k_flags_to_int<<<grid_for(n, 256), 256, 0, s>>>(d_flags, pos.p, n);
     VSDMO_CHECK_LAUNCH();
-    exclusive_scan(pos.p, pos.p, n, tot.p, s);
+    exclusive_scan(pos.p, pos.p, n, d_total, s);
     k_compact_scatter<<<grid_for(n, 256), 256, 0, s>>>(d_flags, pos.p, n, d_out_index);
     VSDMO_CHECK_LAUNCH();
-    return read_scalar(tot.p, s);
 }
 
-int stable_partition_flags(const uint8_t* d_flags, long n, int first_value, int* d_order, cudaStream_t s) {
-    if (n <= 0) return 0;
-    DBuf<int> pos(n, s), tot(1, s);
+void partition_flags(const uint8_t* d_flags, long n, int first_value, int* d_order, int* d_total, cudaStream_t s) {
+    if (n <= 0) {
+        VSDMO_CUDA(cudaMemsetAsync(d_total, 0, sizeof(int), s));
+        return;
+    }
+    DBuf<int> pos(n, s);
     k_match_to_int<<<grid_for(n, 256), 256, 0, s>>>(d_flags, first_value, pos.p, n);
     VSDMO_CHECK_LAUNCH();
-    exclusive_scan(pos.p, pos.p, n, tot.p, s);
-    k_partition_scatter<<<grid_for(n, 256), 256, 0, s>>>(d_flags, first_value, pos.p, tot.p, n, d_order);
+    exclusive_scan(pos.p, pos.p, n, d_total, s);
+    k_partition_scatter<<<grid_for(n, 256), 256, 0, s>>>(d_flags, first_value, pos.p, d_total, n, d_order);
     VSDMO_CHECK_LAUNCH();
-    return read_scalar(tot.p, s);
 }
 
 void rowptr_from_sorted(const uint32_t* d_sorted_keys, long n, int K, int* d_rowptr, cudaStream_t s) {
@@ -372,79 +315,40 @@ void rowptr_from_sorted(const uint32_t* d_sorted_keys, long n, int K, int* d_row
     exclusive_scan(counts.p, d_rowptr, (long)K + 1, nullptr, s);
 }
 
-void csr_unique_from_pairs(const uint32_t* d_keys, const uint32_t* d_vals, long n, int K, int* d_rowptr, int* d_col,
-                           cudaStream_t s) {
-    if (K <= 0) {
-        VSDMO_CUDA(cudaMemsetAsync(d_rowptr, 0, sizeof(int), s));
-        return;
-    }
-    const long cap = std::max(n, 1L);
-    DBuf<int> counts(K, s), rs((long)K + 1, s), cursor(K, s), u(K, s);
-    DBuf<uint32_t> bucket(cap, s), uniq(cap, s);
-    DBuf<uint8_t> keep(cap, s);
-    counts.zero();
-    if (n > 0) {
-        k_count_keys<<<grid_for(n, 256), 256, 0, s>>>(d_keys, n, counts.p);
-        VSDMO_CHECK_LAUNCH();
-    }
-    exclusive_scan(counts.p, rs.p, K, rs.p + K, s);
-    if (n > 0 && longest_row(rs.p, K, s) > SHORT_ROW_MAX) {
-        // a row too long for one warp's quadratic scans: the same CSR from two stable radix sorts
-        // (by value, then by key) and the first pair of every run of equal pairs
-        DBuf<uint32_t> kk(n, s), vv(n, s);
-        DBuf<int> idx(n, s);
-        VSDMO_CUDA(cudaMemcpyAsync(kk.p, d_keys, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
-        VSDMO_CUDA(cudaMemcpyAsync(vv.p, d_vals, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
-        radix_sort_pairs(vv.p, kk.p, n, 32, s);
-        radix_sort_pairs(kk.p, vv.p, n, bits_for((uint32_t)(K > 1 ? K - 1 : 1)), s);
-        u.zero();
-        k_flag_distinct<<<grid_for(n, 256), 256, 0, s>>>(kk.p, vv.p, n, keep.p, u.p);
-        VSDMO_CHECK_LAUNCH();
-        exclusive_scan(u.p, d_rowptr, K, d_rowptr + K, s);
-        const int nu = compact_flags(keep.p, n, idx.p, s);
-        if (nu > 0) {
-            k_gather_col<<<grid_for(nu, 256), 256, 0, s>>>(vv.p, idx.p, nu, d_col);
-            VSDMO_CHECK_LAUNCH();
-        }
-        return;
-    }
-    VSDMO_CUDA(cudaMemcpyAsync(cursor.p, rs.p, sizeof(int) * K, cudaMemcpyDeviceToDevice, s));
-    if (n > 0) {
-        k_bucket_scatter<<<grid_for(n, 256), 256, 0, s>>>(d_keys, d_vals, n, cursor.p, bucket.p);
-        VSDMO_CHECK_LAUNCH();
-    }
-    k_row_unique<<<grid_for((long)K * 32, 256), 256, 0, s>>>(rs.p, bucket.p, K, keep.p, uniq.p, u.p);
-    VSDMO_CHECK_LAUNCH();
-    exclusive_scan(u.p, d_rowptr, K, d_rowptr + K, s);
-    k_row_copy<<<grid_for((long)K * 32, 256), 256, 0, s>>>(rs.p, d_rowptr, uniq.p, K, d_col);
+void rows_from_slots(const uint32_t* d_keys, const int* d_slot, int* d_counts, long n, int K, int* d_rowptr,
+                     uint32_t* d_rows, cudaStream_t s) {
+    exclusive_scan(d_counts, d_rowptr, K, d_rowptr + K, s);
+    if (n <= 0) return;
+    k_scatter_slots<<<grid_for(n, 256), 256, 0, s>>>(d_keys, d_slot, d_rowptr, n, d_rows);
     VSDMO_CHECK_LAUNCH();
 }
 
-int stable_sort_short_rows(uint32_t* d_keys, uint32_t* d_order, long n, int K, int* d_rowptr, cudaStream_t s) {
-    if (K <= 0) return 0;
-    DBuf<int> counts(K, s), cursor(K, s);
-    DBuf<uint32_t> bucket(std::max(n, 1L), s);
+void order_short_rows(const int* d_rowptr, const uint32_t* d_rows, int K, uint32_t* d_order, uint32_t* d_keys,
+                      int* d_longest, cudaStream_t s) {
+    if (K <= 0) return;
+    k_row_order<<<grid_for((long)K * 32, 256), 256, 0, s>>>(d_rowptr, d_rows, K, d_order, d_keys, d_longest);
+    VSDMO_CHECK_LAUNCH();
+}
+
+void sort_short_rows(uint32_t* d_keys, uint32_t* d_order, long n, int K, int* d_rowptr, int* d_longest, cudaStream_t s) {
+    if (K <= 0) return;
+    DBuf<int> counts(K, s), slot(std::max(n, 1L), s);
+    DBuf<uint32_t> rows(std::max(n, 1L), s);
     counts.zero();
     if (n > 0) {
-        k_count_keys<<<grid_for(n, 256), 256, 0, s>>>(d_keys, n, counts.p);
+        k_count_slots<<<grid_for(n, 256), 256, 0, s>>>(d_keys, n, counts.p, slot.p);
         VSDMO_CHECK_LAUNCH();
     }
-    exclusive_scan(counts.p, d_rowptr, K, d_rowptr + K, s);
-    if (n <= 0) return 0;
-    const int longest = longest_row(d_rowptr, K, s);
-    if (longest > SHORT_ROW_MAX) {
-        // a row too long for one warp's quadratic scan: the stable radix sort gives the same arrays
-        k_iota_u32<<<grid_for(n, 256), 256, 0, s>>>(d_order, n);
-        VSDMO_CHECK_LAUNCH();
-        radix_sort_pairs(d_keys, d_order, n, bits_for((uint32_t)(K > 1 ? K - 1 : 1)), s);
-        return longest;
-    }
-    VSDMO_CUDA(cudaMemcpyAsync(cursor.p, d_rowptr, sizeof(int) * K, cudaMemcpyDeviceToDevice, s));
-    k_bucket_index<<<grid_for(n, 256), 256, 0, s>>>(d_keys, n, cursor.p, bucket.p);
+    rows_from_slots(d_keys, slot.p, counts.p, n, K, d_rowptr, rows.p, s);
+    order_short_rows(d_rowptr, rows.p, K, d_order, d_keys, d_longest, s);
+}
+
+void sort_long_rows(const uint32_t* d_keys, uint32_t* d_order, long n, int K, cudaStream_t s) {
+    DBuf<uint32_t> k(n, s);
+    VSDMO_CUDA(cudaMemcpyAsync(k.p, d_keys, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
+    k_iota_u32<<<grid_for(n, 256), 256, 0, s>>>(d_order, n);
     VSDMO_CHECK_LAUNCH();
-    k_row_order<<<grid_for((long)K * 32, 256), 256, 0, s>>>(d_rowptr, bucket.p, K, d_order, d_keys);
-    VSDMO_CHECK_LAUNCH();
-    return longest;
+    radix_sort_pairs(k.p, d_order, n, bits_for((uint32_t)(K > 1 ? K - 1 : 1)), s);
 }
 
 cudaMemPool_t device_pool() {

@@ -100,31 +100,33 @@ inline int grid_for(long n, int block, int cap = 148 * 32) {
 void exclusive_scan(const int* d_in, int* d_out, long n, int* d_total, cudaStream_t s);
 // Stable LSD radix sort of (key, value) pairs on the low `bits` bits of the keys.
 void radix_sort_pairs(uint32_t* keys, uint32_t* vals, long n, int bits, cudaStream_t s);
-// Stable compaction: out[j] = i for the flagged positions i, in increasing order; returns count.
-int compact_flags(const uint8_t* d_flags, long n, int* d_out_index, cudaStream_t s);
+// Stable compaction: out[j] = i for the flagged positions i, in increasing order; their number to
+// *d_total (may be null). No host read.
+void compact_flags(const uint8_t* d_flags, long n, int* d_out_index, int* d_total, cudaStream_t s);
 // stable partition of [0, n) into d_order: indices with (flag != 0) == first_value first, then
-// the rest, each in index order; returns the number of the first group (one host read)
-int stable_partition_flags(const uint8_t* d_flags, long n, int first_value, int* d_order, cudaStream_t s);
-// CSR (rows 0..K-1) of the distinct (key, value) pairs, each row's values ascending: the same
-// arrays as a stable sort by (key, value) followed by dropping repeats. d_rowptr holds K + 1
-// ints, d_col at least n.
-// stable sort of [0, n) by d_keys (values in [0, K)): d_order receives the original indices in
-// (key, index) order, d_keys the keys in that order and d_rowptr (K + 1 ints) the row starts,
-// the same arrays as radix_sort_pairs over (keys, 0..n-1) followed by rowptr_from_sorted. For
-// keys whose rows are short (a vertex's elements or halfedges): each row is ordered by one warp
-// in time quadratic in its length; above SHORT_ROW_MAX entries in a row, by the radix sort.
-// Returns the longest row (one host read).
-int stable_sort_short_rows(uint32_t* d_keys, uint32_t* d_order, long n, int K, int* d_rowptr, cudaStream_t s);
-void csr_unique_from_pairs(const uint32_t* d_keys, const uint32_t* d_vals, long n, int K, int* d_rowptr, int* d_col,
-                           cudaStream_t s);
+// the rest, each in index order; the size of the first group to *d_total. No host read.
+void partition_flags(const uint8_t* d_flags, long n, int first_value, int* d_order, int* d_total, cudaStream_t s);
+// Rows of [0, n) by key (keys in [0, K)) from counts per key and the place of each index within its
+// row (negative: left out): d_rowptr (K + 1 ints) and the indices of each row in arbitrary order.
+void rows_from_slots(const uint32_t* d_keys, const int* d_slot, int* d_counts, long n, int K, int* d_rowptr,
+                     uint32_t* d_rows, cudaStream_t s);
+// Rows of more entries than this are not ordered by one warp's quadratic scan; a surface mesh or a
+// tet mesh's face rows that need it are refused (VSDMO_E_VALENCE). The kernels' ring budgets (at
+// most 512 elements around a vertex) stay far below.
+constexpr int SHORT_ROW_MAX = 4096;
+// each row's indices ascending to d_order (longer rows as they are) and its key beside each (d_keys
+// may be null); *d_longest becomes the maximum of itself and the longest row
+void order_short_rows(const int* d_rowptr, const uint32_t* d_rows, int K, uint32_t* d_order, uint32_t* d_keys,
+                      int* d_longest, cudaStream_t s);
+// Stable sort of [0, n) by d_keys (values in [0, K)): d_order receives the original indices in
+// (key, index) order, d_keys the keys in that order and d_rowptr (K + 1 ints) the row starts, the
+// same arrays as radix_sort_pairs over (keys, 0..n-1), if no row is longer than SHORT_ROW_MAX;
+// else *d_longest says so and d_order holds valid indices in row order only. No host read.
+void sort_short_rows(uint32_t* d_keys, uint32_t* d_order, long n, int K, int* d_rowptr, int* d_longest, cudaStream_t s);
+// the same order for rows of any length, by the radix sort
+void sort_long_rows(const uint32_t* d_keys, uint32_t* d_order, long n, int K, cudaStream_t s);
 // CSR offsets [K+1] from n keys already sorted ascending (keys < K).
 void rowptr_from_sorted(const uint32_t* d_sorted_keys, long n, int K, int* d_rowptr, cudaStream_t s);
-// Rows longer than this are not ordered by one warp's quadratic scans: stable_sort_short_rows and
-// csr_unique_from_pairs switch to radix sorts, and the tet face pairing rejects the mesh
-// (VSDMO_E_VALENCE). The kernels' ring budgets (at most 512 elements around a vertex) stay far below.
-constexpr int SHORT_ROW_MAX = 4096;
-// longest row of a CSR row pointer d_rowptr[0..K] (one host read)
-int longest_row(const int* d_rowptr, long K, cudaStream_t s);
 int bits_for(uint32_t maxval);
 
 // ---- mesh (mesh_build.cu) ----------------------------------------------------------------
