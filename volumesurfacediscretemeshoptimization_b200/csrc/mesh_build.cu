@@ -99,9 +99,10 @@ __device__ __forceinline__ void smallest_first(int a, int b, int c, uint32_t* o)
 // exact repeat is a non-manifold input. A boundary face takes its place among the row's boundary faces in
 // (b, c) order, so rows in vertex order give the lexicographic order of a sort; rec collects
 // them in any order as (b << 32 | c, a << 32 | place) and u counts them per row.
-// Bound by the latency of the gathers. The rows live in shared memory (faces of up to FACE_CAP; longer
-// ones in their own part of spill). Five passes over lists of all faces in global memory before: 260 us
-// for 663,552 tets, 30 us now.
+// Bound by the instructions per face: rows of up to 32 faces (22 on average) pair them with one match
+// over the warp, longer ones scan the row; rows live in shared memory (up to FACE_CAP faces; longer ones in
+// their own part of spill). Five passes over lists of all faces in global memory before: 180 us for
+// 663,552 tets with cold caches, 58 us now (87 us with the scan for every row).
 constexpr int FACE_CAP = 160;
 constexpr int FACE_WARPS = 4;
 __global__ void __launch_bounds__(FACE_WARPS * 32)
@@ -115,36 +116,36 @@ k_tet_boundary(const int* __restrict__ rs, const uint32_t* __restrict__ inc, con
     const unsigned lt = (1u << lane) - 1u;
     const long nw = (long)gridDim.x * FACE_WARPS;
     for (long r = (long)blockIdx.x * FACE_WARPS + warp; r < K; r += nw) {
-        const int b0 = rs[r], m = 3 * (rs[r + 1] - b0);
+        const int b0 = rs[r], m = rs[r + 1] - b0;
         unsigned long long* f = sf[warp];
         uint8_t* bnd = sb[warp];
         int n = 0;
         for (int pass = 0; pass < 2; ++pass) {
             n = 0;
             for (int i0 = 0; i0 < m; i0 += 32) {
-                const int i = i0 + lane;
-                bool own = false;
-                uint32_t o[3];
-                if (i < m) {
-                    const uint32_t e = inc[b0 + i / 3];
-                    const int j = e & 3;
-                    const int4 t = tets[e >> 2];
-                    // the faces of corner j: all but the one opposite
-                    const int skip = j == 0 ? 2 : (j == 1 ? 3 : (j == 2 ? 1 : 0));
-                    const int face = i % 3 + (i % 3 >= skip ? 1 : 0);
-                    // corners of the face in order, two bits each
-                    const unsigned F = face == 0 ? (2u | 1u << 2 | 0u << 4) : face == 1 ? (0u | 1u << 2 | 3u << 4)
-                                     : face == 2 ? (1u | 2u << 2 | 3u << 4) : (0u | 3u << 2 | 2u << 4);
-                    const int p0 = F & 3, p1 = (F >> 2) & 3, p2 = F >> 4;
-                    const int a = p0 == 0 ? t.x : (p0 == 1 ? t.y : t.z), b = p1 == 1 ? t.y : (p1 == 2 ? t.z : t.w),
-                              c = p2 == 0 ? t.x : (p2 == 2 ? t.z : t.w);
-                    smallest_first(a, b, c, o);
-                    own = j == (a < b && a < c ? p0 : (b < a && b < c ? p1 : p2));
+                // lane: one tet and the three faces of corner j (all but the one opposite)
+                const bool has = i0 + lane < m;
+                const uint32_t e = has ? inc[b0 + i0 + lane] : 0u;
+                const int j = e & 3, skip = j == 0 ? 2 : (j == 1 ? 3 : (j == 2 ? 1 : 0));
+                const int4 t = tets[e >> 2];
+#pragma unroll
+                for (int face = 0; face < 4; ++face) {
+                    const int a = face == 0 ? t.z : (face == 2 ? t.y : t.x), b = face == 2 ? t.z : (face == 3 ? t.w : t.y),
+                              c = face == 0 ? t.x : (face == 3 ? t.z : t.w);
+                    const int first = a < b && a < c ? 0 : (b < a && b < c ? 1 : 2);
+                    // the place in the tet of the face's first vertex
+                    const int at0 = face == 0 ? 2 - first : face == 1 ? (first == 2 ? 3 : first) : face == 2 ? 1 + first
+                                  : (first == 0 ? 0 : 4 - first);
+                    const bool own = has && face != skip && at0 == j;
+                    const unsigned mask = __ballot_sync(FULL, own);
+                    const int at = n + __popc(mask & lt);
+                    if (own && (pass == 1 || at < FACE_CAP)) {
+                        uint32_t o[3];
+                        smallest_first(a, b, c, o);
+                        f[at] = ((unsigned long long)o[1] << 32) | o[2];
+                    }
+                    n += __popc(mask);
                 }
-                const unsigned mask = __ballot_sync(FULL, own);
-                const int at = n + __popc(mask & lt);
-                if (own && (pass == 1 || at < FACE_CAP)) f[at] = ((unsigned long long)o[1] << 32) | o[2];
-                n += __popc(mask);
             }
             if (pass == 1 || n <= FACE_CAP || n > SHORT_ROW_MAX) break;
             int at = 0;
@@ -159,17 +160,32 @@ k_tet_boundary(const int* __restrict__ rs, const uint32_t* __restrict__ inc, con
         }
         __syncwarp();
         int cnt = 0;
-        for (int i = lane; i < n; i += 32) {
-            const unsigned long long x = f[i], twin = (x << 32) | (x >> 32);
-            bool paired = false, repeat = false;
-            for (int j = 0; j < n; ++j) {
-                const unsigned long long y = f[j];
-                repeat |= y == x && j != i;
-                paired |= y == twin && j != i;
+        if (n <= 32) {
+            // one face per lane: its peers hold the same two vertices, in this order (a repeat) or the other (its twin)
+            const unsigned long long x = lane < n ? f[lane] : 0ull;
+            const unsigned p = (unsigned)(x >> 32), q = (unsigned)x;
+            const unsigned up = __ballot_sync(FULL, p < q), self = 1u << lane;
+            const unsigned peers = __match_any_sync(FULL, lane < n ? ((unsigned long long)min(p, q) << 32) | max(p, q)
+                                                                   : ~(unsigned long long)lane);
+            const unsigned same = (p < q ? up : ~up) & peers;
+            if (lane < n) {
+                if (same & ~self) atomicMax(err, BE_NONMANIFOLD);
+                bnd[lane] = peers == same ? 1 : 0;
+                cnt = bnd[lane];
             }
-            if (repeat) atomicMax(err, BE_NONMANIFOLD);
-            bnd[i] = paired ? 0 : 1;
-            cnt += paired ? 0 : 1;
+        } else {
+            for (int i = lane; i < n; i += 32) {
+                const unsigned long long x = f[i], twin = (x << 32) | (x >> 32);
+                bool paired = false, repeat = false;
+                for (int j = 0; j < n; ++j) {
+                    const unsigned long long y = f[j];
+                    repeat |= y == x && j != i;
+                    paired |= y == twin && j != i;
+                }
+                if (repeat) atomicMax(err, BE_NONMANIFOLD);
+                bnd[i] = paired ? 0 : 1;
+                cnt += paired ? 0 : 1;
+            }
         }
         cnt = __reduce_add_sync(FULL, cnt);
         if (lane == 0) u[r] = cnt;
@@ -317,8 +333,8 @@ __global__ void k_remap(int* idx, long n, const int* new_of_old) {
 // elements around it to list[(k - 1) * rs[original vertex]], their number beside the row start in
 // info. Neighbours seen more than once are dropped by a small table that keeps the last value of
 // each hash; the few it lets through twice change nothing. Bound by the latency of its gathers
-// (25 us for the 103,823 inner vertices of 663,552 tets); writing, bucketing, deduplicating and copying all
-// neighbour pairs as a CSR before: 450 us.
+// (47 us with cold caches for the 103,823 inner vertices of 663,552 tets); writing, bucketing, deduplicating
+// and copying all neighbour pairs as a CSR before: 445 us.
 constexpr int WAIT_TABLE = 128;
 template <int KC>
 __global__ void __launch_bounds__(128)
@@ -365,7 +381,7 @@ k_wait_lists(const int* __restrict__ rs, const uint32_t* __restrict__ inc, const
 // before (null for the first); when it is 0 nothing is left. A launch always colours the uncoloured vertex
 // of highest priority, so the launches end whatever the order the blocks run in. hist counts
 // the colours below 256, maxc collects the largest. Chains of waiting vertices pass within one
-// launch at the latency of a read through L2 (27 us for 103,823 vertices); a launch per
+// launch at the latency of a read through L2 (45 + 24 + 12 us for 103,823 vertices); a launch per
 // round before: 32 launches of up to 14 us.
 constexpr int COLOUR_TRIES = 32;
 __global__ void __launch_bounds__(256)
