@@ -21,6 +21,7 @@
 // restates it); with N = 8, 3 levels it is the reference kernel.
 #include "vsdmo_internal.cuh"
 #include "batch.cuh"
+#include "chain.cuh"
 #include "flat_search.cuh"
 #include <algorithm>
 #include <cfloat>
@@ -147,12 +148,13 @@ k_dmo_flat(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4*
 constexpr int F8_WARPS = 4;
 template <int FK>
 __global__ void __launch_bounds__(F8_WARPS * 32)
-k_dmo_flat8(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ he, int v0, int v1,
+k_dmo_flat8(float4* pos_, const int* __restrict__ rowptr, const int4* __restrict__ he, int v0, int v1,
             float gs, int depth, int maxk) {
     extern __shared__ float4 f8sm[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 3;
     float* sm = reinterpret_cast<float*>(f8sm) + (size_t)(w * 4 + g) * f8_group_floats(maxk);
     const int base = v0 + (blockIdx.x * F8_WARPS + w) * 4;
+    float4* pos = chain_wait(pos_);
     if (base >= v1) return;
     flat_search8<FK, false>(pos, rowptr, he, base + g, base + g < v1, gs, depth, sm, maxk, lane);
 }
@@ -392,13 +394,8 @@ bool launch_dmo_flat_packed(const Mesh& m, const DmoLaunch& L, cudaStream_t s) {
     if (n < FLAT_PACKED_MIN || maxk > F8_MAX_RING) return false;
     prepare_flat_kernels();
     const int blocks = (n + 4 * F8_WARPS - 1) / (4 * F8_WARPS);
-    if (m.fk == 4)
-        k_dmo_flat8<4><<<blocks, F8_WARPS * 32, flat8_smem(maxk), s>>>(m.pos.p, m.he_rowptr.p, m.he.p, L.v0, L.v1, L.grid_scale,
-                                                                       L.depth, maxk);
-    else
-        k_dmo_flat8<3><<<blocks, F8_WARPS * 32, flat8_smem(maxk), s>>>(m.pos.p, m.he_rowptr.p, m.he.p, L.v0, L.v1, L.grid_scale,
-                                                                       L.depth, maxk);
-    VSDMO_CHECK_LAUNCH();
+    VSDMO_CUDA(launch_chained(m.fk == 4 ? k_dmo_flat8<4> : k_dmo_flat8<3>, blocks, F8_WARPS * 32, flat8_smem(maxk), s, L.chained,
+                              m.pos.p, m.he_rowptr.p, m.he.p, L.v0, L.v1, L.grid_scale, L.depth, maxk));
     return true;
 }
 

@@ -53,9 +53,11 @@ void copy_in(void* dst, const void* src, size_t bytes, int mem_space, cudaStream
     VSDMO_CUDA(cudaMemcpyAsync(dst, src, bytes, mem_space == VSDMO_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
 }
 
-void launch_color(vsdmo_opt_s* o, int c, cudaStream_t s) {
+// follows: the class before this one was launched on the stream just before
+void launch_color(vsdmo_opt_s* o, int c, cudaStream_t s, bool follows = false) {
     const Mesh& m = o->mesh->m;
     DmoLaunch L{o->ranges[c].first, o->ranges[c].second, o->p.grid_scale, o->p.depth};
+    L.chained = follows && !(o->mode == MODE_SURF && o->feat);   // there a copy of the positions comes between
     if (o->mode == MODE_TET && o->model) {
         // learned proposal: ring features + network (one fused tensor-core kernel) -> reduced
         // grid around the proposal -> plain search for the vertices it did not improve
@@ -106,7 +108,7 @@ void run_iteration_body(vsdmo_opt_s* o, cudaStream_t s) {
     if (o->mode == MODE_TET && o->model && o->proposals_once)
         o->model->m.infer_tet(m.pos.p, o->nb.p, o->nbn.p, o->nb_base, o->nb_base, m.nV - o->nb_base, o->Yall.p,
                               mlp::OUTP, s);
-    for (int c = 0; c < (int)o->ranges.size(); ++c) launch_color(o, c, s);
+    for (int c = 0; c < (int)o->ranges.size(); ++c) launch_color(o, c, s, c > 0);
     if (o->volsurf) {
         // boundary passes of a volume mesh, only while the last minimum quality is positive
         // (DMOTetClass::doIteration, dmo/DMOTet.cu:128-170; DMOHexClass::doIteration,
@@ -141,7 +143,7 @@ void run_iteration_body(vsdmo_opt_s* o, cudaStream_t s) {
     if (o->mode == MODE_SURF || o->slide) launch_update_nn(m, o->X0.p, o->nn.p, s);
     if (o->mode == MODE_SURF) update_normals(m, s);
     launch_quality_stats(m, o->kind, o->stats.p, o->d_iter.p, o->pmin.p, o->psum.p, o->pfail.p, o->done.p,
-                         o->p.check_monotone ? 1 : 0, s);
+                         o->p.check_monotone ? 1 : 0, s, !o->ranges.empty());
 }
 
 __global__ void k_surface_state(const float4* pos, int nS, float4* X0, int* nn) {

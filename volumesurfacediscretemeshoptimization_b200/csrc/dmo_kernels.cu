@@ -26,6 +26,7 @@
 // (dmo/DMOTet.cu:45-67) in one deterministic launch; k_quality_histogram and
 // k_element_qualities replace k_qualityHistogram / k_getElementQualities (dmo/DMOTet.cu:31-43,69-75).
 #include "vsdmo_internal.cuh"
+#include "chain.cuh"
 #include "tc_gemm.cuh"
 #include "angle_metrics.cuh"
 #include "tet_search.cuh"
@@ -51,12 +52,6 @@ constexpr int TET_MIN_BLOCKS = 28;   // 72 registers
 constexpr int TRI_WARPS = 4;
 constexpr int TET_MAX_RING = 512;
 constexpr int TRI_MAX_RING = 256;
-
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(FULL, v, o));
-    return v;
-}
 
 // (key, index): larger key wins, equal keys -> lower index (cub::ArgMax semantics)
 __device__ __forceinline__ void warp_argmax(float& k, int& i) {
@@ -107,12 +102,10 @@ __device__ __forceinline__ float tet_key_min(const float4* __restrict__ co, int 
 // (14 instead of 72 gathers for a Kuhn vertex) and two dependent loads reach the positions
 // instead of three (row pointer, halffaces, positions). Larger rings read their halffaces twice.
 __device__ __forceinline__ int tet_setup(const float4* __restrict__ pos, const int* __restrict__ rowptr,
-                                         const int4* __restrict__ hf, const TetRingTable& ring, int v, int maxk,
+                                         const int4* __restrict__ hf, unsigned corner, int nb, int v, int maxk,
                                          float4 c0, int lane, float4* co, float4* scratch, float& sx, float& sy,
                                          float& sz, int& ex) {
-    const size_t row = (size_t)(v - ring.base) * 32 + lane;
-    const unsigned corner = ring.corner[row];
-    const float4 q = pos[ring.nb[row]];
+    const float4 q = pos[nb];
     const unsigned has = __ballot_sync(FULL, corner != TetRingTable::NONE);
     if (__any_sync(FULL, corner == TetRingTable::LARGE)) {
         float mdx = 0.f, mdy = 0.f, mdz = 0.f;
@@ -186,17 +179,21 @@ k_dmo_tet(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* 
     extern __shared__ float4 smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int v = v0 + blockIdx.x * TET_WARPS + w;
-    if (v >= v1) return;
-    if (dirty && !dirty[v]) {
+    // the wait's pointer serves the loads only: one that lived through the search would cost two registers
+    const size_t row = (size_t)(v - ring.base) * 32 + lane;
+    const unsigned corner = ring.corner[row];
+    const int nb = ring.nb[row];
+    const float4* p = chain_wait(pos);
+    if (dirty && !*(volatile uint8_t*)(dirty + v)) {
         if (lane == 0 && skipped) atomicAdd(skipped, 1ull);
         return;
     }
     float4* co = smem + (size_t)w * maxk * 2;
     float* scratch = reinterpret_cast<float*>(smem + (size_t)TET_WARPS * maxk * 2) + w * (TS_WARP_BYTES / 4);
-    const float4 c0 = pos[v];
+    const float4 c0 = p[v];
     float sx, sy, sz;
     int ex;
-    const int k = tet_setup(pos, rowptr, hf, ring, v, maxk, c0, lane, co, reinterpret_cast<float4*>(scratch), sx, sy, sz, ex);
+    const int k = tet_setup(p, rowptr, hf, corner, nb, v, maxk, c0, lane, co, reinterpret_cast<float4*>(scratch), sx, sy, sz, ex);
     if (k == 0) return;
     const float qLast = tet_group_key(co, k, 0.f, 0.f, 0.f, 32, lane);
     float dx, dy, dz;
@@ -227,7 +224,8 @@ k_dmo_tet_list(float4* __restrict__ pos, const int* __restrict__ rowptr, const i
         const float4 c0 = pos[v];
         float sx, sy, sz;
         int ex;
-        const int k = tet_setup(pos, rowptr, hf, ring, v, maxk, c0, lane, co, reinterpret_cast<float4*>(scratch), sx, sy,
+        const size_t row = (size_t)(v - ring.base) * 32 + lane;
+        const int k = tet_setup(pos, rowptr, hf, ring.corner[row], ring.nb[row], v, maxk, c0, lane, co, reinterpret_cast<float4*>(scratch), sx, sy,
                                 sz, ex);
         if (k == 0) continue;
         const float qLast = tet_group_key(co, k, 0.f, 0.f, 0.f, 32, lane);
@@ -463,7 +461,8 @@ k_dmo_tet_learned(float4* __restrict__ pos, const int* __restrict__ rowptr, cons
     float sx, sy, sz;
     int ex;
     float4* scratch = smem + (size_t)TET_WARPS * maxk * 2 + w * 32;
-    const int k = tet_setup(pos, rowptr, hf, ring, v, maxk, c0, lane, co, scratch, sx, sy, sz, ex);
+    const size_t row = (size_t)(v - ring.base) * 32 + lane;
+    const int k = tet_setup(pos, rowptr, hf, ring.corner[row], ring.nb[row], v, maxk, c0, lane, co, scratch, sx, sy, sz, ex);
     if (k == 0) return;
     const float q0 = tet_key_min(co, k, 0.f, 0.f, 0.f, lane);
     // proposal in scaled local coordinates (the features were divided by mm = max(sx, sy, sz) 2^ex)
@@ -640,32 +639,64 @@ __device__ __forceinline__ float tri_key(const float4* co, int k, float x, float
     return am < 0.f ? am : N / D;
 }
 
+// tri_key of (x1, y) and (x2, y): one pass over the ring, the two folds' chains side by side
+__device__ __forceinline__ void tri_key2(const float4* co, int k, float x1, float x2, float y, float& q1, float& q2) {
+    const float t1 = (2.0f * x1) * x1, t2 = (2.0f * x2) * x2, ty = (2.0f * y) * y;
+    float N1 = 0.f, D1 = 1.f, a1 = 0.f, N2 = 0.f, D2 = 1.f, a2 = 0.f;
+    for (int t = 0; t < k; ++t) {
+        const float4 c0 = co[2 * t], c1 = co[2 * t + 1];
+        const float A1 = fmaf(c0.y, y, fmaf(c0.x, x1, c0.z)), A2 = fmaf(c0.y, y, fmaf(c0.x, x2, c0.z));
+        const float L1 = (c0.w + fmaf(c1.x, x1, t1)) + fmaf(c1.y, y, ty), L2 = (c0.w + fmaf(c1.x, x2, t2)) + fmaf(c1.y, y, ty);
+        if (t == 0 || A1 * D1 < N1 * L1) { N1 = A1; D1 = L1; }
+        if (t == 0 || A2 * D2 < N2 * L2) { N2 = A2; D2 = L2; }
+        a1 = t == 0 ? A1 : fminf(a1, A1);
+        a2 = t == 0 ? A2 : fminf(a2, A2);
+    }
+    q1 = a1 < 0.f ? a1 : N1 / D1;
+    q2 = a2 < 0.f ? a2 : N2 / D2;
+}
+
+// One warp per vertex, a class of a few hundred vertices at a time: bound by the latency of its own chain (topology,
+// positions, coefficients, three levels). Chained launches (chain.cuh), the ring read once, both candidates
+// of a lane in one pass and the winner by a warp reduction: 44.9 -> 32.2 us per iteration of the 64^2 grid.
 __global__ void __launch_bounds__(TRI_WARPS * 32)
 k_dmo_tri2d(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ he,
             int v0, int v1, float grid_scale, int depth, int maxk) {
     extern __shared__ float4 smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int v = v0 + blockIdx.x * TRI_WARPS + w;
-    if (v >= v1) return;
     float4* co = smem + (size_t)w * maxk * 2;
-    const int b = rowptr[v], k = rowptr[v + 1] - b;
+    int b = 0, k = 0, first = 0;
+    if (v < v1) {
+        b = rowptr[v];
+        k = rowptr[v + 1] - b;
+        if (lane < k) first = he[b + lane].x;
+    }
+    const float4* src = chain_wait(pos);
     if (k <= 0 || k > maxk) return;
-    const float4 c0 = pos[v];
+    const float4 c0 = src[v];
+    float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f);
     float mdx = 0.f, mdy = 0.f;
     for (int t = lane; t < k; t += 32) {
-        const float4 p = pos[he[b + t].x];
+        const float4 p = src[t == lane ? first : he[b + t].x];
+        if (t == lane) p0 = p;
         mdx = fmaxf(mdx, fabsf(p.x - c0.x));
         mdy = fmaxf(mdy, fabsf(p.y - c0.y));
     }
-    mdx = warp_max(mdx); mdy = warp_max(mdy);
+    mdx = redux_max(mdx); mdy = redux_max(mdy);
     const float mm = fmaxf(mdx, mdy);
     if (!(mm > 0.f) || !(mm < FLT_MAX)) return;
     int ex;
     (void)frexpf(mm, &ex);
     const float p = exp2_exact(-ex);
+    // rings of up to 32 points lie in the lanes' registers
+    const float nx = __shfl_sync(FULL, p0.x, lane + 1 < k ? lane + 1 : 0), ny = __shfl_sync(FULL, p0.y, lane + 1 < k ? lane + 1 : 0);
     for (int t = lane; t < k; t += 32) {
-        const float4 pa = pos[he[b + t].x];
-        const float4 pb = pos[he[b + (t + 1 == k ? 0 : t + 1)].x];
+        float4 pa = p0, pb = make_float4(nx, ny, 0.f, 0.f);
+        if (k > 32) {
+            pa = src[he[b + t].x];
+            pb = src[he[b + (t + 1 == k ? 0 : t + 1)].x];
+        }
         const float ax = scale2(pa.x - c0.x, p, -ex), ay = scale2(pa.y - c0.y, p, -ex);
         const float bx = scale2(pb.x - c0.x, p, -ex), by = scale2(pb.y - c0.y, p, -ex);
         const float ux = bx - ax, uy = by - ay;
@@ -684,14 +715,19 @@ k_dmo_tri2d(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4
     for (int level = 0; level < depth; ++level) {
         const float Sx = ds * sx, Sy = ds * sy;
         const float x1 = fmaf(o1, Sx, dx), x2 = fmaf(o2, Sx, dx), y = fmaf(oj, Sy, dy);
-        const float q1 = tri_key(co, k, x1, y);
-        const float q2 = tri_key(co, k, x2, y);
+        float q1, q2;
+        tri_key2(co, k, x1, x2, y, q1, q2);
         float val = q1;
         if (q2 > q1) val = q2;
         const float selx = (q1 > q2) ? x1 : x2;
         float bv = val;
         int bl = lane;
-        warp_argmax(bv, bl);
+        if (__any_sync(FULL, val != val)) {
+            warp_argmax(bv, bl);
+        } else {
+            bl = __ffs(__ballot_sync(FULL, val == redux_max(val))) - 1;
+            bv = __shfl_sync(FULL, val, bl);
+        }
         if (qLast < bv) {
             dx = __shfl_sync(FULL, selx, bl);
             dy = __shfl_sync(FULL, y, bl);
@@ -876,12 +912,13 @@ constexpr int QS_THREADS = 256;
 constexpr int QS_UNROLL = 4;
 
 __global__ void __launch_bounds__(QS_THREADS)
-k_quality_stats(const int* __restrict__ el, int kind, long nE, const float4* __restrict__ pos, IterStats* stats,
+k_quality_stats(const int* __restrict__ el, int kind, long nE, const float4* pos_, IterStats* stats,
                 int* iter, float* pmin, double* psum, int* pfail, unsigned* done, int check, int init) {
     __shared__ float smin[QS_THREADS / 32];
     __shared__ double ssum[QS_THREADS / 32];
     __shared__ int sfail[QS_THREADS / 32];
     __shared__ bool last;
+    const float4* pos = chain_wait(pos_);
     const int it = *iter;
     const float lastMin = init ? -FLT_MAX : stats[it].min_q;
     const float tol = 1e-6f * fmaxf(fabsf(lastMin), 1e-30f);
@@ -1035,9 +1072,8 @@ void launch_dmo_tet(const Mesh& m, const DmoLaunch& L, const TetRingTable& ring,
     if (n <= 0) return;
     const int maxk = m.maxTets;
     const size_t smem = tet_smem_bytes(maxk);
-    k_dmo_tet<<<(n + TET_WARPS - 1) / TET_WARPS, TET_WARPS * 32, smem, s>>>(
-        m.pos.p, m.hf_rowptr.p, m.hf.p, ring, L.v0, L.v1, L.grid_scale, L.depth, maxk, dirty, skipped);
-    VSDMO_CHECK_LAUNCH();
+    VSDMO_CUDA(launch_chained(k_dmo_tet, (n + TET_WARPS - 1) / TET_WARPS, TET_WARPS * 32, smem, s, L.chained, m.pos.p,
+                              m.hf_rowptr.p, m.hf.p, ring, L.v0, L.v1, L.grid_scale, L.depth, maxk, dirty, skipped));
 }
 
 // Active set with a free boundary: the boundary passes move vertices whose rings hold interior
@@ -1101,19 +1137,17 @@ void launch_dmo_tri2d(const Mesh& m, const DmoLaunch& L, cudaStream_t s) {
     if (n <= 0) return;
     const int maxk = m.maxHE;
     const size_t smem = (size_t)TRI_WARPS * maxk * 2 * sizeof(float4);
-    k_dmo_tri2d<<<(n + TRI_WARPS - 1) / TRI_WARPS, TRI_WARPS * 32, smem, s>>>(
-        m.pos.p, m.he_rowptr.p, m.he.p, L.v0, L.v1, L.grid_scale, L.depth, maxk);
-    VSDMO_CHECK_LAUNCH();
+    VSDMO_CUDA(launch_chained(k_dmo_tri2d, (n + TRI_WARPS - 1) / TRI_WARPS, TRI_WARPS * 32, smem, s, L.chained, m.pos.p,
+                              m.he_rowptr.p, m.he.p, L.v0, L.v1, L.grid_scale, L.depth, maxk));
 }
 
 void launch_quality_stats(const Mesh& m, int kind, IterStats* d_stats, int* d_iter, float* d_partial_min,
                           double* d_partial_sum, int* d_partial_fail, unsigned* d_done, int check_monotone,
-                          cudaStream_t s) {
+                          cudaStream_t s, bool chained) {
     // check_monotone < 0 marks the initial evaluation (slot 0, no check, no increment)
     const int init = check_monotone < 0 ? 1 : 0;
-    k_quality_stats<<<QS_BLOCKS, QS_THREADS, 0, s>>>(m.elems.p, kind, m.nE, m.pos.p, d_stats, d_iter, d_partial_min,
-                                                     d_partial_sum, d_partial_fail, d_done, init ? 0 : check_monotone, init);
-    VSDMO_CHECK_LAUNCH();
+    VSDMO_CUDA(launch_chained(k_quality_stats, QS_BLOCKS, QS_THREADS, 0, s, chained, m.elems.p, kind, m.nE, m.pos.p, d_stats,
+                              d_iter, d_partial_min, d_partial_sum, d_partial_fail, d_done, init ? 0 : check_monotone, init));
 }
 
 void launch_element_qualities(const Mesh& m, int kind, float* d_out, cudaStream_t s) {

@@ -34,6 +34,7 @@
 // operation order, reproduced by the oracle's f32 mirror bit for bit (built with
 // --fmad=false here and without contraction there).
 #include "vsdmo_internal.cuh"
+#include "chain.cuh"
 #include "f32x2.cuh"
 #include "tet_key.cuh"
 #include "hex_key.cuh"
@@ -687,23 +688,24 @@ k_dmo_surf(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4*
     extern __shared__ float4 smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int v = v0 + blockIdx.x * SURF_WARPS + warp;
-    if (v >= v1) return;
-    const int b = rowptr[v], k = rowptr[v + 1] - b;
+    const int b = v < v1 ? rowptr[v] : 0, k = v < v1 ? rowptr[v + 1] - b : 0;
+    const int4 first = lane < k ? he[b + lane] : make_int4(0, 0, 0, 0);
+    const float4* src = chain_wait(pos);
     if (k <= 0 || k > maxk) return;   // maxk is the mesh's largest row, checked on the host
     float4* ring = smem + (size_t)warp * surf_search_f4(FK, Q, maxk);
     float4* nbL = ring + (PACKED ? maxk + 1 : 2 * maxk + 1);
     float4* nbX = nbL + 4 * maxk;
-    const float4 c0 = pos[v];
+    const float4 c0 = src[v];
     float md = 0.f;
     for (int i = lane; i < k; i += 32) {
-        const int4 h = he[b + i];
-        const float4 t = pos[h.x];
+        const int4 h = i < 32 ? first : he[b + i];
+        const float4 t = src[h.x];
         float dx = t.x - c0.x, dy = t.y - c0.y, dz = t.z - c0.z;
         md = fmaxf(md, sqrtf(dot3(dx, dy, dz, dx, dy, dz)));
         if (FK == 3) {
             ring[i] = t;
         } else {
-            const float4 t2 = pos[he[h.w].x];
+            const float4 t2 = src[he[h.w].x];
             ring[2 * i] = t;
             ring[2 * i + 1] = t2;
             dx = t2.x - c0.x; dy = t2.y - c0.y; dz = t2.z - c0.z;
@@ -1367,10 +1369,9 @@ void launch_dmo_surf(const Mesh& m, const DmoLaunch& L, const float4* X0, const 
     const int blocks = (n + SURF_WARPS - 1) / SURF_WARPS;
     auto k = m.fk == 4 ? (crit == 3 ? k_dmo_surf<4, 3> : k_dmo_surf<4, 0>)
                        : (crit == 1 ? k_dmo_surf<3, 1> : (crit == 2 ? k_dmo_surf<3, 2> : k_dmo_surf<3, 0>));
-    k<<<blocks, SURF_WARPS * 32, smem, s>>>(m.pos.p, m.he_rowptr.p, m.he.p, X0, LS, nn, m.vn.p, L.v0, L.v1, L.grid_scale,
-                                            L.depth, maxk, sec ? sec->srow : nullptr, sec ? sec->stab : nullptr,
-                                            sec ? sec->FS : nullptr, sec ? sec->Xs : nullptr, m.nSurf - m.nFeature);
-    VSDMO_CHECK_LAUNCH();
+    VSDMO_CUDA(launch_chained(k, blocks, SURF_WARPS * 32, smem, s, L.chained, m.pos.p, m.he_rowptr.p, m.he.p, X0, LS, nn, m.vn.p,
+                              L.v0, L.v1, L.grid_scale, L.depth, maxk, sec ? sec->srow : nullptr, sec ? sec->stab : nullptr,
+                              sec ? sec->FS : nullptr, sec ? sec->Xs : nullptr, m.nSurf - m.nFeature));
 }
 
 void init_feature_state(const Mesh& m, int flat, float4* LS1, int* fdeg, uint8_t* opt, cudaStream_t s) {

@@ -170,6 +170,7 @@ struct DmoLaunch {
     int v0, v1;          // vertex range of one colour class
     float grid_scale;
     int depth;
+    bool chained = false;   // follows a kernel on the stream that the launch may overlap (chain.cuh)
 };
 // Ring table of the inner vertices of a tet mesh (k_tet_rings), rows of 32 from vertex base on
 struct TetRingTable {
@@ -291,7 +292,7 @@ struct IterStats {
 // against min of the previous slot (or init_min for slot 0), then ++*d_iter.
 void launch_quality_stats(const Mesh& m, int kind, IterStats* d_stats, int* d_iter, float* d_partial_min,
                           double* d_partial_sum, int* d_partial_fail, unsigned* d_done, int check_monotone,
-                          cudaStream_t s);
+                          cudaStream_t s, bool chained = false);
 void launch_element_qualities(const Mesh& m, int kind, float* d_out, cudaStream_t s);
 void launch_quality_histogram(const Mesh& m, int kind, int* d_counts, int n_cols, cudaStream_t s);
 int quality_stats_blocks();
