@@ -1093,6 +1093,7 @@ k_dmo_1d(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* _
     }
     float3 n = make_float3(0.f, 0.f, 0.f);
     if (MODE != 0) n = make_float3(vn[3L * nnv], vn[3L * nnv + 1], vn[3L * nnv + 2]);
+    float qLast = ring_q1d<MODE, true, Q>(ring, ne, c0.x, c0.y, c0.z, n);   // key of (cx, cy, cz)
     float cx = c0.x, cy = c0.y, cz = c0.z;
     const float aff = 1.f / 7.f;
     float ds = grid_scale, lastMax = -FLT_MAX;
@@ -1112,10 +1113,9 @@ k_dmo_1d(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* _
             const float qt = __shfl_sync(FULL, q, t);
             if (qt > bv) { bv = qt; bt = t; }
         }
-        const float qLast = ring_q1d<MODE, true, Q>(ring, ne, cx, cy, cz, n);
         const float bu = __shfl_sync(FULL, u, bt);
         const float bx = __shfl_sync(FULL, p.x, bt), by = __shfl_sync(FULL, p.y, bt), bz = __shfl_sync(FULL, p.z, bt);
-        if (qLast < bv) { cx = bx; cy = by; cz = bz; cu = bu; }
+        if (qLast < bv) { cx = bx; cy = by; cz = bz; cu = bu; qLast = bv; }
         lastMax = bv;
         ds = ds * (2.f / 7.f);
     }
@@ -1168,6 +1168,7 @@ k_dmo_surf_vol(float4* __restrict__ pos, const int* __restrict__ rowptr, const i
         cv = dot3(dx, dy, dz, L.l2.x, L.l2.y, L.l2.z);
     }
     const float qOld = ring.key(c0.x, c0.y, c0.z);
+    float qLast = qOld;   // key of (cx, cy, cz)
     const int i1 = lane >> 3, j1 = lane & 7, i2 = i1 + 4;
     const float o1 = (float)(7 - 2 * i1) / 7.f, oj = (float)(7 - 2 * j1) / 7.f, o2 = (float)(7 - 2 * i2) / 7.f;
     float cx = c0.x, cy = c0.y, cz = c0.z;
@@ -1180,20 +1181,15 @@ k_dmo_surf_vol(float4* __restrict__ pos, const int* __restrict__ rowptr, const i
         const float q1 = ring.key(p1.x, p1.y, p1.z);
         const float q2 = ring.key(p2.x, p2.y, p2.z);
         const bool second = q2 > q1;
-        const float val = second ? q2 : q1;
-        float bv = __shfl_sync(FULL, val, 0);
-        int bt = 0;
-        for (int t = 1; t < 32; ++t) {
-            const float vt = __shfl_sync(FULL, val, t);
-            if (vt > bv) { bv = vt; bt = t; }
-        }
-        const float qLast = ring.key(cx, cy, cz);
+        float bv;
+        int bt;
+        first_max(second ? q2 : q1, bv, bt);
         const float bu = __shfl_sync(FULL, second ? u2 : u1, bt);
         const float bw = __shfl_sync(FULL, vv, bt);
         const float bx = __shfl_sync(FULL, second ? p2.x : p1.x, bt);
         const float by = __shfl_sync(FULL, second ? p2.y : p1.y, bt);
         const float bz = __shfl_sync(FULL, second ? p2.z : p1.z, bt);
-        if (qLast < bv) { cx = bx; cy = by; cz = bz; cu = bu; cv = bw; }
+        if (qLast < bv) { cx = bx; cy = by; cz = bz; cu = bu; cv = bw; qLast = bv; }
         lastMax = bv;
         ds = ds * (2.0f / 7.0f);
     }
@@ -1243,6 +1239,8 @@ k_dmo_1d_vol(float4* __restrict__ pos, const int* __restrict__ rowptr, const int
         const float qx = c0.x - l0.x, qy = c0.y - l0.y, qz = c0.z - l0.z;
         cu = dot3(qx, qy, qz, l1.x, l1.y, l1.z);
     }
+    const float qOld = ring.key(c0.x, c0.y, c0.z);
+    float qLast = qOld;   // key of (cx, cy, cz)
     float cx = c0.x, cy = c0.y, cz = c0.z;
     const float aff = 1.f / 7.f;
     float ds = grid_scale, lastMax = -FLT_MAX;
@@ -1262,14 +1260,12 @@ k_dmo_1d_vol(float4* __restrict__ pos, const int* __restrict__ rowptr, const int
             const float qt = __shfl_sync(FULL, q, t);
             if (qt > bv) { bv = qt; bt = t; }
         }
-        const float qLast = ring.key(cx, cy, cz);
         const float bu = __shfl_sync(FULL, u, bt);
         const float bx = __shfl_sync(FULL, p.x, bt), by = __shfl_sync(FULL, p.y, bt), bz = __shfl_sync(FULL, p.z, bt);
-        if (qLast < bv) { cx = bx; cy = by; cz = bz; cu = bu; }
+        if (qLast < bv) { cx = bx; cy = by; cz = bz; cu = bu; qLast = bv; }
         lastMax = bv;
         ds = ds * (2.f / 7.f);
     }
-    const float qOld = ring.key(c0.x, c0.y, c0.z);
     if (lane == 0 && qOld < lastMax) pos[v] = make_float4(cx, cy, cz, c0.w);
 }
 
