@@ -60,6 +60,27 @@ static __device__ float tet_key1(const float4* co, int k, float x, float y, floa
     return dm < 0.f ? dm : N / D;
 }
 
+// tet_key1 of two candidates, the two folds' chains side by side in one pass over the ring
+static __device__ void tet_key2(const float4* co, int k, float x0, float y0, float z0, float x1, float y1, float z1, float& q0, float& q1) {
+    const float tx0 = (3.0f * x0) * x0, ty0 = (3.0f * y0) * y0, tz0 = (3.0f * z0) * z0;
+    const float tx1 = (3.0f * x1) * x1, ty1 = (3.0f * y1) * y1, tz1 = (3.0f * z1) * z1;
+    float N0 = 0.f, D0 = 1.f, m0 = 0.f, N1 = 0.f, D1 = 1.f, m1 = 0.f;
+#pragma unroll 2
+    for (int t = 0; t < k; ++t) {
+        const float4 c0 = co[2 * t], c1 = co[2 * t + 1];
+        const float d0 = fmaf(c0.z, z0, fmaf(c0.y, y0, fmaf(c0.x, x0, c0.w))), d1 = fmaf(c0.z, z1, fmaf(c0.y, y1, fmaf(c0.x, x1, c0.w)));
+        const float L0 = ((c1.w + fmaf(c1.x, x0, tx0)) + fmaf(c1.y, y0, ty0)) + fmaf(c1.z, z0, tz0);
+        const float L1 = ((c1.w + fmaf(c1.x, x1, tx1)) + fmaf(c1.y, y1, ty1)) + fmaf(c1.z, z1, tz1);
+        const float n0 = d0 * d0, n1 = d1 * d1, e0 = (L0 * L0) * L0, e1 = (L1 * L1) * L1;
+        if (t == 0 || n0 * D0 < N0 * e0) { N0 = n0; D0 = e0; }
+        if (t == 0 || n1 * D1 < N1 * e1) { N1 = n1; D1 = e1; }
+        m0 = t == 0 ? d0 : fminf(m0, d0);
+        m1 = t == 0 ? d1 : fminf(m1, d1);
+    }
+    q0 = m0 < 0.f ? m0 : N0 / D0;
+    q1 = m1 < 0.f ? m1 : N1 / D1;
+}
+
 // tet_key1 at the local origin (the vertex itself): det = d0 and L = C exactly there (every term
 // that carries the candidate is a product with +-0 added to them), so the same fold runs on the
 // constant coefficients alone and returns the same key
