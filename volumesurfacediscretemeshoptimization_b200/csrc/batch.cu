@@ -34,11 +34,18 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int BATCH_WARPS = 8;
-// vertices of a colour class from which on four vertices share a warp: below, a warp per vertex is the
+// vertices of a single mesh's colour class from which on four vertices share a warp: below, a warp per vertex is the
 // shorter chain and fits in one wave (flat triangles / quads, ms per iteration, packed against not:
 // 64^2 (classes of 550) 0.049 / 0.064 : 0.042 / 0.063; 128^2 (2,300) 0.053 / 0.065 : 0.057 / 0.079; 500^2
 // (35,000) 0.167 / 0.199 : 0.407 / 0.575)
 constexpr int FLAT_PACKED_MIN = 2048;
+// A work item of the batch is what one warp searches in sequence: up to eight steps, fewer where the classes
+// of all meshes together would leave resident warps without an item: eight steps always against this
+// rule 1.93 / 0.61 ms for 3 iterations of 33 meshes of up to 9,953 vertices, 13.9 / 13.9 for 256 of up to
+// 50,000. With items that short four vertices a warp win over a warp per vertex whatever the size (ms for
+// 10 iterations, unpacked / packed: 16 meshes of up to 2,000 vertices 1.55 / 1.12, 4 of up to 1,000
+// 1.05 / 0.94, 40 of up to 700 1.00 / 1.02).
+constexpr long BATCH_RESIDENT_WARPS = 148L * 4 * BATCH_WARPS;
 constexpr unsigned long long BWAIT_NS = 1000000000ull;
 // limit of a colour-class wait: BWAIT_NS unless the test-only vsdmo_debug_set_wait_limit_ns
 // lowered it to make waits expire
@@ -502,8 +509,8 @@ void Batch::build(const std::vector<MeshInput>& inputs, uint32_t seed) {
 
 int Batch::n_colors_total() const { return (int)csize.n; }
 
-// Meshes searched four vertices per warp: 8 x 8 grids whose rings fit, where the caller asks for 8 lanes
-// per vertex or the colour classes of the meshes in `sel` (all when empty) together fill the device.
+// Meshes searched four vertices per warp: 8 x 8 grids whose rings fit; and the size of a colour class over
+// the meshes in `sel` (all when empty), which sets the length of a work item.
 void Batch::choose_packed(const std::vector<int>& sel) {
     std::vector<int> ms = sel;
     if (ms.empty())
@@ -514,15 +521,18 @@ void Batch::choose_packed(const std::vector<int>& sel) {
         if (!hm[i].col.empty()) free_v += hm[i].col.back() - hm[i].col.front();
         maxc = std::max(maxc, hm[i].n_colors);
     }
-    const bool fills = free_v / maxc >= FLAT_PACKED_MIN;
+    class_avg = free_v / maxc;
     all_packed = true;
     for (int i : ms) {
-        hm[i].packed = cfg[i].nq == 8 && maxk <= F8_MAX_RING && (fills || cfg[i].lanes == 8);
+        hm[i].packed = cfg[i].nq == 8 && maxk <= F8_MAX_RING;
         all_packed = all_packed && hm[i].packed;
     }
 }
 
-int Batch::chunk(int i) const { return 8 * (hm[i].packed ? 4 : 32 / cfg[i].lanes); }
+int Batch::chunk(int i) const {
+    const int per = hm[i].packed ? 4 : 32 / cfg[i].lanes;   // vertices a warp searches at once
+    return per * (int)std::min(8L, std::max(1L, class_avg / (per * BATCH_RESIDENT_WARPS)));
+}
 
 void Batch::upload_meshes(const std::vector<int>& sel) {
     choose_packed(sel);
@@ -560,8 +570,7 @@ void Batch::invalidate_graph() {
 }
 
 // Work items of the meshes in `sel` (all when empty) in colour-major order: every mesh's colour
-// c before any mesh's colour c + 1. An item is a chunk of 8 steps of one warp (8 x the vertices a warp
-// searches at once).
+// c before any mesh's colour c + 1. An item is a chunk of up to 8 steps of one warp.
 std::vector<BatchItem> Batch::make_items(const std::vector<int>& sel) const {
     std::vector<int> ms = sel;
     if (ms.empty())

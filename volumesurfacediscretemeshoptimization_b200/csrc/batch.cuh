@@ -97,6 +97,7 @@ struct Batch {
     void set_positions(const float* d_xyz_in);
     int n_colors_total() const;
     int chunk(int i) const;       // vertices of one work item of mesh i
+    long class_avg = 0;           // vertices of a colour class over all meshes
 
    private:
     void choose_packed(const std::vector<int>& sel);

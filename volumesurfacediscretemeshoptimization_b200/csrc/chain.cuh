@@ -6,7 +6,7 @@
 // of a chained kernel calls chain_wait() before its first access to anything an earlier kernel
 // reads or writes, early returns included, so a kernel that has finished implies that all before it
 // have. Measured per iteration, plain against chained: flat triangles 64^2 (seven classes of 600 vertices) 36.2 /
-// 32.2 us, tets 10^3 1.108 / 1.059 ms for 20 iterations, tets 48^3 0.4035 / 0.400 ms, icosphere level 7 0.3914 /
+// 32.2 us, tets 10^3 1.108 / 1.035 ms for ten iterations, tets 48^3 0.4035 / 0.400 ms, icosphere level 7 0.3914 /
 // 0.3910 ms. k_dmo_hex stays plain: 0.551 / 0.561 ms (its blocks hold the shared memory of the class before it).
 #pragma once
 #include <cuda_runtime.h>
