@@ -172,11 +172,13 @@ __host__ __device__ constexpr int batch_warp_floats(int maxk) {
     return maxk > F8_MAX_RING || maxk * BCO > f8_group_floats(maxk) ? 4 * maxk * BCO : 4 * f8_group_floats(maxk);
 }
 
-// PACKED: every mesh is searched four vertices per warp (the other search stays out of the kernel:
-// with both in one, half the stalls were instruction fetches)
+// SEARCH: every mesh is searched four vertices per warp (PACKED), none is (GENERAL), or some are (MIXED): only
+// what is needed is in the kernel (with both in one, half the stalls were instruction fetches; 4 x 4 grids on 256
+// meshes, 32 / 8 lanes: 8.28 / 2.18 ms per iteration with both, 7.48 / 1.94 with the general search alone).
 // Registers: four blocks per SM at 64 (48 bytes of spills) against three at 80 and two at 96: 2.28 / 2.33
 // / 2.80 ms per iteration of 256 meshes.
-template <bool PACKED>
+enum { PACKED, GENERAL, MIXED };
+template <int SEARCH>
 __global__ void __launch_bounds__(BATCH_WARPS * 32, 4)
 k_batch_iter(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ he,
              const BatchItem* __restrict__ items, int n_items, const BatchMeshDev* __restrict__ meshes,
@@ -217,14 +219,16 @@ k_batch_iter(float4* __restrict__ pos, const int* __restrict__ rowptr, const int
                 continue;
             }
         }
-        if (PACKED || mh.packed) {
-            float* sm = wco + (size_t)(lane >> 3) * f8_group_floats(maxk);
-            for (int base = it.v0; base < it.v1; base += 4) {
-                const int v = base + (lane >> 3);
-                if (mh.fk == 3) flat_search8<3, true>(pos, rowptr, he, v, v < it.v1, gs, mh.depth, sm, maxk, lane);
-                else flat_search8<4, true>(pos, rowptr, he, v, v < it.v1, gs, mh.depth, sm, maxk, lane);
+        if (SEARCH == PACKED || (SEARCH == MIXED && mh.packed)) {
+            if constexpr (SEARCH != GENERAL) {
+                float* sm = wco + (size_t)(lane >> 3) * f8_group_floats(maxk);
+                for (int base = it.v0; base < it.v1; base += 4) {
+                    const int v = base + (lane >> 3);
+                    if (mh.fk == 3) flat_search8<3, true>(pos, rowptr, he, v, v < it.v1, gs, mh.depth, sm, maxk, lane);
+                    else flat_search8<4, true>(pos, rowptr, he, v, v < it.v1, gs, mh.depth, sm, maxk, lane);
+                }
             }
-        } else if constexpr (!PACKED) {
+        } else if constexpr (SEARCH != PACKED) {
             const int L = mh.lanes, groups = 32 / L, g = lane / L, gl = lane % L;
             const unsigned gmask = L == 32 ? FULL : (((1u << L) - 1u) << (g * L));
             float* co = wco + (size_t)g * maxk * BCO;
@@ -373,8 +377,8 @@ void prepare_flat_kernels() {
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat8<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)flat8_smem(F8_MAX_RING)));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    VSDMO_CUDA(cudaFuncSetAttribute(k_batch_iter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bmx));
-    VSDMO_CUDA(cudaFuncSetAttribute(k_batch_iter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bmx));
+    for (auto k : {k_batch_iter<PACKED>, k_batch_iter<GENERAL>, k_batch_iter<MIXED>})
+        VSDMO_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bmx));
     done = true;
 }
 
@@ -522,10 +526,11 @@ void Batch::choose_packed(const std::vector<int>& sel) {
         maxc = std::max(maxc, hm[i].n_colors);
     }
     class_avg = free_v / maxc;
-    all_packed = true;
+    all_packed = none_packed = true;
     for (int i : ms) {
         hm[i].packed = cfg[i].nq == 8 && maxk <= F8_MAX_RING;
         all_packed = all_packed && hm[i].packed;
+        none_packed = none_packed && !hm[i].packed;
     }
 }
 
@@ -605,7 +610,7 @@ void Batch::ensure_launch_setup() {
     int dev = 0, sms = 148, per = 1;
     VSDMO_CUDA(cudaGetDevice(&dev));
     VSDMO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    VSDMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_iter<false>, BATCH_WARPS * 32, batch_smem(maxk)));
+    VSDMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_iter<MIXED>, BATCH_WARPS * 32, batch_smem(maxk)));
     blocks = sms * std::max(per, 1);
 }
 
@@ -620,7 +625,7 @@ void Batch::quality(BatchStats* out, int* d_it, int init, int advance, cudaStrea
 void Batch::launch_iteration(const BatchItem* d_it, int n, bool with_stats, cudaStream_t s) {
     VSDMO_CUDA(cudaMemsetAsync(done.p, 0, sizeof(int) * done.n, s));
     VSDMO_CUDA(cudaMemsetAsync(head.p, 0, sizeof(int), s));
-    const auto kernel = all_packed ? k_batch_iter<true> : k_batch_iter<false>;
+    const auto kernel = all_packed ? k_batch_iter<PACKED> : none_packed ? k_batch_iter<GENERAL> : k_batch_iter<MIXED>;
     kernel<<<blocks, BATCH_WARPS * 32, batch_smem(maxk), s>>>(pos.p, rowptr.p, he.p, d_it, n, d_meshes.p, csize.p, done.p,
                                                               head.p, maxk, grid_scale, err.p);
     VSDMO_CHECK_LAUNCH();

@@ -77,7 +77,7 @@ struct Batch {
     DBuf<int> qfirst;            // [meshes + 1] first chunk of each mesh
     DBuf<BatchStats> qpart;      // per-chunk partials
     int n_qchunks = 0;
-    bool all_packed = false;
+    bool all_packed = false, none_packed = false;
     int n_items = 0;
     bool items_dirty = true;
     int blocks = 0;
