@@ -18,10 +18,11 @@
 //     and the halfhex CSR (mesh/MeshHexGPU.cu:116-139, mesh/MeshGPUCommon.cu:1334-1368);
 //   * boundary / feature flags (dihedral > 20 deg, mesh/MeshGPUCommon.cu:466-495) and face /
 //     vertex normals (:363-434).
-// Sorting uses the stable LSD radix sort of prim.cu. Colouring runs the reference's JPL round
+// Elements keep the input's numbering until the end; one table of the elements around each vertex
+// serves the boundary faces, the colouring and the halfface rows. Colouring follows the reference's JPL round
 // rule (mesh/VertexColoring.cu:76-105): by default with seeded hash priorities, each vertex
 // taking the smallest colour none of its higher-priority neighbours has (the greedy colouring in
-// priority order, computed round by round); with VSDMO_COLOR_ROUNDS in the seed the colour is the
+// priority order, each vertex as soon as those neighbours are coloured); with VSDMO_COLOR_ROUNDS in the seed the colour is the
 // round (the reference's rule) with the hashed priorities of the seed's other bits; with
 // VSDMO_COLOR_REFERENCE the colour is the round and the priorities are the reference's own n - i
 // (VertexColoring.cu:107-125).

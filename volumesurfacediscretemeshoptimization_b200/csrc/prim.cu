@@ -1,8 +1,8 @@
 // prim.cu -- device-wide primitives used by the connectivity build: exclusive scan, stable
-// LSD radix sort of (key, value) pairs, stable compaction and CSR offsets. These replace the
+// LSD radix sort of (key, value) pairs, stable compaction, rows by key and CSR offsets. These replace the
 // thrust::sort_by_key / remove_if / inclusive_scan calls of the reference's mesh build
 // (e.g. mesh/MeshTriGPU.cu:142,162-170, mesh/MeshTetGPU.cu:125) and k_find_first_n
-// (mesh/SortUtil.cu:3-35). The build runs once per mesh; these kernels are HBM-bound.
+// (mesh/SortUtil.cu:3-35). The build runs once per mesh and is bound by launches and latency.
 #include "vsdmo_internal.cuh"
 #include <mutex>
 
