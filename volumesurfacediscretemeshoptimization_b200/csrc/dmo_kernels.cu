@@ -728,11 +728,9 @@ k_dmo_tri2d(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4
             bl = __ffs(__ballot_sync(FULL, val == redux_max(val))) - 1;
             bv = __shfl_sync(FULL, val, bl);
         }
-        if (qLast < bv) {
-            dx = __shfl_sync(FULL, selx, bl);
-            dy = __shfl_sync(FULL, y, bl);
-            qLast = bv;
-        }
+        // outside of the branch: with NaN keys the lanes need not agree on bv, and a shuffle waits for all of them
+        const float wx = __shfl_sync(FULL, selx, bl), wy = __shfl_sync(FULL, y, bl);
+        if (qLast < bv) { dx = wx; dy = wy; qLast = bv; }
         lastMax = bv;
         ds = ds * (2.0f / 7.0f);
     }
