@@ -1,6 +1,8 @@
 """Searches on rings where the ring fold of keys is not an ordinary minimum: coincident ring points (0 / 0 at
 a candidate that falls on them), points that nearly coincide, NaN positions. Bit for bit against the oracle
 (the same operations in the same order on both sides, so no tolerance)."""
+import os
+
 import numpy as np
 import pytest
 
@@ -42,3 +44,59 @@ def test_nan_key_on_one_lane(oracle_mod, vsdmo, use_graph):
     want = om.dmo_flat_f32(x, 0, 1, nq=8, depth=3)
     assert not np.array_equal(want[0], x[0])   # it moves
     assert np.array_equal(gm.positions().view(np.uint32), want.view(np.uint32))
+
+
+def _on_lattice(xyz, q):
+    """Rounded to a lattice coarser than the mesh: many coincident points and candidates that fall on them."""
+    return (np.round(xyz / q) * q).astype(np.float32)
+
+
+def _near(xyz, el, seed, eps):
+    """Two corners of some elements within eps of a third."""
+    g = np.random.default_rng(seed)
+    x = xyz.astype(np.float64)
+    for e in el[g.random(len(el)) < 0.02]:
+        x[e[1:3], :2] = x[e[0], :2] + eps * g.normal(size=(2, 2))
+    return x.astype(np.float32)
+
+
+def _with_nan(xyz, seed):
+    x = xyz.copy()
+    g = np.random.default_rng(seed)
+    x[g.random(len(x)) < 0.01, g.integers(0, 2)] = np.nan
+    return x
+
+
+CASES = {"lattice": lambda x, el: _on_lattice(x, 1 / 80), "lattice8": lambda x, el: _on_lattice(x, 1 / 128),
+         "near": lambda x, el: _near(x, el, 5, 1e-6), "nan": lambda x, el: _with_nan(x, 7)}
+
+
+@pytest.mark.parametrize("depth", [1, 3])
+@pytest.mark.parametrize("case", CASES)
+def test_packed_flat_against_general_search(vsdmo, case, depth):
+    """Four vertices per warp, in a batch and in a single mesh of large classes, against the search of a warp per
+    vertex (which a mesh with a larger ring brings to the whole batch), bit for bit: NaN keys leave the winner to
+    the order of its lanes, which the oracle does not have."""
+    from volumesurfacediscretemeshoptimization_b200 import meshgen as G
+    meshes = [(TRI, *G.tri_grid(130, 1)), (QUAD, *G.quad_grid(100, 2)), (TRI, *G.tri_grid(20, 3))]
+    start = [CASES[case](x, el) for _, x, el in meshes]
+    large = (TRI, *_fan(17))
+    got = []
+    for ms, xs in ((meshes, start), (meshes + [large], start + [large[1]])):
+        b = vsdmo.BatchDMO(ms)
+        assert (b.info()["max_halfedges"] > 16) == (len(ms) > 3)
+        b.set_config(8, depth, 32)
+        b.set_positions(np.concatenate(xs))
+        b.restart()
+        b.iterate(2)
+        got.append(b)
+    for i, (_, xyz, el) in enumerate(meshes):
+        want = got[1].mesh_positions(i)
+        assert not np.array_equal(want, start[i], equal_nan=True)
+        assert np.array_equal(got[0].mesh_positions(i).view(np.uint32), want.view(np.uint32)), i
+    gm = vsdmo.DMOMeshTri(*meshes[0][1:])
+    opt = vsdmo.DMOTriFlatClass(gm, n_iter=2, depth=depth, check_monotone=False)
+    gm.set_positions(start[0], original_order=True)
+    opt.restart()
+    opt.iterate(2)
+    assert np.array_equal(gm.positions(original_order=True).view(np.uint32), got[1].mesh_positions(0).view(np.uint32))

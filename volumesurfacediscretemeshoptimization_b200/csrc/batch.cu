@@ -154,7 +154,7 @@ k_dmo_flat(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4*
 // the same for four vertices per warp (8 x 8 candidates, rings of up to F8_MAX_RING)
 constexpr int F8_WARPS = 4;
 template <int FK>
-__global__ void __launch_bounds__(F8_WARPS * 32)
+__global__ void __launch_bounds__(F8_WARPS * 32, 8)
 k_dmo_flat8(float4* pos_, const int* __restrict__ rowptr, const int4* __restrict__ he, int v0, int v1,
             float gs, int depth, int maxk) {
     extern __shared__ float4 f8sm[];
@@ -163,7 +163,7 @@ k_dmo_flat8(float4* pos_, const int* __restrict__ rowptr, const int4* __restrict
     const int base = v0 + (blockIdx.x * F8_WARPS + w) * 4;
     float4* pos = chain_wait(pos_);
     if (base >= v1) return;
-    flat_search8<FK, false>(pos, rowptr, he, base + g, base + g < v1, gs, depth, sm, maxk, lane);
+    flat_search8<FK, false>(pos, rowptr, he, base + g, base + g < v1, gs, depth, sm, maxk, lane, 32);
 }
 
 // ---- the persistent batched iteration -----------------------------------------------------------
@@ -175,8 +175,8 @@ __host__ __device__ constexpr int batch_warp_floats(int maxk) {
 // SEARCH: every mesh is searched four vertices per warp (PACKED), none is (GENERAL), or some are (MIXED): only
 // what is needed is in the kernel (with both in one, half the stalls were instruction fetches; 4 x 4 grids on 256
 // meshes, 32 / 8 lanes: 8.28 / 2.18 ms per iteration with both, 7.48 / 1.94 with the general search alone).
-// Registers: four blocks per SM at 64 (48 bytes of spills) against three at 80 and two at 96: 2.28 / 2.33
-// / 2.80 ms per iteration of 256 meshes.
+// Registers: four blocks per SM at 64 against three at 80 and two at 96: 2.28 / 2.33 / 2.80 ms per iteration
+// of 256 meshes (measured without the rings searched apart, which take four blocks to 2.35).
 enum { PACKED, GENERAL, MIXED };
 template <int SEARCH>
 __global__ void __launch_bounds__(BATCH_WARPS * 32, 4)
@@ -224,8 +224,8 @@ k_batch_iter(float4* __restrict__ pos, const int* __restrict__ rowptr, const int
                 float* sm = wco + (size_t)(lane >> 3) * f8_group_floats(maxk);
                 for (int base = it.v0; base < it.v1; base += 4) {
                     const int v = base + (lane >> 3);
-                    if (mh.fk == 3) flat_search8<3, true>(pos, rowptr, he, v, v < it.v1, gs, mh.depth, sm, maxk, lane);
-                    else flat_search8<4, true>(pos, rowptr, he, v, v < it.v1, gs, mh.depth, sm, maxk, lane);
+                    if (mh.fk == 3) flat_search8<3, true>(pos, rowptr, he, v, v < it.v1, gs, mh.depth, sm, maxk, lane, mh.lanes);
+                    else flat_search8<4, true>(pos, rowptr, he, v, v < it.v1, gs, mh.depth, sm, maxk, lane, mh.lanes);
                 }
             }
         } else if constexpr (SEARCH != PACKED) {

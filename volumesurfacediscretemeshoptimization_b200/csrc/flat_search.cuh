@@ -18,8 +18,9 @@
 //
 // Bound: issue (66 % of the slots on 256 mixed meshes). The search with a warp per vertex spends most of
 // its slots on the idle lanes of a six-element ring and on reductions per vertex: 8.35 ms per
-// iteration of 256 meshes (3.2 M vertices), this one 2.28 ms. Loops over the ring are not unrolled:
-// unrolled by four they overflowed the instruction cache (3.46 ms, half the stalls instruction fetches).
+// iteration of 256 meshes (3.2 M vertices), this one 2.28 ms, and 2.35 ms with the rings searched apart
+// (their code costs the kernel registers). Loops over the ring are not unrolled: unrolled by four they
+// overflowed the instruction cache (3.46 ms, half the stalls instruction fetches).
 #pragma once
 #include "f32x2.cuh"
 #include "flat_key.cuh"
@@ -106,9 +107,15 @@ struct F8 {
 
 // One vertex per group of eight lanes (on: the group has one). sm: the group's f8_group_floats(maxk).
 // All lanes of the warp call this together.
+//
+// Keys are a minimum only while every edge sum L is positive: at a candidate on (or, with the rounding of
+// L, beside) two coincident ring points the fold meets 0 / 0 or a negative L and its result depends on
+// the order of the elements, and so it does with NaN positions. Rings in which L is not bounded well
+// above its rounding (2^-15 of the magnitudes that enter it, on the whole search box) are searched apart, by
+// the steps of the general search of L lanes on the coefficients at hand.
 template <int FK, bool COHERENT>
 __device__ void flat_search8(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ he, int v,
-                             bool on, float gs, int depth, float* __restrict__ sm, int maxk, int lane) {
+                             bool on, float gs, int depth, float* __restrict__ sm, int maxk, int lane, int L) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int CS = F8<FK>::CS;
     const int gl = lane & 7, g0 = lane & 24;
@@ -154,6 +161,7 @@ __device__ void flat_search8(float4* __restrict__ pos, const int* __restrict__ r
     (void)frexpf(mm, &ex);
     const float ps = bexp2(-ex);
     const float sx = bscale(mdx, ps, -ex), sy = bscale(mdy, ps, -ex);
+    bool odd = false;
     // the levels' half-extents sum to at most 1.4 gs
     const float Xm = (1.5f * gs) * sx, Ym = (1.5f * gs) * sy;
 #pragma unroll 1
@@ -176,10 +184,57 @@ __device__ void flat_search8(float4* __restrict__ pos, const int* __restrict__ r
         }
         const float w = __fdividef(1.f, l2);
         const float ml = fmaf(fabsf(l0), Xm, fmaf(fabsf(l1), Ym, fmaf(2.f * Xm, Xm, fmaf(2.f * Ym, Ym, l2))));
+        // L is smallest where its gradient vanishes; where that is too small, on the part of the box nearest to the corners
+        const float least = fmaf(-0.125f, fmaf(l0, l0, l1 * l1), l2), limit = 0x1p-15f * fmaxf(ml, 0x1p-10f);
+        if (!(least > limit)) {
+            const float ax = fmaxf(fabsf(bscale(a.x, ps, -ex)) - Xm, 0.f), ay = fmaxf(fabsf(bscale(a.y, ps, -ex)) - Ym, 0.f);
+            const float nx = fmaxf(fabsf(bscale(n.x, ps, -ex)) - Xm, 0.f), ny = fmaxf(fabsf(bscale(n.y, ps, -ex)) - Ym, 0.f);
+            if (least != least || !((ax * ax + ay * ay) + (nx * nx + ny * ny) > limit)) odd = true;
+        }
         fc[2 * t] = make_float4(w * a0, w * a1, w * a2, w * l0);
         fc[2 * t + 1] = make_float4(w * l1, w, (0x1p-18f * w) * ma, (0x1p-18f * w) * ml);
     }
     __syncwarp();
+    for (unsigned apart = __ballot_sync(FULL, odd); apart;) {
+        const int first = (__ffs((int)apart) - 1) & 24;
+        apart &= ~(0xffu << first);
+        const float* c = co + ((first - g0) >> 3) * f8_group_floats(maxk);
+        const int n = __shfl_sync(FULL, k, first);
+        const float fx = __shfl_sync(FULL, sx, first), fy = __shfl_sync(FULL, sy, first);
+        const float q0 = F8<FK>::key_again(c, n, 0.f, 0.f);
+        float mx = 0.f, my = 0.f, ql = q0, top = -FLT_MAX, h = gs;
+#pragma unroll 1
+        for (int level = 0; level < depth; ++level) {
+            float bv = -FLT_MAX, bx = 0.f, by = 0.f;
+            int bt = 1 << 30;
+#pragma unroll 1
+            for (int t = lane; t < 32 && lane < L; t += L) {
+                const float x1 = fmaf(boffset(t >> 3, 8), h * fx, mx), x2 = fmaf(boffset((t >> 3) + 4, 8), h * fx, mx);
+                const float y = fmaf(boffset(t & 7, 8), h * fy, my);
+                const float q1 = F8<FK>::key_again(c, n, x1, y), q2 = F8<FK>::key_again(c, n, x2, y);
+                const float val = q2 > q1 ? q2 : q1;
+                if (bt == (1 << 30) || val > bv) { bv = val; bt = t; bx = q1 > q2 ? x1 : x2; by = y; }
+            }
+#pragma unroll 1
+            for (int o = L >> 1; o; o >>= 1) {
+                const float ov = __shfl_xor_sync(FULL, bv, o), ox = __shfl_xor_sync(FULL, bx, o), oy = __shfl_xor_sync(FULL, by, o);
+                const int ot = __shfl_xor_sync(FULL, bt, o);
+                if (ov > bv || (ov == bv && ot < bt)) { bv = ov; bt = ot; bx = ox; by = oy; }
+            }
+            if (ql < bv) { mx = bx; my = by; ql = bv; }
+            top = bv;
+            h = h * (2.0f / 7.0f);
+        }
+        // NaN keys may leave the lanes with different winners: the first one's counts
+        mx = __shfl_sync(FULL, mx, 0);
+        my = __shfl_sync(FULL, my, 0);
+        const int better = __shfl_sync(FULL, q0 < top ? 1 : 0, 0);
+        if (lane == first && better) {
+            const float pu = bexp2(ex);
+            pos[v] = make_float4(c0.x + bscale(mx, pu, ex), c0.y + bscale(my, pu, ex), c0.z, c0.w);
+        }
+        if (g0 == first) k = -1;
+    }
     const float off = boffset(gl, 8);   // offset i of an axis is lane i's of the group
     float dx = 0.f, dy = 0.f, ds = gs;
     float qOld = 0.f, qLast = 0.f;
@@ -252,8 +307,9 @@ __device__ void flat_search8(float4* __restrict__ pos, const int* __restrict__ r
             for (int t = gl; t < k; t += 8) {
                 const float4 f = fc[2 * t], e = fc[2 * t + 1];
                 const float w2 = 2.f * e.y;
-                const float L = fmaf(f.w, dx, fmaf(e.x, dy, fmaf(w2 * dx, dx, fmaf(w2 * dy, dy, 1.f))));
-                const float r = L - fmaf(fabsf(fmaf(2.f * w2, dx, f.w)), Sx, fabsf(fmaf(2.f * w2, dy, e.x)) * Sy);
+                const float l = fmaf(f.w, dx, fmaf(e.x, dy, fmaf(w2 * dx, dx, fmaf(w2 * dy, dy, 1.f))));
+                // (less the rounding of l and its gradient: e.w is 2^-18 of their magnitudes)
+                const float r = l - fmaf(fabsf(fmaf(2.f * w2, dx, f.w)), Sx, fmaf(fabsf(fmaf(2.f * w2, dy, e.x)), Sy, e.w));
                 rho = fminf(rho, r > 0.f ? r : 0.f);
             }
             // the candidate of the largest bound: the index replaces the low three bits of the bound
@@ -290,7 +346,7 @@ __device__ void flat_search8(float4* __restrict__ pos, const int* __restrict__ r
             for (int i = 0; i < 8; ++i)
                 if (!(s[i] < (again ? 0.f : cut))) alive |= 1u << i;
             if (found && gl == pj) alive &= ~(1u << pi);
-            if (k == 0 || all < 0.f) alive = 0;
+            if (k <= 0 || all < 0.f) alive = 0;
             if (__any_sync(FULL, alive)) {
                 do {
                     const int i = alive ? __ffs((int)alive) - 1 : 0;
