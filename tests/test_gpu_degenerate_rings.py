@@ -100,3 +100,26 @@ def test_packed_flat_against_general_search(vsdmo, case, depth):
     opt.restart()
     opt.iterate(2)
     assert np.array_equal(gm.positions(original_order=True).view(np.uint32), got[1].mesh_positions(0).view(np.uint32))
+
+
+@pytest.mark.parametrize("ring", range(3))
+def test_tet_rings_of_collapsed_tets_bitwise(oracle_mod, vsdmo, ring):
+    """Recorded rings with tets a thousandth of their size and smaller: the sum of squared edges is lost in
+    its rounding beside such a tet, or products of the fold are no normal numbers."""
+    data = np.load(os.path.join(os.path.dirname(__file__), "golden", "odd_tet_rings.npz"))
+    start, el, gs = data[f"xyz{ring}"], data[f"tets{ring}"], float(data[f"grid_scale{ring}"])
+    xyz = np.random.default_rng(0).normal(size=start.shape)   # the mesh is built on a round ring
+    xyz /= np.linalg.norm(xyz, axis=1)[:, None]
+    xyz[0] = 0
+    om = oracle_mod.OracleMesh(TET, xyz.astype(np.float32), el)
+    gm = vsdmo.DMOMeshTet(xyz, el)
+    x = om.xyz.copy()
+    x[om.array(oracle_mod.A_NEW_OF_OLD)] = start
+    opt = vsdmo.DMOTetClass(gm, gridScale=gs, n_iter=1, check_monotone=False)
+    gm.set_positions(x)
+    opt.restart()
+    opt.iterate(1)
+    v0, v1 = om.color_ranges()[0]
+    want = om.dmo_color_f32(x, v0, v1, grid_scale=gs)
+    assert not np.array_equal(want, x)
+    assert np.array_equal(gm.positions().view(np.uint32), want.view(np.uint32))

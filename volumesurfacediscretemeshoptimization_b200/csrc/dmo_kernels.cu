@@ -95,16 +95,19 @@ __device__ __forceinline__ float tet_key_min(const float4* __restrict__ co, int 
 // Setup of one tet vertex shared by the plain and the learned search: per-axis extent of the
 // ring (DMOTetImplCub.h:54-64), the exact power-of-two scale 2^ex and the element coefficients
 // in shared memory. Returns the number of tets, 0 when the vertex is left alone (an empty,
-// oversized or degenerate ring). scratch: 512 bytes of shared memory per warp.
+// oversized or degenerate ring). scratch: 512 bytes of shared memory per warp. odd: some tet's L is not
+// bounded well above zero on the search box (tet_least), so ring keys depend on the order of the tets (ODD).
 //
 // Rings of up to 32 tets and 32 vertices come from the ring table: one coalesced row of ring
 // vertices and one of 16-bit corner triples per vertex, so every ring position is loaded once
 // (14 instead of 72 gathers for a Kuhn vertex) and two dependent loads reach the positions
 // instead of three (row pointer, halffaces, positions). Larger rings read their halffaces twice.
+template <bool ODD>
 __device__ __forceinline__ int tet_setup(const float4* __restrict__ pos, const int* __restrict__ rowptr,
                                          const int4* __restrict__ hf, unsigned corner, int nb, int v, int maxk,
-                                         float4 c0, int lane, float4* co, float4* scratch, float& sx, float& sy,
-                                         float& sz, int& ex) {
+                                         float4 c0, int lane, float grid_scale, float4* co, float4* scratch, float& sx,
+                                         float& sy, float& sz, int& ex, bool& odd) {
+    odd = false;
     const float4 q = pos[nb];
     const unsigned has = __ballot_sync(FULL, corner != TetRingTable::NONE);
     if (__any_sync(FULL, corner == TetRingTable::LARGE)) {
@@ -126,11 +129,14 @@ __device__ __forceinline__ int tet_setup(const float4* __restrict__ pos, const i
         for (int t = lane; t < k; t += 32) {
             const int4 h = hf[b + t];
             const float4 pa = pos[h.x], pb = pos[h.y], pc = pos[h.z];
-            tet_coeffs(scale2(pa.x - c0.x, p, -ex), scale2(pa.y - c0.y, p, -ex), scale2(pa.z - c0.z, p, -ex),
-                       scale2(pb.x - c0.x, p, -ex), scale2(pb.y - c0.y, p, -ex), scale2(pb.z - c0.z, p, -ex),
-                       scale2(pc.x - c0.x, p, -ex), scale2(pc.y - c0.y, p, -ex), scale2(pc.z - c0.z, p, -ex),
-                       co[2 * t], co[2 * t + 1]);
+            const float3 a = make_float3(scale2(pa.x - c0.x, p, -ex), scale2(pa.y - c0.y, p, -ex), scale2(pa.z - c0.z, p, -ex));
+            const float3 b3 = make_float3(scale2(pb.x - c0.x, p, -ex), scale2(pb.y - c0.y, p, -ex), scale2(pb.z - c0.z, p, -ex));
+            const float3 c = make_float3(scale2(pc.x - c0.x, p, -ex), scale2(pc.y - c0.y, p, -ex), scale2(pc.z - c0.z, p, -ex));
+            tet_coeffs(a.x, a.y, a.z, b3.x, b3.y, b3.z, c.x, c.y, c.z, co[2 * t], co[2 * t + 1]);
+            if (ODD && !(tet_least(co[2 * t + 1]) > tet_odd_limit(grid_scale)))
+                odd |= tet_odd(a, b3, c, grid_scale, scale2(mdx, p, -ex), scale2(mdy, p, -ex), scale2(mdz, p, -ex));
         }
+        if (ODD) odd = __any_sync(FULL, odd);
         __syncwarp();
         sx = scale2(mdx, p, -ex); sy = scale2(mdy, p, -ex); sz = scale2(mdz, p, -ex);
         return k;
@@ -146,10 +152,20 @@ __device__ __forceinline__ int tet_setup(const float4* __restrict__ pos, const i
     __syncwarp();
     if (lane < k) {
         const float4 a = scratch[corner & 31u], b = scratch[(corner >> 5) & 31u], c = scratch[corner >> 10];
-        tet_coeffs(a.x, a.y, a.z, b.x, b.y, b.z, c.x, c.y, c.z, co[2 * lane], co[2 * lane + 1]);
+        float4 K1;
+        tet_coeffs(a.x, a.y, a.z, b.x, b.y, b.z, c.x, c.y, c.z, co[2 * lane], K1);
+        co[2 * lane + 1] = K1;
+        odd = ODD && !(tet_least(K1) > tet_odd_limit(grid_scale));
+    }
+    sx = scale2(mdx, p, -ex); sy = scale2(mdy, p, -ex); sz = scale2(mdz, p, -ex);
+    if (ODD && __any_sync(FULL, odd)) {
+        if (odd) {
+            const float4 a = scratch[corner & 31u], b = scratch[(corner >> 5) & 31u], c = scratch[corner >> 10];
+            odd = tet_odd(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z), make_float3(c.x, c.y, c.z), grid_scale, sx, sy, sz);
+        }
+        odd = __any_sync(FULL, odd);
     }
     __syncwarp();
-    sx = scale2(mdx, p, -ex); sy = scale2(mdy, p, -ex); sz = scale2(mdz, p, -ex);
     return k;
 }
 
@@ -193,11 +209,12 @@ k_dmo_tet(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* 
     const float4 c0 = p[v];
     float sx, sy, sz;
     int ex;
-    const int k = tet_setup(p, rowptr, hf, corner, nb, v, maxk, c0, lane, co, reinterpret_cast<float4*>(scratch), sx, sy, sz, ex);
+    bool odd;
+    const int k = tet_setup<true>(p, rowptr, hf, corner, nb, v, maxk, c0, lane, grid_scale, co, reinterpret_cast<float4*>(scratch), sx, sy,
+                            sz, ex, odd);
     if (k == 0) return;
-    const float qLast = tet_group_key(co, k, 0.f, 0.f, 0.f, 32, lane);
     float dx, dy, dz;
-    const bool moved = tet_plain_search(co, scratch, k, sx, sy, sz, grid_scale, depth, lane, qLast, dx, dy, dz);
+    const bool moved = tet_search(co, scratch, k, odd, sx, sy, sz, grid_scale, depth, lane, dx, dy, dz);
     if (moved && lane == 0) pos[v] = tet_unscale(c0, dx, dy, dz, ex);
     if (dirty) {
         if (moved) tet_mark_ring(hf, rowptr[v], k, lane, dirty);
@@ -225,12 +242,12 @@ k_dmo_tet_list(float4* __restrict__ pos, const int* __restrict__ rowptr, const i
         float sx, sy, sz;
         int ex;
         const size_t row = (size_t)(v - ring.base) * 32 + lane;
-        const int k = tet_setup(pos, rowptr, hf, ring.corner[row], ring.nb[row], v, maxk, c0, lane, co, reinterpret_cast<float4*>(scratch), sx, sy,
-                                sz, ex);
+        bool odd;
+        const int k = tet_setup<true>(pos, rowptr, hf, ring.corner[row], ring.nb[row], v, maxk, c0, lane, grid_scale, co,
+                                reinterpret_cast<float4*>(scratch), sx, sy, sz, ex, odd);
         if (k == 0) continue;
-        const float qLast = tet_group_key(co, k, 0.f, 0.f, 0.f, 32, lane);
         float dx, dy, dz;
-        const bool moved = tet_plain_search(co, scratch, k, sx, sy, sz, grid_scale, depth, lane, qLast, dx, dy, dz);
+        const bool moved = tet_search(co, scratch, k, odd, sx, sy, sz, grid_scale, depth, lane, dx, dy, dz);
         if (moved && lane == 0) {
             pos[v] = tet_unscale(c0, dx, dy, dz, ex);
             atomicAdd(moved_count, 1ull);
@@ -462,7 +479,8 @@ k_dmo_tet_learned(float4* __restrict__ pos, const int* __restrict__ rowptr, cons
     int ex;
     float4* scratch = smem + (size_t)TET_WARPS * maxk * 2 + w * 32;
     const size_t row = (size_t)(v - ring.base) * 32 + lane;
-    const int k = tet_setup(pos, rowptr, hf, ring.corner[row], ring.nb[row], v, maxk, c0, lane, co, scratch, sx, sy, sz, ex);
+    bool odd;   // unused: keys here are a minimum over the tets
+    const int k = tet_setup<false>(pos, rowptr, hf, ring.corner[row], ring.nb[row], v, maxk, c0, lane, grid_scale, co, scratch, sx, sy, sz, ex, odd);
     if (k == 0) return;
     const float q0 = tet_key_min(co, k, 0.f, 0.f, 0.f, lane);
     // proposal in scaled local coordinates (the features were divided by mm = max(sx, sy, sz) 2^ex)

@@ -143,9 +143,9 @@ static __device__ __forceinline__ bool quad_filter(const Ring& ring, const QuadL
             const float w = __fdividef(1.f, r3);
             const float b = 1.5f * (lv.sq * r), a = 0.5f * (lv.sq * r3);
             // magnitudes of all that enters g, for the rounding allowance
+            const float magL = fmaf(fabsf(B.x), Xm, fmaf(fabsf(B.y), Ym, fmaf(fabsf(B.z), Zm, fmaf(alpha, R2, fabsf(B.w)))));
             const float mag = fmaf(fabsf(A.x), Xm, fmaf(fabsf(A.y), Ym, fmaf(fabsf(A.z), Zm, fabsf(A.w)))) +
-                              fmaf(b, fmaf(fabsf(B.x), Xm, fmaf(fabsf(B.y), Ym, fmaf(fabsf(B.z), Zm, fmaf(alpha, R2, fabsf(B.w))))),
-                                   a + fabsf(lv.low));
+                              fmaf(b, magL, a + fabsf(lv.low));
             const float slack = 0x1p-18f * mag;
             const float g = w * (((det - lv.low) + fmaf(-b, L, a)) + slack);
             const float a2 = 2.f * alpha;   // gradient of L
@@ -214,7 +214,7 @@ static __device__ __forceinline__ bool quad_filter(const Ring& ring, const QuadL
                 for (int i = 0; i < 4; ++i) upk2(v[i], e[i], e[4 + i]);
                 *reinterpret_cast<float4*>(u + 32) = make_float4(e[0], e[1], e[2], e[3]);
                 *reinterpret_cast<float4*>(u + 36) = make_float4(e[4], e[5], e[6], e[7]);
-                const float T = w * fmaf(1.5f * r, Lmin, -0.5f * r3);
+                const float T = w * fmaf(1.5f * r, fmaf(-0x1p-20f, magL, Lmin), -0.5f * r3);   // less the rounding of Lmin
                 rho = fminf(rho, T > 0.f ? T : 0.f);
             }
             first = base + m1;

@@ -15,12 +15,37 @@
 // Bound: issue (69 % of the slots, 2,370 to 4,975 warp instructions per vertex from the converged
 // cube to the jittered start). On the 48^3 cube (20 iterations, 104 k vertices) the filter by
 // fractions over six tets took 0.864 ms per iteration; this one took 0.472 ms over all tets, judging
-// every survivor, and takes 0.404 ms over the critical tets with the pruning.
+// every survivor, and took 0.404 ms over the critical tets with the pruning; it takes 0.416 ms with the check for rings that the
+// filter does not hold for and the search that they take instead.
 #pragma once
 #include "tet_key.cuh"
 #include "quad_filter.cuh"
 
 namespace vsdmo {
+
+// Ring keys are a minimum over the tets, in whatever order they are folded, only while every L is positive
+// and its cube and the products of the fold are normal numbers: at a candidate beside a tet's collapsed base
+// the rounding of L decides, and NaN positions make the fold depend on the order. Rings with a tet whose L is
+// not bounded above the limit (in units of the ring's extent; edges of a percent) on the search box are searched
+// without the filter.
+static __device__ __forceinline__ float tet_odd_limit(float grid_scale) { return 0x1p-12f * fmaxf(1.f, grid_scale * grid_scale); }
+// L of a tet where its gradient vanishes: below L everywhere; NaN when a corner is
+static __device__ __forceinline__ float tet_least(float4 K1) {
+    return fmaf(-1.f / 12.f, fmaf(K1.x, K1.x, fmaf(K1.y, K1.y, K1.z * K1.z)), K1.w);
+}
+// the same bound from the box's distances to the corners a, b, c (the levels' half-extents sum to at most 1.4 grid_scale)
+static __device__ __noinline__ bool tet_odd(float3 a, float3 b, float3 c, float grid_scale, float sx, float sy, float sz) {
+    const float X = (1.5f * grid_scale) * sx, Y = (1.5f * grid_scale) * sy, Z = (1.5f * grid_scale) * sz;
+    const float3 p[3] = { a, b, c };
+    float d = 0.f, sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const float x = fmaxf(fabsf(p[i].x) - X, 0.f), y = fmaxf(fabsf(p[i].y) - Y, 0.f), z = fmaxf(fabsf(p[i].z) - Z, 0.f);
+        d += (x * x + y * y) + z * z;
+        sum += (p[i].x + p[i].y) + p[i].z;
+    }
+    return sum != sum || !(d > tet_odd_limit(grid_scale));
+}
 
 // tet_key1 of the candidate (x, y, z) by the P lanes of an aligned group (P a power of two up to
 // 32, the same on all lanes; the candidate is the group's): each lane folds every P-th tet and the
@@ -122,6 +147,46 @@ static __device__ __forceinline__ bool tet_plain_search(const float4* __restrict
         }
     }
     return moved;
+}
+
+// The same search of a ring whose keys depend on the order of its tets (odd): every candidate by tet_key1. NaN keys never win.
+static __device__ __forceinline__ bool tet_full_search(const float4* __restrict__ co, int k, float sx, float sy, float sz,
+                                                       float grid_scale, int depth, int lane, float& dx, float& dy, float& dz) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const float off = grid_offset(lane & 7);
+    dx = 0.f; dy = 0.f; dz = 0.f;
+    bool moved = false;
+    float ds = grid_scale, qLast = tet_key1(co, k, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int level = 0; level < depth; ++level) {
+        const QuadLevel lv{dx, dy, dz, ds * sx, ds * sy, ds * sz, 0.f, 0.f, 0.f, false};
+        ds = ds * (2.0f / 7.0f);
+        float bk = -FLT_MAX;
+        int bi = 1 << 30;
+#pragma unroll 1
+        for (int i = lane; i < 512; i += 32) {
+            const float3 c = grid_candidate(i, off, lv);
+            const float key = tet_key1(co, k, c.x, c.y, c.z);
+            if (key > bk) { bk = key; bi = i; }
+        }
+        const float best = redux_max(bk);
+        bi = (int)__reduce_min_sync(FULL, bk == best ? (unsigned)bi : 1u << 30);
+        if (bi < 512 && qLast < best) {
+            const float3 c = grid_candidate(bi, off, lv);
+            dx = c.x; dy = c.y; dz = c.z;
+            qLast = best;
+            moved = true;
+        }
+    }
+    return moved;
+}
+
+static __device__ __forceinline__ bool tet_search(const float4* __restrict__ co, float* __restrict__ scratch, int k, bool odd,
+                                                  float sx, float sy, float sz, float grid_scale, int depth, int lane, float& dx,
+                                                  float& dy, float& dz) {
+    if (odd) return tet_full_search(co, k, sx, sy, sz, grid_scale, depth, lane, dx, dy, dz);
+    const float qLast = tet_group_key(co, k, 0.f, 0.f, 0.f, 32, lane);
+    return tet_plain_search(co, scratch, k, sx, sy, sz, grid_scale, depth, lane, qLast, dx, dy, dz);
 }
 
 }  // namespace vsdmo
