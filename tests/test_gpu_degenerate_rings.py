@@ -123,3 +123,32 @@ def test_tet_rings_of_collapsed_tets_bitwise(oracle_mod, vsdmo, ring):
     want = om.dmo_color_f32(x, v0, v1, grid_scale=gs)
     assert not np.array_equal(want, x)
     assert np.array_equal(gm.positions().view(np.uint32), want.view(np.uint32))
+
+
+def _hex_collapsed(xyz, el, seed):
+    """A thousand times larger, where the metric's thresholds are small beside the ring; corners of some
+    elements within 1e-5 of one another."""
+    g = np.random.default_rng(seed)
+    x = xyz.astype(np.float64) * 1000
+    for e in el[g.random(len(el)) < 0.1]:
+        x[e[1:4]] = x[e[0]] + 1e-2 * g.normal(size=(3, 3))
+    return x.astype(np.float32)
+
+
+@pytest.mark.parametrize("case", ["nan", "collapsed"])
+def test_hex_rings_bitwise(oracle_mod, vsdmo, case):
+    from volumesurfacediscretemeshoptimization_b200 import meshgen as G
+    xyz, el = G.hex_cube(8, 1)
+    start = _with_nan(xyz, 5) if case == "nan" else _hex_collapsed(xyz, el, 5)
+    om = oracle_mod.OracleMesh(HEX, xyz, el)
+    gm = vsdmo.DMOMeshHex(xyz, el)
+    x = om.xyz.copy()
+    x[om.array(oracle_mod.A_NEW_OF_OLD)] = start
+    opt = vsdmo.DMOHexClass(gm, n_iter=2, check_monotone=False)
+    gm.set_positions(x)
+    opt.restart()
+    opt.iterate(2)
+    for _ in range(2):
+        for v0, v1 in om.color_ranges():
+            x = om.dmo_color_f32(x, v0, v1)
+    assert np.array_equal(gm.positions(), x, equal_nan=True)

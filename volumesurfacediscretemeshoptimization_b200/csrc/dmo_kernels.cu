@@ -623,6 +623,9 @@ k_dmo_hex(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* 
     (void)frexpf(mm, &ex);
     const float p2 = exp2_exact(-ex);
     const float es = ldexpf(HEX_EPS, -3 * ex), ea = ldexpf(HEX_EPS, -2 * ex);
+    const float sx = scale2(mn0, p2, -ex), sy = scale2(mn1, p2, -ex), sz = scale2(mn2, p2, -ex);
+    const float X = (1.5f * grid_scale) * sx, Y = (1.5f * grid_scale) * sy, Z = (1.5f * grid_scale) * sz;
+    bool odd = false;
     __syncwarp();
     for (int h = lane; h < k; h += 32) {
         float r[7][3];
@@ -632,13 +635,21 @@ k_dmo_hex(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* 
             r[c][0] = scale2(d.x, p2, -ex); r[c][1] = scale2(d.y, p2, -ex); r[c][2] = scale2(d.z, p2, -ex);
         }
         hex_coeffs(r, es, ea, co + HEX_CO * h);
+        odd |= hex_odd(co + HEX_CO * h, X, Y, Z);
     }
     __syncwarp();
     const HexItems ring{co, k, es, ea, nullptr, 0};
     float* scratch = reinterpret_cast<float*>(corner);
     float dx, dy, dz;
-    const bool moved = hex_plain_search(ring, scratch, reinterpret_cast<unsigned short*>(scratch + TS_WARP_BYTES / 4), scale2(mn0, p2, -ex), scale2(mn1, p2, -ex),
-                                        scale2(mn2, p2, -ex), grid_scale, depth, lane, dx, dy, dz);
+    bool moved;
+    if (__any_sync(FULL, odd)) {
+        const float3 d = hex_full_search(co, k, es, ea, sx, sy, sz, grid_scale, depth);
+        dx = d.x; dy = d.y; dz = d.z;
+        moved = dx != 0.f || dy != 0.f || dz != 0.f;
+    } else {
+        moved = hex_plain_search(ring, scratch, reinterpret_cast<unsigned short*>(scratch + TS_WARP_BYTES / 4), sx, sy, sz, grid_scale, depth,
+                                 lane, dx, dy, dz);
+    }
     if (moved && lane == 0) pos[v] = tet_unscale(c0, dx, dy, dz, ex);
 }
 

@@ -144,6 +144,53 @@ struct HexItems {
     }
 };
 
+// Keys are a minimum over the items, in whatever order they are folded, only while every A is positive and the
+// products of the fold are normal numbers. The thresholds es and ea see to that where the ring's extent is
+// about 1, but they shrink with a growing extent, and NaN positions make the fold depend on the order. Whether
+// a halfhex (coefficients c, box half-extents X, Y, Z) has such an item: a constant part with a small A, or a
+// sub-tet whose A is bounded above 2^-12 neither where its gradient vanishes nor by its tangent at the origin.
+static __device__ __forceinline__ bool hex_odd(const float* __restrict__ c, float X, float Y, float Z) {
+    bool odd = !(c[1] > 0x1p-36f) || c[0] != c[0];
+#pragma unroll 1
+    for (int j = 0; j < 5; ++j) {
+        const float* q = c + 3 + 8 * j;
+        const float least = fmaf((j == 1 || j == 4) ? -1.f / 12.f : -0.25f, fmaf(q[4], q[4], fmaf(q[5], q[5], q[6] * q[6])), q[7]);
+        const float tangent = q[7] - fmaf(fabsf(q[4]), X, fmaf(fabsf(q[5]), Y, fabsf(q[6]) * Z));
+        if (!(fmaxf(least, tangent) > 0x1p-12f) || q[3] != q[3]) odd = true;
+    }
+    return odd;
+}
+
+// The search of a ring with such a halfhex: every candidate by hex_key1. NaN keys never win.
+static __device__ __noinline__ float3 hex_full_search(const float* __restrict__ co, int k, float es, float ea, float sx, float sy, float sz,
+                                                      float grid_scale, int depth) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const float off = grid_offset(lane & 7);
+    float dx = 0.f, dy = 0.f, dz = 0.f, ds = grid_scale, qLast = hex_key1(co, k, 0.f, 0.f, 0.f, es, ea);
+#pragma unroll 1
+    for (int level = 0; level < depth; ++level) {
+        const QuadLevel lv{dx, dy, dz, ds * sx, ds * sy, ds * sz, 0.f, 0.f, 0.f, false};
+        ds = ds * (2.0f / 7.0f);
+        float bk = -FLT_MAX;
+        int bi = 1 << 30;
+#pragma unroll 1
+        for (int i = lane; i < 512; i += 32) {
+            const float3 c = grid_candidate(i, off, lv);
+            const float key = hex_key1(co, k, c.x, c.y, c.z, es, ea);
+            if (key > bk) { bk = key; bi = i; }
+        }
+        const float best = redux_max(bk);
+        bi = (int)__reduce_min_sync(FULL, bk == best ? (unsigned)bi : 1u << 30);
+        if (bi < 512 && qLast < best) {
+            const float3 c = grid_candidate(bi, off, lv);
+            dx = c.x; dy = c.y; dz = c.z;
+            qLast = best;
+        }
+    }
+    return make_float3(dx, dy, dz);
+}
+
 // Search from the local origin; returns whether the vertex moved. scratch: TS_WARP_BYTES of the warp,
 // subset: 6 k places.
 static __device__ __forceinline__ bool hex_plain_search(HexItems ring, float* __restrict__ scratch,
