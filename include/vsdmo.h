@@ -369,6 +369,9 @@ VSDMO_API vsdmo_status vsdmo_debug_gemm_bf16(const float* A, const float* B, int
  * waits that let copies and MMAs in flight land after an expiry keep 1 s. Synchronises the
  * device; call it with none of the library's work in flight. */
 VSDMO_API vsdmo_status vsdmo_debug_set_wait_limit_ns(int64_t ns);
+/* The same for the waits on MMAs of the fused training step alone, whose operand loads keep their
+ * limit (vsdmo_debug_set_wait_limit_ns sets both). */
+VSDMO_API vsdmo_status vsdmo_debug_set_train_mma_wait_limit_ns(int64_t ns);
 
 /* Feature-vertex state of an optimiser with feature vertices (surfaces with features, flat
  * meshes with sliding boundaries), internal numbering: curves [nSurf x 12] (p0[3] a, e0[3] 0,

@@ -550,6 +550,11 @@ def debug_set_wait_limit_ns(ns: int) -> None:
     check(_capi.lib().vsdmo_debug_set_wait_limit_ns(int(ns)))
 
 
+def debug_set_train_mma_wait_limit_ns(ns: int) -> None:
+    """Test entry point: the same for the fused training step's waits on MMAs alone."""
+    check(_capi.lib().vsdmo_debug_set_train_mma_wait_limit_ns(int(ns)))
+
+
 class DMOHexClass(_DMOBase):
     """``DMO::DMOHexClass`` (``dmo/DMOHex.h``): interior hex DMO with ``shapeMetricHex``."""
 

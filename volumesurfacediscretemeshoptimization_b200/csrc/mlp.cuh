@@ -89,6 +89,8 @@ struct Model {
 void prepare(cudaStream_t s);
 void prepare_train();
 void set_train_wait_limit(unsigned long long ns);
+// limit of the training step's MMA waits alone (test-only lowering)
+void set_train_mma_wait_limit(unsigned long long ns);
 void debug_gemm(const float* hA, const float* hB, int M, int N, int K, float* hD, cudaStream_t s);
 // limit of the reported tensor-core waits on the current device (test-only lowering)
 void set_wait_limit(unsigned long long ns);

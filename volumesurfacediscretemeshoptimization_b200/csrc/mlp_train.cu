@@ -38,6 +38,8 @@ using tc::pk_off;
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
+// limit of the MMA waits, apart from the load waits' (tc::g_wait_limit_ns) so that a test can make them alone expire
+static __device__ unsigned long long g_mma_wait_limit_ns = tc::WAIT_NS;
 constexpr int TT = 256;   // threads: warp w takes rows 32 (w & 3) .. + 31, columns 64 (w >> 2) .. + 63
 // shared memory (bytes)
 constexpr uint32_t S_X = 0, S_H1 = S_X + 24576, S_H2 = S_H1 + 32768, S_H3 = S_H2 + 32768, S_DY = S_H3 + 32768;
@@ -191,7 +193,9 @@ __global__ void __launch_bounds__(TT, 1) k_train_tile(TileArgs p) {
     extern __shared__ __align__(1024) uint8_t sm[];
     __shared__ __align__(8) uint64_t bars[4];
     __shared__ uint32_t tmem_slot;
-    __shared__ int s_fail;
+    // two flags, each written on one side of a phase's first barrier and read on the other side of its next one: a
+    // warp that is late in reading one cannot meet the next phase's write
+    __shared__ int s_noload, s_nomma;
     __shared__ __align__(16) float s_bias[3 * HID + 4];
     if ((int)blockIdx.x == p.ctas) {
         // its state was last written by this block of the step before, two launches ago
@@ -210,7 +214,7 @@ __global__ void __launch_bounds__(TT, 1) k_train_tile(TileArgs p) {
     if (tid == 0) {
         for (int i = 0; i < 4; ++i) tc::mbar_init(tc::smem_u32(&bars[i]), 1);
         tc::mbar_init_fence();
-        s_fail = 0;
+        s_noload = s_nomma = 0;
     }
     if (warp == 0) tc::tmem_alloc(tc::smem_u32(&tmem_slot), 512);
     tc::tc_fence_before();
@@ -231,7 +235,7 @@ __global__ void __launch_bounds__(TT, 1) k_train_tile(TileArgs p) {
                     make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
         }
     };
-    const unsigned long long limit = tc::wait_limit();
+    const unsigned long long limit = tc::wait_limit(), mma_limit = *(volatile unsigned long long*)&g_mma_wait_limit_ns;
     int loads[3] = { 0, 0, 0 }, seen[3] = { 0, 0, 0 };   // thread 0: loads issued / waited for, per buffer
     uint32_t mphase = 0;
     bool pending = false;
@@ -290,7 +294,7 @@ __global__ void __launch_bounds__(TT, 1) k_train_tile(TileArgs p) {
                 if (buf >= 0 && ph != 4) {
                     ok = tc::mbar_wait_within(bar_w[buf], (uint32_t)(seen[buf] & 1), limit);
                     if (ok) ++seen[buf];
-                    else { atomicExch(p.err, tc::TC_TIMEOUT_LOAD); s_fail = 1; }
+                    else { atomicExch(p.err, tc::TC_TIMEOUT_LOAD); s_noload = 1; }
                 }
                 if (ok) {
                     tc::tc_fence_after();
@@ -317,10 +321,11 @@ __global__ void __launch_bounds__(TT, 1) k_train_tile(TileArgs p) {
                 }
             }
             __syncthreads();
-            if (s_fail) { stop = true; break; }   // nothing was issued
+            if (s_noload) { stop = true; break; }   // nothing was issued
             pending = true;
-            if (!tc::mbar_wait_within(bar_m, mphase, limit)) {
-                if (lane == 0) { atomicExch(p.err, tc::TC_TIMEOUT_MMA); s_fail = 1; }
+            // the epilogues are warp-wide: a warp takes part when the wait of all its lanes succeeded
+            if (!__all_sync(FULL, tc::mbar_wait_within(bar_m, mphase, mma_limit))) {
+                if (lane == 0) { atomicExch(p.err, tc::TC_TIMEOUT_MMA); s_nomma = 1; }
             } else {
                 pending = false;
                 mphase ^= 1u;
@@ -404,7 +409,7 @@ __global__ void __launch_bounds__(TT, 1) k_train_tile(TileArgs p) {
             }
             tc::tc_fence_before();
             __syncthreads();
-            if (s_fail) { stop = true; break; }
+            if (s_nomma) { stop = true; break; }
         }
     }
     launch_dependents();
@@ -554,7 +559,15 @@ void prepare_train() {
 }
 
 // (the limit is a variable of each translation unit that waits)
-void set_train_wait_limit(unsigned long long ns) { VSDMO_CUDA(cudaMemcpyToSymbol(tc::g_wait_limit_ns, &ns, sizeof(ns))); }
+void set_train_wait_limit(unsigned long long ns) {
+    VSDMO_CUDA(cudaMemcpyToSymbol(tc::g_wait_limit_ns, &ns, sizeof(ns)));
+    VSDMO_CUDA(cudaMemcpyToSymbol(g_mma_wait_limit_ns, &ns, sizeof(ns)));
+}
+void set_train_mma_wait_limit(unsigned long long ns) {
+    VSDMO_CUDA(cudaDeviceSynchronize());
+    VSDMO_CUDA(cudaMemcpyToSymbol(g_mma_wait_limit_ns, &ns, sizeof(ns)));
+    VSDMO_CUDA(cudaDeviceSynchronize());
+}
 
 int fused_tiles(int B) {
     const int tiles = B / 128, parts = wgrad_parts(B);
