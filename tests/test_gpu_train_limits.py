@@ -1,4 +1,5 @@
-"""The fused training step at its edges: waits on MMAs that expire with the MMAs in flight."""
+"""The fused training step at its edges: waits on MMAs that expire with the MMAs in flight, device arrays
+on any float boundary."""
 import numpy as np
 import pytest
 
@@ -32,3 +33,21 @@ def test_expired_mma_wait_is_reported_and_recovers(vsdmo, batch):
     fresh = vsdmo.ProposalModel(seed=7)
     for a, b in zip(m.gradients(X[:384], T[:384]), fresh.gradients(X[:384], T[:384])):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_device_arrays_on_any_float_boundary(vsdmo, offset):
+    import torch
+    X, T = _pairs(700, 4)
+    params = []
+    for o in (0, offset):
+        f = torch.zeros(X.size + 4, device="cuda")
+        t = torch.zeros(T.size + 4, device="cuda")
+        f[o:o + X.size] = torch.from_numpy(X.ravel()).cuda()
+        t[o:o + T.size] = torch.from_numpy(T.ravel()).cuda()
+        torch.cuda.synchronize()
+        m = vsdmo.ProposalModel(seed=3)
+        hist = m.train(None, None, steps=3, batch=256, lr=1e-3, seed=2, n_rows=len(X),
+                       device_ptrs=(f.data_ptr() + 4 * o, t.data_ptr() + 4 * o))
+        params.append((hist, m.get_params()))
+    assert np.array_equal(params[0][0], params[1][0]) and np.array_equal(params[0][1], params[1][1])

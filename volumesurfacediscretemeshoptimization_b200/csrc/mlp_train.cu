@@ -258,10 +258,15 @@ __global__ void __launch_bounds__(TT, 1) k_train_tile(TileArgs p) {
         {
             const int r = tid & 127, half = tid >> 7;   // the first half's r is its epilogue row
             const long src = p.idx ? __ldcg(p.idx + tile * 128 + r) : (long)tile * 128 + r;
-            const float4* f = reinterpret_cast<const float4*>(p.feats + src * IN) + half * 12;
+            const float* f = p.feats + src * IN + half * 48;
             float4 q[12];
+            if ((reinterpret_cast<size_t>(p.feats) & 15) == 0) {
 #pragma unroll
-            for (int i = 0; i < 12; ++i) q[i] = __ldg(f + i);
+                for (int i = 0; i < 12; ++i) q[i] = __ldg(reinterpret_cast<const float4*>(f) + i);
+            } else {   // a caller's device array on no 16-byte boundary
+#pragma unroll
+                for (int i = 0; i < 12; ++i) q[i] = make_float4(__ldg(f + 4 * i), __ldg(f + 4 * i + 1), __ldg(f + 4 * i + 2), __ldg(f + 4 * i + 3));
+            }
 #pragma unroll
             for (int j = 0; j < OUT; ++j) T3[j] = __ldg(p.targets + src * OUT + j);
 #pragma unroll
