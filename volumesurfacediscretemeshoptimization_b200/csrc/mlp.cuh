@@ -48,7 +48,20 @@ struct TrainBuffers {
     int rows = 0, cap_parts = 0;
     DBuf<float> part, ws, loss_rows, loss;
     DBuf<int> idx;
-    void ensure(int B, cudaStream_t s);
+    // the sizes count once every buffer has them: a failed allocation leaves none behind
+    void ensure(int B, cudaStream_t s) {
+        const int parts = wgrad_parts(B);
+        if (B <= rows && parts <= cap_parts) return;
+        const int r = std::max(B, rows), c = std::max(parts, cap_parts);
+        rows = cap_parts = 0;
+        part.alloc((size_t)c * TRAIN_PART, s);
+        ws.alloc((size_t)(r / 32) * (3 * HID + OUTP), s);
+        loss_rows.alloc(r, s);
+        loss.alloc(1, s);
+        idx.alloc(2 * (size_t)r, s);
+        rows = r;
+        cap_parts = c;
+    }
 };
 
 struct Model {

@@ -579,18 +579,6 @@ int fused_tiles(int B) {
     return tiles % parts == 0 ? tiles / parts : 0;
 }
 
-void TrainBuffers::ensure(int B, cudaStream_t s) {
-    const int parts = wgrad_parts(B);
-    if (B <= rows && parts <= cap_parts) return;
-    rows = std::max(B, rows);
-    cap_parts = std::max(parts, cap_parts);
-    part.alloc((size_t)cap_parts * TRAIN_PART, s);
-    ws.alloc((size_t)(rows / 32) * (3 * HID + OUTP), s);
-    loss_rows.alloc(rows, s);
-    loss.alloc(1, s);
-    idx.alloc(2 * (size_t)rows, s);
-}
-
 namespace {
 // launch that may start while its predecessor on the stream drains
 template <class Args>

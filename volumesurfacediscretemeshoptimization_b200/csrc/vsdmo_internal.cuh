@@ -58,8 +58,10 @@ struct DBuf {
     void alloc(size_t count, cudaStream_t st) {
         release();
         s = st;
+        T* q = nullptr;   // a failed allocation leaves an empty buffer
+        if (count) VSDMO_CUDA(cudaMallocFromPoolAsync((void**)&q, count * sizeof(T), device_pool(), st));
+        p = q;
         n = count;
-        if (count) VSDMO_CUDA(cudaMallocFromPoolAsync((void**)&p, count * sizeof(T), device_pool(), st));
     }
     void release() {
         if (p) cudaFreeAsync(p, s);
