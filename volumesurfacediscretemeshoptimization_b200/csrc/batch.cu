@@ -368,9 +368,9 @@ size_t batch_smem(int maxk) { return (size_t)BATCH_WARPS * batch_warp_floats(max
 
 int flat_max_ring() { return 64; }
 
+// Raises the shared-memory limits on the current device (they belong to the device): once per optimiser and batch,
+// outside of any capture.
 void prepare_flat_kernels() {
-    static bool done = false;
-    if (done) return;
     const int mx = (int)flat_smem(flat_max_ring(), 4);
     const int bmx = (int)std::max(batch_smem(flat_max_ring()), batch_smem(F8_MAX_RING));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat8<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)flat8_smem(F8_MAX_RING)));
@@ -379,14 +379,12 @@ void prepare_flat_kernels() {
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     for (auto k : {k_batch_iter<PACKED>, k_batch_iter<GENERAL>, k_batch_iter<MIXED>})
         VSDMO_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bmx));
-    done = true;
 }
 
 void launch_dmo_flat(const Mesh& m, const DmoLaunch& L, int nq, int lanes, cudaStream_t s) {
     const int n = L.v1 - L.v0;
     if (n <= 0) return;
     if (m.maxHE > flat_max_ring()) throw Error(VSDMO_E_VALENCE, "a vertex has more halfedges than the flat kernel's ring budget");
-    prepare_flat_kernels();
     const int groups = 32 / lanes;
     const int maxk = std::max(m.maxHE, 1);
     const int per_block = BATCH_WARPS * groups;
@@ -403,7 +401,6 @@ void launch_dmo_flat(const Mesh& m, const DmoLaunch& L, int nq, int lanes, cudaS
 bool launch_dmo_flat_packed(const Mesh& m, const DmoLaunch& L, cudaStream_t s) {
     const int n = L.v1 - L.v0, maxk = std::max(m.maxHE, 1);
     if (n < FLAT_PACKED_MIN || maxk > F8_MAX_RING) return false;
-    prepare_flat_kernels();
     const int blocks = (n + 4 * F8_WARPS - 1) / (4 * F8_WARPS);
     VSDMO_CUDA(launch_chained(m.fk == 4 ? k_dmo_flat8<4> : k_dmo_flat8<3>, blocks, F8_WARPS * 32, flat8_smem(maxk), s, L.chained,
                               m.pos.p, m.he_rowptr.p, m.he.p, L.v0, L.v1, L.grid_scale, L.depth, maxk));

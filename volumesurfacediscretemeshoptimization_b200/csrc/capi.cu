@@ -690,6 +690,7 @@ VSDMO_API vsdmo_status vsdmo_opt_create(vsdmo_mesh_t mesh, const vsdmo_params* p
         o->done.alloc(1, s); o->done.zero();
         prepare_dmo_kernels();
         if (o->mode == MODE_ANGLE) prepare_angle_kernels();
+        if (o->mode == MODE_TRI2D || o->mode == MODE_FLAT) prepare_flat_kernels();
         if (o->kind == MK_HEX_COND) prepare_hex_cond_kernels();
         if (o->volsurf) prepare_surf_kernels();
         if (o->mode == MODE_SURF || o->slide || o->volsurf) init_surface_state(o.get());
