@@ -735,6 +735,7 @@ std::vector<std::string> Batch::autotune(int probe_iters) {
     cudaEvent_t e0, e1;
     VSDMO_CUDA(cudaEventCreate(&e0));
     VSDMO_CUDA(cudaEventCreate(&e1));
+    const std::vector<BatchConfig> before = cfg;
     std::vector<BatchConfig> chosen = cfg;
     try {
         for (auto& kv : buckets) {
@@ -791,8 +792,15 @@ std::vector<std::string> Batch::autotune(int probe_iters) {
             report.push_back(line);
         }
     } catch (...) {
+        // positions, configurations and all that upload_meshes derives from them (for one bucket so far) as they were
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
+        cfg = before;
+        try {
+            VSDMO_CUDA(cudaMemcpyAsync(pos.p, saved.p, sizeof(float4) * nV, cudaMemcpyDeviceToDevice, stream));
+            upload_meshes();
+        } catch (...) {   // the first error is the one to report
+        }
         throw;
     }
     cudaEventDestroy(e0);
