@@ -400,7 +400,8 @@ VSDMO_API vsdmo_status vsdmo_opt_estimate_surface_points(vsdmo_opt_t opt, int vi
 /* Many independent flat (z = 0) tri and quad meshes optimised together: one persistent launch
  * per iteration takes (mesh, colour class, vertex chunk) work items in colour-major order, each
  * mesh with its own grid (4 or 8 candidates per axis), refinement levels (1..4) and lanes per
- * vertex (8, 16 or 32); iterations are replayed from a captured CUDA graph. The search per
+ * vertex (8, 16 or 32; 8 x 8 grids of batches without a vertex of more than 16 halfedges are
+ * searched by eight lanes per vertex whatever is set); iterations are replayed from a captured CUDA graph. The search per
  * vertex is that of DMOTriFlatClass (dmo/DMOTriFlatImplCub.h:24-152, the reference runs one
  * mesh per process). The reference has no batched mode: this replaces a loop over
  * DMOTriFlatClass objects, one per mesh.
@@ -438,7 +439,8 @@ VSDMO_API vsdmo_status vsdmo_batch_set_config(vsdmo_batch_t batch, const int32_t
                                               const int32_t* lanes);
 /* Autotuner: per size bucket (free vertices < 2,000 / < 10,000 / more) the configuration with
  * the least device time to reach, within 1e-4, the mean and minimum quality that 8 / 3 / 32
- * reaches in probe_iters iterations. Positions are left as they were. The report (one line per
+ * reaches in probe_iters iterations; lanes stay 32 where they make no difference. Positions are
+ * left as they were, on an error also the configurations. The report (one line per
  * bucket) is written to `report` (truncated to report_len bytes, may be NULL). */
 VSDMO_API vsdmo_status vsdmo_batch_autotune(vsdmo_batch_t batch, int probe_iters, char* report, int report_len);
 /* Counts: 0 meshes, 1 vertices, 2 work items per iteration, 3 colour classes (all meshes),

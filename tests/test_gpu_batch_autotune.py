@@ -30,3 +30,15 @@ def test_failed_trial_leaves_the_batch_as_it_was(vsdmo):
     fresh.set_config(*config)
     fresh.iterate(3)
     assert np.array_equal(b.positions(), fresh.positions())
+
+
+def test_lanes_are_tried_only_where_the_search_has_them(vsdmo):
+    """8 x 8 grids with rings of up to 16 run eight lanes per vertex whatever is configured: trials that differ in
+    lanes alone would be the same search, and the choice among them noise."""
+    meshes = [(TRI, *G.tri_grid(n, n)) for n in (20, 30, 40)] + [(QUAD, *G.quad_grid(n, n)) for n in (60, 70, 80, 110, 120)]
+    for repeat in range(3):
+        b = vsdmo.BatchDMO(meshes)
+        report = b.autotune(2)
+        n, depth, lanes = b.config()
+        assert np.all(lanes[n == 8] == 32), report
+        b.close()

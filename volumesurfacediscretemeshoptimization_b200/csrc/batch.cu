@@ -707,7 +707,7 @@ void Batch::set_positions(const float* d_in) {
 // reference configuration (8 candidates per axis, 3 levels, 32 lanes) runs `probe_iters`
 // iterations of the bucket's meshes from their current positions; its mean (over the bucket)
 // of the meshes' mean quality and its minimum of their minimum quality are the target. Every
-// other configuration (4 or 8 per axis, 2-4 levels, 8 / 16 / 32 lanes per vertex) runs up to
+// other configuration (4 or 8 per axis, 2-4 levels, 8 / 16 / 32 lanes per vertex where the search has lanes to choose) runs up to
 // 2 x probe_iters iterations from the same positions until it reaches the target (within
 // 1e-4); the configuration with the least device time to the target wins. Timing: CUDA
 // events around each iteration's launch. Positions and statistics are restored afterwards.
@@ -730,8 +730,10 @@ std::vector<std::string> Batch::autotune(int probe_iters) {
     cands.push_back({8, 3, 32});
     for (int nq : {8, 4})
         for (int d : {2, 3, 4})
-            for (int l : {32, 16, 8})
+            for (int l : {32, 16, 8}) {
+                if (nq == 8 && maxk <= F8_MAX_RING && l != 32) continue;   // packed: lanes make no difference
                 if (!(nq == 8 && d == 3 && l == 32)) cands.push_back({nq, d, l});
+            }
     cudaEvent_t e0, e1;
     VSDMO_CUDA(cudaEventCreate(&e0));
     VSDMO_CUDA(cudaEventCreate(&e1));
