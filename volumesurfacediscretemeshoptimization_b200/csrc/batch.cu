@@ -167,10 +167,6 @@ k_dmo_flat8(float4* pos_, const int* __restrict__ rowptr, const int4* __restrict
 }
 
 // ---- the persistent batched iteration -----------------------------------------------------------
-// floats of shared memory per warp: up to 4 groups of either search
-__host__ __device__ constexpr int batch_warp_floats(int maxk) {
-    return maxk > F8_MAX_RING || maxk * BCO > f8_group_floats(maxk) ? 4 * maxk * BCO : 4 * f8_group_floats(maxk);
-}
 
 // SEARCH: every mesh is searched four vertices per warp (PACKED), none is (GENERAL), or some are (MIXED): only
 // what is needed is in the kernel (with both in one, half the stalls were instruction fetches; 4 x 4 grids on 256
@@ -178,6 +174,11 @@ __host__ __device__ constexpr int batch_warp_floats(int maxk) {
 // Registers: four blocks per SM at 64 against three at 80 and two at 96: 2.28 / 2.33 / 2.80 ms per iteration
 // of 256 meshes (measured without the rings searched apart, which take four blocks to 2.35).
 enum { PACKED, GENERAL, MIXED };
+// floats of shared memory per warp: up to 4 groups of the searches in the kernel (the general one alone fits four
+// blocks per SM up to rings of 42, with the packed one's 36 floats per element it was three from 12 on)
+__host__ __device__ constexpr int batch_warp_floats(int search, int maxk) {
+    return search == GENERAL || maxk > F8_MAX_RING || maxk * BCO > f8_group_floats(maxk) ? 4 * maxk * BCO : 4 * f8_group_floats(maxk);
+}
 template <int SEARCH>
 __global__ void __launch_bounds__(BATCH_WARPS * 32, 4)
 k_batch_iter(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ he,
@@ -186,7 +187,7 @@ k_batch_iter(float4* __restrict__ pos, const int* __restrict__ rowptr, const int
              int* __restrict__ err) {
     extern __shared__ float4 bsm4[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float* wco = reinterpret_cast<float*>(bsm4) + (size_t)w * batch_warp_floats(maxk);
+    float* wco = reinterpret_cast<float*>(bsm4) + (size_t)w * batch_warp_floats(SEARCH, maxk);
     while (true) {
         int idx = 0;
         if (lane == 0) idx = atomicAdd(head, 1);
@@ -364,7 +365,7 @@ __global__ void k_batch_concat_int(const int* in, int n, int off, int* out) {
 // ---- host ---------------------------------------------------------------------------------------------
 size_t flat_smem(int maxk, int groups) { return (size_t)BATCH_WARPS * groups * maxk * BCO * sizeof(float); }
 size_t flat8_smem(int maxk) { return (size_t)F8_WARPS * 4 * f8_group_floats(maxk) * sizeof(float); }
-size_t batch_smem(int maxk) { return (size_t)BATCH_WARPS * batch_warp_floats(maxk) * sizeof(float); }
+size_t batch_smem(int search, int maxk) { return (size_t)BATCH_WARPS * batch_warp_floats(search, maxk) * sizeof(float); }
 
 int flat_max_ring() { return 64; }
 
@@ -372,7 +373,7 @@ int flat_max_ring() { return 64; }
 // outside of any capture.
 void prepare_flat_kernels() {
     const int mx = (int)flat_smem(flat_max_ring(), 4);
-    const int bmx = (int)std::max(batch_smem(flat_max_ring()), batch_smem(F8_MAX_RING));
+    const int bmx = (int)std::max(batch_smem(MIXED, flat_max_ring()), batch_smem(MIXED, F8_MAX_RING));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat8<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)flat8_smem(F8_MAX_RING)));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat8<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)flat8_smem(F8_MAX_RING)));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_flat<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
@@ -601,14 +602,19 @@ void Batch::ensure_items() {
     items_dirty = false;
 }
 
+int Batch::search_kind() const { return all_packed ? PACKED : none_packed ? GENERAL : MIXED; }
+
 void Batch::ensure_launch_setup() {
-    if (blocks) return;
+    if (blocks[0]) return;
     prepare_flat_kernels();
-    int dev = 0, sms = 148, per = 1;
+    int dev = 0, sms = 148;
     VSDMO_CUDA(cudaGetDevice(&dev));
     VSDMO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    VSDMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_iter<MIXED>, BATCH_WARPS * 32, batch_smem(maxk)));
-    blocks = sms * std::max(per, 1);
+    int per[3];
+    VSDMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[PACKED], k_batch_iter<PACKED>, BATCH_WARPS * 32, batch_smem(PACKED, maxk)));
+    VSDMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[GENERAL], k_batch_iter<GENERAL>, BATCH_WARPS * 32, batch_smem(GENERAL, maxk)));
+    VSDMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[MIXED], k_batch_iter<MIXED>, BATCH_WARPS * 32, batch_smem(MIXED, maxk)));
+    for (int i = 2; i >= 0; --i) blocks[i] = sms * std::max(per[i], 1);
 }
 
 void Batch::quality(BatchStats* out, int* d_it, int init, int advance, cudaStream_t s) {
@@ -622,9 +628,10 @@ void Batch::quality(BatchStats* out, int* d_it, int init, int advance, cudaStrea
 void Batch::launch_iteration(const BatchItem* d_it, int n, bool with_stats, cudaStream_t s) {
     VSDMO_CUDA(cudaMemsetAsync(done.p, 0, sizeof(int) * done.n, s));
     VSDMO_CUDA(cudaMemsetAsync(head.p, 0, sizeof(int), s));
-    const auto kernel = all_packed ? k_batch_iter<PACKED> : none_packed ? k_batch_iter<GENERAL> : k_batch_iter<MIXED>;
-    kernel<<<blocks, BATCH_WARPS * 32, batch_smem(maxk), s>>>(pos.p, rowptr.p, he.p, d_it, n, d_meshes.p, csize.p, done.p,
-                                                              head.p, maxk, grid_scale, err.p);
+    const int search = search_kind();
+    const auto kernel = search == PACKED ? k_batch_iter<PACKED> : search == GENERAL ? k_batch_iter<GENERAL> : k_batch_iter<MIXED>;
+    kernel<<<blocks[search], BATCH_WARPS * 32, batch_smem(search, maxk), s>>>(pos.p, rowptr.p, he.p, d_it, n, d_meshes.p, csize.p, done.p,
+                                                                      head.p, maxk, grid_scale, err.p);
     VSDMO_CHECK_LAUNCH();
     if (with_stats) quality(stats.p, d_iter.p, 0, 1, s);
 }

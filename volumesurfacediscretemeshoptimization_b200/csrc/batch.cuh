@@ -80,7 +80,7 @@ struct Batch {
     bool all_packed = false, none_packed = false;
     int n_items = 0;
     bool items_dirty = true;
-    int blocks = 0;
+    int blocks[3] = { 0, 0, 0 };   // resident blocks of the iteration kernel, per search_kind
     int iters_done = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -96,6 +96,7 @@ struct Batch {
     void get_positions(float* d_xyz_out) const;        // input numbering, [nV x 3]
     void set_positions(const float* d_xyz_in);
     int n_colors_total() const;
+    int search_kind() const;      // which searches the iteration's kernel needs
     int chunk(int i) const;       // vertices of one work item of mesh i
     long class_avg = 0;           // vertices of a colour class over all meshes
 

@@ -194,7 +194,7 @@ VSDMO_API long vsdmo_batch_info(vsdmo_batch_t batch, int which) {
     }
     case 3: return b.n_colors_total();
     case 4: return b.iters_done;
-    case 5: return b.blocks;
+    case 5: return b.blocks[b.search_kind()];
     case 6: return b.maxk;
     default: return -1;
     }
