@@ -641,15 +641,8 @@ k_dmo_hex(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* 
     const HexItems ring{co, k, es, ea, nullptr, 0};
     float* scratch = reinterpret_cast<float*>(corner);
     float dx, dy, dz;
-    bool moved;
-    if (__any_sync(FULL, odd)) {
-        const float3 d = hex_full_search(co, k, es, ea, sx, sy, sz, grid_scale, depth);
-        dx = d.x; dy = d.y; dz = d.z;
-        moved = dx != 0.f || dy != 0.f || dz != 0.f;
-    } else {
-        moved = hex_plain_search(ring, scratch, reinterpret_cast<unsigned short*>(scratch + TS_WARP_BYTES / 4), sx, sy, sz, grid_scale, depth,
-                                 lane, dx, dy, dz);
-    }
+    const bool moved = hex_plain_search(ring, __any_sync(FULL, odd), scratch, reinterpret_cast<unsigned short*>(scratch + TS_WARP_BYTES / 4),
+                                        sx, sy, sz, grid_scale, depth, lane, dx, dy, dz);
     if (moved && lane == 0) pos[v] = tet_unscale(c0, dx, dy, dz, ex);
 }
 

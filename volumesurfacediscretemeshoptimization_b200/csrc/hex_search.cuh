@@ -161,39 +161,65 @@ static __device__ __forceinline__ bool hex_odd(const float* __restrict__ c, floa
     return odd;
 }
 
-// The search of a ring with such a halfhex: every candidate by hex_key1. NaN keys never win.
-static __device__ __noinline__ float3 hex_full_search(const float* __restrict__ co, int k, float es, float ea, float sx, float sy, float sz,
-                                                      float grid_scale, int depth) {
+// All candidates of a level by hex_key1, four along x at a time (they share what depends on y and z): the largest
+// key and, on ties, the lowest linear index, on every lane; NaN keys never win.
+static __device__ __noinline__ float2 hex_level(const float* __restrict__ co, int k, float es, float ea, QuadLevel lv) {
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const float off = grid_offset(lane & 7);
-    float dx = 0.f, dy = 0.f, dz = 0.f, ds = grid_scale, qLast = hex_key1(co, k, 0.f, 0.f, 0.f, es, ea);
+    float bk = -FLT_MAX;
+    int bi = 1 << 30;
+    const float y = fmaf(grid_offset(lane & 7), lv.Sy, lv.dy), t1y = y * y, t3y = (3.f * y) * y;
 #pragma unroll 1
-    for (int level = 0; level < depth; ++level) {
-        const QuadLevel lv{dx, dy, dz, ds * sx, ds * sy, ds * sz, 0.f, 0.f, 0.f, false};
-        ds = ds * (2.0f / 7.0f);
-        float bk = -FLT_MAX;
-        int bi = 1 << 30;
-#pragma unroll 1
-        for (int i = lane; i < 512; i += 32) {
-            const float3 c = grid_candidate(i, off, lv);
-            const float key = hex_key1(co, k, c.x, c.y, c.z, es, ea);
-            if (key > bk) { bk = key; bi = i; }
+    for (int part = 0; part < 4; ++part) {
+        const int zi = (lane >> 3) + 4 * (part >> 1), x0 = 4 * (part & 1);
+        const float z = fmaf(grid_offset(zi), lv.Sz, lv.dz), t1z = z * z, t3z = (3.f * z) * z;
+        float x[4], N[4], D[4];
+        unsigned zero = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            x[i] = fmaf(grid_offset(x0 + i), lv.Sx, lv.dx);
+            N[i] = co[0]; D[i] = co[1];
         }
-        const float best = redux_max(bk);
-        bi = (int)__reduce_min_sync(FULL, bk == best ? (unsigned)bi : 1u << 30);
-        if (bi < 512 && qLast < best) {
-            const float3 c = grid_candidate(bi, off, lv);
-            dx = c.x; dy = c.y; dz = c.z;
-            qLast = best;
+#pragma unroll 1
+        for (int h = 0; h < k; ++h) {
+            const float* c = co + HEX_CO * h;
+            const float cn = c[0], cd = c[1];
+            if (c[2] != 0.f) zero = 15u;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (h > 0 && cn * D[i] < N[i] * cd) { N[i] = cn; D[i] = cd; }
+#pragma unroll
+            for (int j = 0; j < 5; ++j) {
+                const float* q = c + 3 + 8 * j;
+                const bool a3 = (j == 1 || j == 4);
+                const float sY = fmaf(q[1], y, fmaf(q[2], z, q[3]));
+                const float aY = (q[7] + fmaf(q[6], z, a3 ? t3z : t1z)) + fmaf(q[5], y, a3 ? t3y : t1y);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float s = fmaf(q[0], x[i], sY);
+                    const float A = aY + fmaf(q[4], x[i], a3 ? (3.f * x[i]) * x[i] : x[i] * x[i]);
+                    if (s < es || A < ea) { zero |= 1u << i; continue; }
+                    const float num = s * s, den = (A * A) * A;
+                    if (num * D[i] < N[i] * den) { N[i] = num; D[i] = den; }
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float key = (zero >> i) & 1u ? 0.f : N[i] / D[i];
+            const int idx = x0 + i + 8 * (lane & 7) + 64 * zi;
+            if (key > bk || (key == bk && idx < bi)) { bk = key; bi = idx; }
         }
     }
-    return make_float3(dx, dy, dz);
+    const float best = redux_max(bk);
+    bi = (int)__reduce_min_sync(FULL, bk == best ? (unsigned)bi : 1u << 30);
+    return make_float2(best, __int_as_float(bi));
 }
 
 // Search from the local origin; returns whether the vertex moved. scratch: TS_WARP_BYTES of the warp,
 // subset: 6 k places.
-static __device__ __forceinline__ bool hex_plain_search(HexItems ring, float* __restrict__ scratch,
+// odd: every level in full (hex_odd).
+static __device__ __forceinline__ bool hex_plain_search(HexItems ring, bool odd, float* __restrict__ scratch,
                                                         unsigned short* __restrict__ subset, float sx, float sy, float sz,
                                                         float grid_scale, int depth, int lane, float& dx, float& dy,
                                                         float& dz) {
@@ -209,49 +235,63 @@ static __device__ __forceinline__ bool hex_plain_search(HexItems ring, float* __
         if (h == 0 || c[0] * D < N * c[1]) { N = c[0]; D = c[1]; }
     }
     const float Q = N / D;
-    float qLast = ring.group_key(0.f, 0.f, 0.f, 32, lane);
+    float qLast = odd ? hex_key1(ring.co, ring.k, 0.f, 0.f, 0.f, ring.es, ring.ea) : ring.group_key(0.f, 0.f, 0.f, 32, lane);
     bool moved = false;
     float ds = grid_scale;
     for (int level = 0; level < depth; ++level) {
         QuadLevel lv{dx, dy, dz, ds * sx, ds * sy, ds * sz, 0.f, 0.f, 0.f, false};
         ds = ds * (2.0f / 7.0f);
-        const float U = fminf(ring.upper(lv, lane), Q);
-        const float clear_of_U = U + (U * 0x1p-13f + 1e-37f);
-        if (clear_of_U < qLast) continue;   // nothing on the box can beat the current key
-        lv.sq2 = sqrt_approx(clear_of_U) * (1.f + 0x1p-20f);
-        lv.ties = U == Q;
-        const float thr = key_below(fminf(qLast, U));
-        if (thr > 0.f) lv.sq = sqrt_approx(thr) * (1.f - 0x1p-20f);
-        else lv.low = ring.es * 0.999f;   // a key above zero needs det >= es
-        float s[16], rho, above;
-        quad_filter<HexItems, true, false>(ring, lv, scratch, lane, s, rho, above, subset, ring.m);
-        ring.subset = subset;
-        const bool ties = lv.ties && above < FLT_MAX;   // candidates clearly above have the key Q
-        float bk = -FLT_MAX, cut = 0.f;
+        if (lv.Sx == 0.f && lv.Sy == 0.f && lv.Sz == 0.f) continue;   // a lattice: every candidate is the centre
+        float bk = -FLT_MAX;
         int bi = 1 << 30;
-        unsigned clear = ties ? at_least(s, above) : 0u;
-        if (qLast < Q) {
-            int place;
-            const float top = top_candidate(s, bi, place);
-            if (top < 0.f) continue;   // every candidate is dropped
-            if (top >= 0.f) {
-                const float3 c = grid_candidate(bi, off, lv);
-                bk = ring.m > 8 ? ring.group_key(c.x, c.y, c.z, 32, lane) : ring.key(c.x, c.y, c.z);
-                if (thr > 0.f && bk > qLast) cut = (sqrt_approx(key_below(bk)) * (1.f - 0x1p-20f) - lv.sq) * (rho * 0.999f);
-                if (!(cut > 0.f)) cut = 0.f;
-            } else {
-                bi = 1 << 30;
-            }
-            if (ties) {
-                int low = 1 << 30;
+        bool full = odd;
+        if (!full) {
+            const float U = fminf(ring.upper(lv, lane), Q);
+            const float clear_of_U = U + (U * 0x1p-13f + 1e-37f);
+            if (clear_of_U < qLast) continue;   // nothing on the box can beat the current key
+            lv.sq2 = sqrt_approx(clear_of_U) * (1.f + 0x1p-20f);
+            lv.ties = U == Q;
+            const float thr = key_below(fminf(qLast, U));
+            if (thr > 0.f) lv.sq = sqrt_approx(thr) * (1.f - 0x1p-20f);
+            else lv.low = ring.es * 0.999f;   // a key above zero needs det >= es
+            float s[16], rho, above;
+            quad_filter<HexItems, true, false>(ring, lv, scratch, lane, s, rho, above, subset, ring.m);
+            ring.subset = subset;
+            const bool ties = lv.ties && above < FLT_MAX;   // candidates clearly above have the key Q
+            float cut = 0.f;
+            unsigned clear = ties ? at_least(s, above) : 0u;
+            if (qLast < Q) {
+                int place;
+                const float top = top_candidate(s, bi, place);
+                if (top < 0.f) continue;   // every candidate is dropped
+                if (top >= 0.f) {
+                    const float3 c = grid_candidate(bi, off, lv);
+                    bk = ring.m > 8 ? ring.group_key(c.x, c.y, c.z, 32, lane) : ring.key(c.x, c.y, c.z);
+                    if (thr > 0.f && bk > qLast) cut = (sqrt_approx(key_below(bk)) * (1.f - 0x1p-20f) - lv.sq) * (rho * 0.999f);
+                    if (!(cut > 0.f)) cut = 0.f;
+                } else {
+                    bi = 1 << 30;
+                }
+                if (ties) {
+                    int low = 1 << 30;
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (clear & (0x8000u >> i)) low = min(low, grid_index(lane, i));
-                low = (int)__reduce_min_sync(FULL, (unsigned)low);
-                if (low < 512 && (Q > bk || (Q == bk && low < bi))) { bk = Q; bi = low; }
+                    for (int i = 0; i < 16; ++i)
+                        if (clear & (0x8000u >> i)) low = min(low, grid_index(lane, i));
+                    low = (int)__reduce_min_sync(FULL, (unsigned)low);
+                    if (low < 512 && (Q > bk || (Q == bk && low < bi))) { bk = Q; bi = low; }
+                }
             }
+            const unsigned alive = at_least(s, cut) & ~clear;
+            // Boxes that shrink with the smallest ring distance can leave every candidate within the margins. Judged one
+            // per lane, a candidate and item costs some 35 instructions; in full, four candidates and a halfhex 120.
+            full = ((__reduce_add_sync(FULL, __popc(alive)) + 31) >> 5) * ring.m > 14 * ring.k;
+            if (!full) judge(ring, lv, alive, off, list, lane, bk, bi);
         }
-        judge(ring, lv, at_least(s, cut) & ~clear, off, list, lane, bk, bi);
+        if (full) {
+            const float2 best = hex_level(ring.co, ring.k, ring.es, ring.ea, lv);
+            bk = best.x;
+            bi = __float_as_int(best.y);
+        }
         if (bi < 512 && qLast < bk) {
             const float3 c = grid_candidate(bi, off, lv);
             dx = c.x; dy = c.y; dz = c.z;
