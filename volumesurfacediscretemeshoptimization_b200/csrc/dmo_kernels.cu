@@ -585,6 +585,10 @@ k_dmo_tet_learned(float4* __restrict__ pos, const int* __restrict__ rowptr, cons
 // takes 0.50 ms: 17 colour classes of up to 2,600 vertices, one wave each, bound by one search's latency.
 constexpr int HEX_MAX_RING = 64;
 constexpr int HEX_MIN_BLOCKS = 20;   // 96 registers
+// Classes of up to so many vertices (one wave of five blocks per SM) get four warps per vertex, for the levels that are
+// evaluated in full: a lattice of 12^3 cells with 1e-6 of jitter takes 441 us per iteration, 868 with one warp (554 with
+// every candidate in a block of 128 threads, as before the filter).
+constexpr int HEX_TEAM_MAX = 148 * (HEX_MIN_BLOCKS / 4);
 
 // coefficients, then the corners of the setup or the search's scratch and item list
 size_t hex_smem_bytes(int maxk) {
@@ -592,12 +596,10 @@ size_t hex_smem_bytes(int maxk) {
            std::max((size_t)TS_WARP_BYTES + 6 * maxk * sizeof(unsigned short), (size_t)7 * maxk * sizeof(float4));
 }
 
-__global__ void __launch_bounds__(32, HEX_MIN_BLOCKS)
-k_dmo_hex(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ hh, int v0,
-          float grid_scale, int depth, int maxk) {
-    extern __shared__ float4 smem[];
-    const int lane = threadIdx.x;
-    const int v = v0 + blockIdx.x;
+template <int W>
+__device__ __forceinline__ void hex_vertex(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ hh, int v,
+                                           float grid_scale, int depth, int maxk, float4* smem, HexTeam* team) {
+    const int lane = threadIdx.x & 31;
     float* co = reinterpret_cast<float*>(smem);
     float4* corner = smem + maxk * (HEX_CO / 4);
     const int b = rowptr[v], k = rowptr[v + 1] - b;
@@ -641,9 +643,30 @@ k_dmo_hex(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* 
     const HexItems ring{co, k, es, ea, nullptr, 0};
     float* scratch = reinterpret_cast<float*>(corner);
     float dx, dy, dz;
-    const bool moved = hex_plain_search(ring, __any_sync(FULL, odd), scratch, reinterpret_cast<unsigned short*>(scratch + TS_WARP_BYTES / 4),
+    const bool moved = hex_plain_search<W>(ring, __any_sync(FULL, odd), team, scratch, reinterpret_cast<unsigned short*>(scratch + TS_WARP_BYTES / 4),
                                         sx, sy, sz, grid_scale, depth, lane, dx, dy, dz);
     if (moved && lane == 0) pos[v] = tet_unscale(c0, dx, dy, dz, ex);
+}
+
+template <int W>
+__global__ void __launch_bounds__(32 * W, W == 1 ? HEX_MIN_BLOCKS : HEX_MIN_BLOCKS / W)
+k_dmo_hex(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ hh, int v0,
+          float grid_scale, int depth, int maxk) {
+    extern __shared__ float4 smem[];
+    const int v = v0 + blockIdx.x;
+    if (W == 1) {
+        hex_vertex<1>(pos, rowptr, hh, v, grid_scale, depth, maxk, smem, nullptr);
+        return;
+    }
+    __shared__ HexTeam team;
+    const int w = threadIdx.x >> 5;
+    if (w > 0) {
+        hex_team_help(&team, reinterpret_cast<float*>(smem), w);
+        return;
+    }
+    hex_vertex<W>(pos, rowptr, hh, v, grid_scale, depth, maxk, smem, &team);
+    if ((threadIdx.x & 31) == 0) team.go = 0;
+    __syncthreads();
 }
 
 // ---- flat triangles ---------------------------------------------------------------------------
@@ -1063,7 +1086,8 @@ void launch_dmo_hex(const Mesh& m, const DmoLaunch& L, cudaStream_t s) {
     const int n = L.v1 - L.v0;
     if (n <= 0) return;
     const int maxk = m.maxTets;
-    k_dmo_hex<<<n, 32, hex_smem_bytes(maxk), s>>>(m.pos.p, m.hf_rowptr.p, m.hh.p, L.v0, L.grid_scale, L.depth, maxk);
+    const auto kernel = n <= HEX_TEAM_MAX ? k_dmo_hex<4> : k_dmo_hex<1>;
+    kernel<<<n, n <= HEX_TEAM_MAX ? 128 : 32, hex_smem_bytes(maxk), s>>>(m.pos.p, m.hf_rowptr.p, m.hh.p, L.v0, L.grid_scale, L.depth, maxk);
     VSDMO_CHECK_LAUNCH();
 }
 
@@ -1080,8 +1104,8 @@ void prepare_dmo_kernels() {
                                     TET_WARPS * (TET_MAX_RING * 2 + 32) * (int)sizeof(float4)));
     VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_tet_list, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)tet_smem_bytes(TET_MAX_RING)));
-    VSDMO_CUDA(cudaFuncSetAttribute(k_dmo_hex, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)hex_smem_bytes(HEX_MAX_RING)));
+    for (auto k : {k_dmo_hex<1>, k_dmo_hex<4>})
+        VSDMO_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hex_smem_bytes(HEX_MAX_RING)));
 }
 int dmo_tri2d_max_ring() { return TRI_MAX_RING; }
 int quality_stats_blocks() { return QS_BLOCKS; }

@@ -161,33 +161,43 @@ static __device__ __forceinline__ bool hex_odd(const float* __restrict__ c, floa
     return odd;
 }
 
-// All candidates of a level by hex_key1, four along x at a time (they share what depends on y and z): the largest
-// key and, on ties, the lowest linear index, on every lane; NaN keys never win.
-static __device__ __noinline__ float2 hex_level(const float* __restrict__ co, int k, float es, float ea, QuadLevel lv) {
+// All candidates of a level by hex_key1, eight (four) along x at a time: they share the loads and what depends on y and
+// z, and their folds are independent chains. By one warp, or by warp w of a team of four, a quarter each: the
+// largest key and, on ties, the lowest linear index, on every lane of the warp; NaN keys never win.
+template <int W>
+static __device__ __noinline__ float2 hex_level(const float* __restrict__ co, int k, float es, float ea, QuadLevel lv, int w) {
     constexpr unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
+    constexpr int NX = W == 1 ? 8 : 4;
+    const int lane = threadIdx.x & 31, x0 = W == 1 ? 0 : 4 * (w & 1);
     float bk = -FLT_MAX;
     int bi = 1 << 30;
     const float y = fmaf(grid_offset(lane & 7), lv.Sy, lv.dy), t1y = y * y, t3y = (3.f * y) * y;
+    float x[NX], t1x[NX], t3x[NX];
+#pragma unroll
+    for (int i = 0; i < NX; ++i) {
+        x[i] = fmaf(grid_offset(x0 + i), lv.Sx, lv.dx);
+        t1x[i] = x[i] * x[i];
+        t3x[i] = (3.f * x[i]) * x[i];
+    }
 #pragma unroll 1
-    for (int part = 0; part < 4; ++part) {
-        const int zi = (lane >> 3) + 4 * (part >> 1), x0 = 4 * (part & 1);
+    for (int part = W == 1 ? 0 : w >> 1; part < (W == 1 ? 2 : (w >> 1) + 1); ++part) {
+        const int zi = (lane >> 3) + 4 * part;
         const float z = fmaf(grid_offset(zi), lv.Sz, lv.dz), t1z = z * z, t3z = (3.f * z) * z;
-        float x[4], N[4], D[4];
+        float N[NX], D[NX];
         unsigned zero = 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            x[i] = fmaf(grid_offset(x0 + i), lv.Sx, lv.dx);
-            N[i] = co[0]; D[i] = co[1];
-        }
+        for (int i = 0; i < NX; ++i) { N[i] = co[0]; D[i] = co[1]; }
 #pragma unroll 1
         for (int h = 0; h < k; ++h) {
             const float* c = co + HEX_CO * h;
             const float cn = c[0], cd = c[1];
-            if (c[2] != 0.f) zero = 15u;
+            if (c[2] != 0.f) zero = 0xffu;
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (h > 0 && cn * D[i] < N[i] * cd) { N[i] = cn; D[i] = cd; }
+            for (int i = 0; i < NX; ++i) {
+                const bool less = h > 0 && cn * D[i] < N[i] * cd;
+                N[i] = less ? cn : N[i];
+                D[i] = less ? cd : D[i];
+            }
 #pragma unroll
             for (int j = 0; j < 5; ++j) {
                 const float* q = c + 3 + 8 * j;
@@ -195,17 +205,20 @@ static __device__ __noinline__ float2 hex_level(const float* __restrict__ co, in
                 const float sY = fmaf(q[1], y, fmaf(q[2], z, q[3]));
                 const float aY = (q[7] + fmaf(q[6], z, a3 ? t3z : t1z)) + fmaf(q[5], y, a3 ? t3y : t1y);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < NX; ++i) {
                     const float s = fmaf(q[0], x[i], sY);
-                    const float A = aY + fmaf(q[4], x[i], a3 ? (3.f * x[i]) * x[i] : x[i] * x[i]);
-                    if (s < es || A < ea) { zero |= 1u << i; continue; }
+                    const float A = aY + fmaf(q[4], x[i], a3 ? t3x[i] : t1x[i]);
+                    const bool null = s < es || A < ea;   // the key is zero, whatever the fold holds
                     const float num = s * s, den = (A * A) * A;
-                    if (num * D[i] < N[i] * den) { N[i] = num; D[i] = den; }
+                    const bool less = num * D[i] < N[i] * den;
+                    zero |= null ? 1u << i : 0u;
+                    N[i] = less ? num : N[i];
+                    D[i] = less ? den : D[i];
                 }
             }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < NX; ++i) {
             const float key = (zero >> i) & 1u ? 0.f : N[i] / D[i];
             const int idx = x0 + i + 8 * (lane & 7) + 64 * zi;
             if (key > bk || (key == bk && idx < bi)) { bk = key; bi = idx; }
@@ -216,10 +229,47 @@ static __device__ __noinline__ float2 hex_level(const float* __restrict__ co, in
     return make_float2(best, __int_as_float(bi));
 }
 
+// What a team of four warps per vertex shares: the first one searches, the others wait for levels to be evaluated in full
+struct HexTeam {
+    QuadLevel lv;
+    float es, ea;
+    int k, go;
+    float2 best[4];
+};
+
+// the other warps' loop; every barrier pairs with one of hex_team_level or, with go = 0, of the end
+static __device__ __forceinline__ void hex_team_help(HexTeam* team, const float* __restrict__ co, int w) {
+    while (true) {
+        __syncthreads();
+        if (!team->go) return;
+        const float2 r = hex_level<4>(co, team->k, team->es, team->ea, team->lv, w);
+        if ((threadIdx.x & 31) == 0) team->best[w] = r;
+        __syncthreads();
+    }
+}
+
+static __device__ __forceinline__ float2 hex_team_level(HexTeam* team, const float* __restrict__ co, int k, float es, float ea, const QuadLevel& lv) {
+    if ((threadIdx.x & 31) == 0) {
+        team->lv = lv;
+        team->es = es; team->ea = ea; team->k = k; team->go = 1;
+    }
+    __syncthreads();
+    float2 best = hex_level<4>(co, k, es, ea, lv, 0);
+    __syncthreads();
+#pragma unroll
+    for (int w = 1; w < 4; ++w) {
+        const float2 r = team->best[w];
+        if (r.x > best.x || (r.x == best.x && __float_as_int(r.y) < __float_as_int(best.y))) best = r;
+    }
+    __syncwarp();
+    return best;
+}
+
 // Search from the local origin; returns whether the vertex moved. scratch: TS_WARP_BYTES of the warp,
 // subset: 6 k places.
-// odd: every level in full (hex_odd).
-static __device__ __forceinline__ bool hex_plain_search(HexItems ring, bool odd, float* __restrict__ scratch,
+// odd: every level in full (hex_odd). W: warps of the team (1: no team).
+template <int W>
+static __device__ __forceinline__ bool hex_plain_search(HexItems ring, bool odd, HexTeam* team, float* __restrict__ scratch,
                                                         unsigned short* __restrict__ subset, float sx, float sy, float sz,
                                                         float grid_scale, int depth, int lane, float& dx, float& dy,
                                                         float& dz) {
@@ -236,7 +286,7 @@ static __device__ __forceinline__ bool hex_plain_search(HexItems ring, bool odd,
     }
     const float Q = N / D;
     float qLast = odd ? hex_key1(ring.co, ring.k, 0.f, 0.f, 0.f, ring.es, ring.ea) : ring.group_key(0.f, 0.f, 0.f, 32, lane);
-    bool moved = false;
+    bool moved = false, full = odd;   // full: for good, where a level drops nothing a smaller one does not either
     float ds = grid_scale;
     for (int level = 0; level < depth; ++level) {
         QuadLevel lv{dx, dy, dz, ds * sx, ds * sy, ds * sz, 0.f, 0.f, 0.f, false};
@@ -244,7 +294,6 @@ static __device__ __forceinline__ bool hex_plain_search(HexItems ring, bool odd,
         if (lv.Sx == 0.f && lv.Sy == 0.f && lv.Sz == 0.f) continue;   // a lattice: every candidate is the centre
         float bk = -FLT_MAX;
         int bi = 1 << 30;
-        bool full = odd;
         if (!full) {
             const float U = fminf(ring.upper(lv, lane), Q);
             const float clear_of_U = U + (U * 0x1p-13f + 1e-37f);
@@ -282,13 +331,15 @@ static __device__ __forceinline__ bool hex_plain_search(HexItems ring, bool odd,
                 }
             }
             const unsigned alive = at_least(s, cut) & ~clear;
-            // Boxes that shrink with the smallest ring distance can leave every candidate within the margins. Judged one
-            // per lane, a candidate and item costs some 35 instructions; in full, four candidates and a halfhex 120.
-            full = ((__reduce_add_sync(FULL, __popc(alive)) + 31) >> 5) * ring.m > 14 * ring.k;
+            // Boxes that shrink with the smallest ring distance can leave every candidate within the margins: judged one per
+            // lane, a round of 32 candidates over the whole ring takes about half as long as all of them in full, and longer
+            // than a team of four takes for that (lattice with 1 % of jitter, 12^3 cells, us per iteration with the
+            // factor 2 / 4 / 7: 381 / 494 / 568; jittered 16^3 396 / 464 / 467).
+            full = ((__reduce_add_sync(FULL, __popc(alive)) + 31) >> 5) * ring.m > (W == 1 ? 14 : 2) * ring.k;
             if (!full) judge(ring, lv, alive, off, list, lane, bk, bi);
         }
         if (full) {
-            const float2 best = hex_level(ring.co, ring.k, ring.es, ring.ea, lv);
+            const float2 best = W == 1 ? hex_level<1>(ring.co, ring.k, ring.es, ring.ea, lv, 0) : hex_team_level(team, ring.co, ring.k, ring.es, ring.ea, lv);
             bk = best.x;
             bi = __float_as_int(best.y);
         }
