@@ -67,7 +67,7 @@ def _with_nan(xyz, seed):
     return x
 
 
-CASES = {"lattice": lambda x, el: _on_lattice(x, 1 / 80), "lattice8": lambda x, el: _on_lattice(x, 1 / 128),
+CASES = {"lattice": lambda x, el: _on_lattice(x, 1 / 180), "lattice8": lambda x, el: _on_lattice(x, 1 / 256),
          "near": lambda x, el: _near(x, el, 5, 1e-6), "nan": lambda x, el: _with_nan(x, 7)}
 
 
@@ -78,7 +78,7 @@ def test_packed_flat_against_general_search(vsdmo, case, depth):
     vertex (which a mesh with a larger ring brings to the whole batch), bit for bit: NaN keys leave the winner to
     the order of its lanes, which the oracle does not have."""
     from volumesurfacediscretemeshoptimization_b200 import meshgen as G
-    meshes = [(TRI, *G.tri_grid(130, 1)), (QUAD, *G.quad_grid(100, 2)), (TRI, *G.tri_grid(20, 3))]
+    meshes = [(TRI, *G.tri_grid(300, 1)), (QUAD, *G.quad_grid(160, 2)), (TRI, *G.tri_grid(20, 3))]
     start = [CASES[case](x, el) for _, x, el in meshes]
     large = (TRI, *_fan(17))
     got = []
@@ -94,12 +94,13 @@ def test_packed_flat_against_general_search(vsdmo, case, depth):
         want = got[1].mesh_positions(i)
         assert not np.array_equal(want, start[i], equal_nan=True)
         assert np.array_equal(got[0].mesh_positions(i).view(np.uint32), want.view(np.uint32)), i
-    gm = vsdmo.DMOMeshTri(*meshes[0][1:])
-    opt = vsdmo.DMOTriFlatClass(gm, n_iter=2, depth=depth, check_monotone=False)
-    gm.set_positions(start[0], original_order=True)
-    opt.restart()
-    opt.iterate(2)
-    assert np.array_equal(gm.positions(original_order=True).view(np.uint32), got[1].mesh_positions(0).view(np.uint32))
+    for i, mesh, cls in ((0, vsdmo.DMOMeshTri, vsdmo.DMOTriFlatClass), (1, vsdmo.DMOMeshQuad, vsdmo.DMOQuadFlatClass)):
+        gm = mesh(*meshes[i][1:])
+        opt = cls(gm, n_iter=2, depth=depth, check_monotone=False)
+        gm.set_positions(start[i], original_order=True)
+        opt.restart()
+        opt.iterate(2)
+        assert np.array_equal(gm.positions(original_order=True).view(np.uint32), got[1].mesh_positions(i).view(np.uint32))
 
 
 @pytest.mark.parametrize("ring", range(3))

@@ -34,11 +34,14 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int BATCH_WARPS = 8;
-// vertices of a single mesh's colour class from which on four vertices share a warp: below, a warp per vertex is the
-// shorter chain and fits in one wave (flat triangles / quads, ms per iteration, packed against not:
-// 64^2 (classes of 550) 0.049 / 0.064 : 0.042 / 0.063; 128^2 (2,300) 0.053 / 0.065 : 0.057 / 0.079; 500^2
-// (35,000) 0.167 / 0.199 : 0.407 / 0.575)
-constexpr int FLAT_PACKED_MIN = 2048;
+// Vertices of a single mesh's colour class from which on four vertices share a warp. Below, a warp per vertex is the
+// shorter chain and the class fits in a few waves, most of all while the mesh is far from converged and
+// candidates survive the filter. The lines are where no count of iterations is slower than without
+// (us for 1 / 5 / 20 iterations from a jittered start, packed against not: triangles, classes of 5,800
+// 143 / 410 / 1,164 : 103 / 325 / 1,135; 14,000 187 / 571 / 1,688 : 148 / 547 / 1,997; 23,000 233 / 729 / 2,144 :
+// 207 / 784 / 2,946; 58,000 416 / 1,319 / 3,822 : 379 / 1,661 / 6,431. Quads, whose search without is the
+// general one, 3,100 149 / 446 / 1,462 : 137 / 466 / 1,711; 4,700 148 / 464 / 1,474 : 147 / 528 / 1,979)
+constexpr int FLAT_PACKED_MIN_TRI = 16384, FLAT_PACKED_MIN_QUAD = 4096;
 // A work item of the batch is what one warp searches in sequence: up to eight steps, fewer where the classes
 // of all meshes together would leave resident warps without an item: eight steps always against this
 // rule 1.93 / 0.61 ms for 3 iterations of 33 meshes of up to 9,953 vertices, 13.9 / 13.9 for 256 of up to
@@ -401,7 +404,7 @@ void launch_dmo_flat(const Mesh& m, const DmoLaunch& L, int nq, int lanes, cudaS
 
 bool launch_dmo_flat_packed(const Mesh& m, const DmoLaunch& L, cudaStream_t s) {
     const int n = L.v1 - L.v0, maxk = std::max(m.maxHE, 1);
-    if (n < FLAT_PACKED_MIN || maxk > F8_MAX_RING) return false;
+    if (n < (m.fk == 4 ? FLAT_PACKED_MIN_QUAD : FLAT_PACKED_MIN_TRI) || maxk > F8_MAX_RING) return false;
     const int blocks = (n + 4 * F8_WARPS - 1) / (4 * F8_WARPS);
     VSDMO_CUDA(launch_chained(m.fk == 4 ? k_dmo_flat8<4> : k_dmo_flat8<3>, blocks, F8_WARPS * 32, flat8_smem(maxk), s, L.chained,
                               m.pos.p, m.he_rowptr.p, m.he.p, L.v0, L.v1, L.grid_scale, L.depth, maxk));
