@@ -954,14 +954,15 @@ constexpr int QS_BLOCKS = 148 * 3;
 constexpr int QS_THREADS = 256;
 constexpr int QS_UNROLL = 4;
 
+template <bool CHAINED>
 __global__ void __launch_bounds__(QS_THREADS)
-k_quality_stats(const int* __restrict__ el, int kind, long nE, const float4* pos_, IterStats* stats,
+k_quality_stats(const int* __restrict__ el, int kind, long nE, const float4* __restrict__ pos_, IterStats* stats,
                 int* iter, float* pmin, double* psum, int* pfail, unsigned* done, int check, int init) {
     __shared__ float smin[QS_THREADS / 32];
     __shared__ double ssum[QS_THREADS / 32];
     __shared__ int sfail[QS_THREADS / 32];
     __shared__ bool last;
-    const float4* pos = chain_wait(pos_);
+    const float4* __restrict__ pos = CHAINED ? chain_wait(pos_) : pos_;
     const int it = *iter;
     const float lastMin = init ? -FLT_MAX : stats[it].min_q;
     const float tol = 1e-6f * fmaxf(fabsf(lastMin), 1e-30f);
@@ -1190,8 +1191,9 @@ void launch_quality_stats(const Mesh& m, int kind, IterStats* d_stats, int* d_it
                           cudaStream_t s, bool chained) {
     // check_monotone < 0 marks the initial evaluation (slot 0, no check, no increment)
     const int init = check_monotone < 0 ? 1 : 0;
-    VSDMO_CUDA(launch_chained(k_quality_stats, QS_BLOCKS, QS_THREADS, 0, s, chained, m.elems.p, kind, m.nE, m.pos.p, d_stats,
-                              d_iter, d_partial_min, d_partial_sum, d_partial_fail, d_done, init ? 0 : check_monotone, init));
+    VSDMO_CUDA(launch_chained(chained ? k_quality_stats<true> : k_quality_stats<false>, QS_BLOCKS, QS_THREADS, 0, s, chained, m.elems.p, kind,
+                              m.nE, m.pos.p, d_stats, d_iter, d_partial_min, d_partial_sum, d_partial_fail, d_done,
+                              init ? 0 : check_monotone, init));
 }
 
 void launch_element_qualities(const Mesh& m, int kind, float* d_out, cudaStream_t s) {
