@@ -91,18 +91,18 @@ __device__ void flat_vertex(float4* __restrict__ pos, const int* __restrict__ ro
         const int4 h = he[b + t];
         const float4 pa = ldpos<COHERENT>(pos + h.x);
         const float4 pn = ldpos<COHERENT>(pos + he[b + (t + 1 == k ? 0 : t + 1)].x);
-        const float ax = bscale(pa.x - c0.x, p2, -ex), ay = bscale(pa.y - c0.y, p2, -ex);
-        const float nx = bscale(pn.x - c0.x, p2, -ex), ny = bscale(pn.y - c0.y, p2, -ex);
+        const float ax = bscale_here(pa.x - c0.x, p2, -ex), ay = bscale_here(pa.y - c0.y, p2, -ex);
+        const float nx = bscale_here(pn.x - c0.x, p2, -ex), ny = bscale_here(pn.y - c0.y, p2, -ex);
         if (FK == 3) {
             btri_co(ax, ay, nx, ny, co + BCO * t);
         } else {
             const float4 pb = ldpos<COHERENT>(pos + he[h.w].x);
-            const float bx = bscale(pb.x - c0.x, p2, -ex), by = bscale(pb.y - c0.y, p2, -ex);
+            const float bx = bscale_here(pb.x - c0.x, p2, -ex), by = bscale_here(pb.y - c0.y, p2, -ex);
             bquad_co(ax, ay, bx, by, nx, ny, co + BCO * t);
         }
     }
     __syncwarp(gmask);
-    const float sx = bscale(mdx, p2, -ex), sy = bscale(mdy, p2, -ex);
+    const float sx = bscale_here(mdx, p2, -ex), sy = bscale_here(mdy, p2, -ex);
     const int nvt = nq * nq / 2;
     float dx = 0.f, dy = 0.f;
     const float qOld = bkey<FK>(co, k, 0.f, 0.f);
@@ -134,7 +134,7 @@ __device__ void flat_vertex(float4* __restrict__ pos, const int* __restrict__ ro
     }
     if (gl == 0 && qOld < lastMax) {
         const float pu = bexp2(ex);
-        pos[v] = make_float4(c0.x + bscale(dx, pu, ex), c0.y + bscale(dy, pu, ex), c0.z, c0.w);
+        pos[v] = make_float4(c0.x + bscale_here(dx, pu, ex), c0.y + bscale_here(dy, pu, ex), c0.z, c0.w);
     }
     __syncwarp(gmask);
 }

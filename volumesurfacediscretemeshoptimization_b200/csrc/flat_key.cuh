@@ -11,6 +11,8 @@ static __device__ __forceinline__ float bexp2(int e) { return (e >= -126 && e <=
 // x 2^e when 2^e is no normal number: kept out of line (its code at every use crowds the instruction cache)
 static __device__ __noinline__ float bscale_far(float x, int e) { return ldexpf(x, e); }
 static __device__ __forceinline__ float bscale(float x, float p, int e) { return p != 0.f ? x * p : bscale_far(x, e); }
+// the same in line, for the general search
+static __device__ __forceinline__ float bscale_here(float x, float p, int e) { return p != 0.f ? x * p : ldexpf(x, e); }
 
 template <bool COHERENT>
 static __device__ __forceinline__ float4 ldpos(const float4* p) {
