@@ -26,9 +26,9 @@ namespace vsdmo {
 // Ring keys are a minimum over the tets, in whatever order they are folded, only while every L is positive
 // and its cube and the products of the fold are normal numbers: at a candidate beside a tet's collapsed base
 // the rounding of L decides, and NaN positions make the fold depend on the order. Rings with a tet whose L is
-// not bounded above the limit (in units of the ring's extent; edges of a percent) on the search box are searched
+// not bounded above the limit (in units of the ring's extent; edges of a quarter of a percent) on the search box are searched
 // without the filter.
-static __device__ __forceinline__ float tet_odd_limit(float grid_scale) { return 0x1p-12f * fmaxf(1.f, grid_scale * grid_scale); }
+static __device__ __forceinline__ float tet_odd_limit(float grid_scale) { return 0x1p-16f * fmaxf(1.f, grid_scale * grid_scale); }
 // L of a tet where its gradient vanishes: below L everywhere; NaN when a corner is
 static __device__ __forceinline__ float tet_least(float4 K1) {
     return fmaf(-1.f / 12.f, fmaf(K1.x, K1.x, fmaf(K1.y, K1.y, K1.z * K1.z)), K1.w);
