@@ -459,7 +459,7 @@ __device__ __forceinline__ float reduced_offset(int i, int n) { return (float)(n
 // accept and the minimum quality never decreases. counters: [0] reduced accepted,
 // [1] fallbacks, [2] fallbacks that moved, [3] skipped by the active set. rscale: first
 // reduced half-extent in units of grid_scale x the per-axis ring extent.
-constexpr int TET_LEARNED_MIN_BLOCKS = 32;   // 64 registers (24 bytes of spills): 32 warps per SM
+constexpr int TET_LEARNED_MIN_BLOCKS = 32;   // 64 registers (32 bytes of spills): 32 warps per SM
 __global__ void __launch_bounds__(TET_WARPS * 32, TET_LEARNED_MIN_BLOCKS)
 k_dmo_tet_learned(float4* __restrict__ pos, const int* __restrict__ rowptr, const int4* __restrict__ hf,
                   TetRingTable ring, int v0, int v1, float grid_scale, int maxk, const float* __restrict__ Y, int ldy, int rn, int rdepth,

@@ -286,7 +286,7 @@ static __device__ __forceinline__ bool hex_plain_search(HexItems ring, bool odd,
     }
     const float Q = N / D;
     float qLast = odd ? hex_key1(ring.co, ring.k, 0.f, 0.f, 0.f, ring.es, ring.ea) : ring.group_key(0.f, 0.f, 0.f, 32, lane);
-    bool moved = false, full = odd;   // full: for good, where a level drops nothing a smaller one does not either
+    bool moved = false, full = odd;   // once a level is evaluated in full, so are the smaller ones
     float ds = grid_scale;
     for (int level = 0; level < depth; ++level) {
         QuadLevel lv{dx, dy, dz, ds * sx, ds * sy, ds * sz, 0.f, 0.f, 0.f, false};

@@ -2,7 +2,7 @@
 //
 // The step as separate GEMM, reduction, Adam and packing launches (mlp.cu) is about thirty launches
 // of a few microseconds of work each: 275 us per step of 8,192 rows, of which the tensor cores need
-// two. In two launches it takes 27 us (25 us at 2,048 rows), now bound by the tile kernel's chain of
+// two. In two launches it takes 29 us of a training call, now bound by the tile kernel's chain of
 // dependent phases: 12 us of MMAs and epilogues, 4 us of gathering the rows (behind the update before
 // it) and 4 us of writing the gradient partials.
 //
