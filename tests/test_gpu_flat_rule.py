@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 def test_first_iteration_grows_with_the_mesh_only(vsdmo):
     """One iteration from a jittered start, latency bound at both sizes: classes of up to 2,700 vertices against
-    1,800. 1.1 times as long with a warp per vertex, 1.5 with four vertices per warp."""
+    1,800. 1.1 times as long with a warp per vertex, 1.9 with four vertices per warp."""
     import torch
     times = []
     for n in (90, 110):
@@ -26,4 +26,4 @@ def test_first_iteration_grows_with_the_mesh_only(vsdmo):
             opt.iterate(1)
             best = min(best, time.perf_counter() - t)
         times.append(best)
-    assert times[1] < 1.3 * times[0], times
+    assert times[1] < 1.5 * times[0], times
